@@ -891,7 +891,7 @@ bib_status import_populations(bib_ctx* c, Lattice& L, const double* src, Wire w)
     const int64_t n = d.n, plane = (int64_t)d.nx * d.ny, xplane = (int64_t)d.ny * d.nz;
     const size_t bytes = (size_t)(w.per ? w.per : Q) * n * sizeof(double);
     if (const double* m = static_cast<const double*>(device_view_of_host(src, bytes))) {
-        if (w.per) launch_import_aos(L, m, w.per, 0, n, c->stream);
+        if (w.per) launch_import_aos(L, m, w.per, 0, d.nx, c->stream);
         else launch_import_planes(L, m, 0, d.nz, n, c->stream);
         BIB_CHECK_LAUNCH(c);
         BIB_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -922,7 +922,7 @@ bib_status import_populations(bib_ctx* c, Lattice& L, const double* src, Wire w)
         }
         BIB_CUDA(c, cudaEventRecord(c->tx_ready[k & 1], c->copy_stream));
         BIB_CUDA(c, cudaStreamWaitEvent(c->stream, c->tx_ready[k & 1], 0));
-        if (w.per) launch_import_aos(L, buf, w.per, a * xplane, cnt * xplane, c->stream);
+        if (w.per) launch_import_aos(L, buf, w.per, (int)a, (int)cnt, c->stream);
         else launch_import_planes(L, buf, (int)a, (int)cnt, plane * cnt, c->stream);
         BIB_CHECK_LAUNCH(c);
         BIB_CUDA(c, cudaEventRecord(c->tx_free[k & 1], c->stream));
@@ -938,7 +938,7 @@ bib_status export_populations(bib_ctx* c, Lattice& L, double* dst, Wire w) {
     const int64_t n = d.n, plane = (int64_t)d.nx * d.ny, xplane = (int64_t)d.ny * d.nz;
     const size_t bytes = (size_t)(w.per ? w.per : Q) * n * sizeof(double);
     if (double* m = static_cast<double*>(const_cast<void*>(device_view_of_host(dst, bytes)))) {
-        if (w.per) launch_export_aos(L, m, w.per, 0, n, c->stream);
+        if (w.per) launch_export_aos(L, m, w.per, 0, d.nx, c->stream);
         else launch_export_planes(L, m, 0, d.nz, n, c->stream);
         BIB_CHECK_LAUNCH(c);
         BIB_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -955,7 +955,7 @@ bib_status export_populations(bib_ctx* c, Lattice& L, double* dst, Wire w) {
         const int64_t a = (int64_t)k * P, cnt = std::min<int64_t>(P, total - a);
         double* buf = c->stage + (size_t)(k & 1) * half;
         if (k >= 2) BIB_CUDA(c, cudaStreamWaitEvent(c->stream, c->tx_free[k & 1], 0));
-        if (w.per) launch_export_aos(L, buf, w.per, a * xplane, cnt * xplane, c->stream);
+        if (w.per) launch_export_aos(L, buf, w.per, (int)a, (int)cnt, c->stream);
         else launch_export_planes(L, buf, (int)a, (int)cnt, plane * cnt, c->stream);
         BIB_CHECK_LAUNCH(c);
         BIB_CUDA(c, cudaEventRecord(c->tx_ready[k & 1], c->stream));
