@@ -1335,17 +1335,20 @@ __device__ __forceinline__ bool tri_ray_z(const double* v0, const double* v1, co
     return true;
 }
 
-// One CTA per particle, one thread per triangle: z-rays through the integer (x, y) points of
+// One thread per triangle, one warp per CTA (grid: particles x blocks of 32 triangles): z-rays through the integer (x, y) points of
 // the triangle's xy box (RayTracer::find_intersections_z, RayTracer.hh:18-40); each hit goes
 // to its (periodically wrapped) column, height wrapped into [-1/2, nz - 1/2) (ZBuffer::put,
 // Arithmetic1D::remap_pos).  Columns are numbered x fastest.
-__global__ void __launch_bounds__(128) k_voxel_rays(LatticeDesc d, const ParticleDev* __restrict__ parts,
+// Bound by the FP64 pipe (about 80 operations per ray, 2 lanes per cycle and SM): warps spread over all
+// SMs.  One 128-thread CTA per particle kept one capsule of 1280 triangles on one SM for 97 us; with 40
+// one-warp CTAs the whole step of that capsule (80^3 cells, phase field) went from 250 to 127 us.
+__global__ void __launch_bounds__(32) k_voxel_rays(LatticeDesc d, const ParticleDev* __restrict__ parts,
                                                      const double* __restrict__ pos, int* __restrict__ count,
                                                      double* __restrict__ zbuf, int cap, int* __restrict__ overflow) {
     const ParticleDev& P = parts[blockIdx.x];
     const double* pv = pos + 3LL * P.v0;
     const int64_t ncol = (int64_t)d.nx * d.ny;
-    for (int t = threadIdx.x; t < P.nt; t += blockDim.x) {
+    for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < P.nt; t += gridDim.y * blockDim.x) {
         const double* v0 = pv + 3 * P.tri[3 * t];
         const double* v1 = pv + 3 * P.tri[3 * t + 1];
         const double* v2 = pv + 3 * P.tri[3 * t + 2];
@@ -1827,7 +1830,8 @@ void launch_spread(const Lattice& L, int fbuf, cudaStream_t s, bool record) {
 // *overflow (the column keeps its first cap crossings, the triangle casts no rays).
 void launch_voxelize(const Lattice& L, const double* pos, cudaStream_t s) {
     if (!L.phase || L.parts.empty()) return;
-    k_voxel_rays<<<(int)L.parts.size(), 128, 0, s>>>(L.d, L.pdev, pos, L.vox_count, L.vox_z, kVoxelCap, L.vox_err);
+    const dim3 rays((unsigned)L.parts.size(), (unsigned)std::min(65535, (L.max_nt + 31) / 32));
+    k_voxel_rays<<<rays, 32, 0, s>>>(L.d, L.pdev, pos, L.vox_count, L.vox_z, kVoxelCap, L.vox_err);
     const int64_t ncol = (int64_t)L.d.nx * L.d.ny;
     k_voxel_fill<<<(unsigned)((ncol + 127) / 128), 128, 0, s>>>(L.d, L.vox_count, L.vox_z, kVoxelCap, L.phase);
 }
