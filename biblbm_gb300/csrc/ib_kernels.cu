@@ -46,55 +46,6 @@ __device__ __forceinline__ W dirac_eval(int dirac, W x) {
                                         : W(2) * (W(1) + fast_sqrt(W(1) - W(3) * dx * dx)));
 }
 
-__device__ __forceinline__ double half_support(int dirac) { return dirac == BIB_DIRAC_PESKIN ? 2.0 : 1.5; }
-__device__ __forceinline__ int support(int dirac) { return dirac == BIB_DIRAC_PESKIN ? 4 : 3; }
-
-// Node classes of a single-block domain (ImmersedBoundaryDynamics.hh:46-66, 351-363): a
-// vertex is in the envelope when, on every axis, the min-mod distance from the domain
-// centre (N - 1)/2 is below the half width (N - 1)/2 + h (the bulk / envelope split only
-// selects between two interpolators with the same result here).  On a periodic axis the
-// min-mod distance is at most N/2 < (N - 1)/2 + h, so only walled axes can put a vertex
-// outside.  Non-finite positions are outside.
-__device__ __forceinline__ bool inside_envelope(const LatticeDesc& d, int dirac, const double* p) {
-    const double h = half_support(dirac);
-    const int N[3] = {d.nx, d.ny, d.nz};
-    const int per[3] = {d.px, d.py, d.pz};
-    bool in = true;
-    for (int a = 0; a < 3; ++a) {
-        if (per[a]) {
-            in = in && isfinite(p[a]);
-        } else {
-            const double top = (double)(N[a] - 1);
-            const double elo = 0.0 - h, ehi = top + h;
-            in = in && fabs(0.5 * (elo + ehi) - p[a]) < 0.5 * (ehi - elo);
-        }
-    }
-    return in;
-}
-
-// Positive remainder of x modulo N; the division is only taken more than a period away.
-__device__ __forceinline__ int pmod(int64_t x, int N) {
-    if (x >= 0 && x < N) return (int)x;
-    if (x < 0 && x >= -(int64_t)N) return (int)(x + N);
-    if (x >= N && x < 2LL * N) return (int)(x - N);
-    const int64_t r = x % N;
-    return (int)(r < 0 ? r + N : r);
-}
-
-// Arithmetic1D::remap_int(i, offset) with i0 = 0, Periodicity.h:106-110; returns a global
-// index, or -1 for a non-periodic index outside the domain.
-__device__ __forceinline__ int remap_global(int periodic, int N, int64_t i_local, int off) {
-    int64_t g;
-    if (periodic) {
-        int val = pmod(i_local + off, N) - off;
-        if (val < 0) val += N;
-        g = (int64_t)val + off;
-    } else {
-        g = i_local + off;
-    }
-    return (g < 0 || g >= N) ? -1 : (int)g;
-}
-
 // First support node of one axis as the spreading records it for the sparse force reset: on a
 // periodic axis reduced to one period (remap_global of lo + m is unchanged), so that it fits 32
 // bits; on a walled axis a vertex inside the envelope is within h + 1 of the domain.
