@@ -397,6 +397,8 @@ void free_particles(Lattice& L) {
         cudaFree(L.pgrid.keys[k]);
         cudaFree(L.pgrid.ids[k]);
     }
+    cudaFree(L.pgrid.cell);
+    cudaFree(L.pgrid.posf);
     cudaFree(L.pgrid.start);
     cudaFree(L.pgrid.end);
     cudaFree(L.pgrid.temp);
@@ -559,6 +561,8 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
             BIB_ALLOC(c, (void**)&G.ids[k], L.nvert * sizeof(uint32_t));
         }
         BIB_CUDA(c, cudaMemset(G.keys[1], 0, L.nvert * sizeof(uint32_t)));
+        BIB_ALLOC(c, (void**)&G.cell, L.nvert * sizeof(int4));
+        BIB_ALLOC(c, (void**)&G.posf, L.nvert * sizeof(float4));
         BIB_ALLOC(c, (void**)&G.start, G.table * sizeof(int));
         BIB_ALLOC(c, (void**)&G.end, G.table * sizeof(int));
         BIB_CUDA(c, cudaMemset(G.start, 0, G.table * sizeof(int)));

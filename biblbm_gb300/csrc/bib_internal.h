@@ -132,6 +132,8 @@ struct PairGrid {
     int bits = 0;
     uint32_t* keys[2] = {nullptr, nullptr};
     uint32_t* ids[2] = {nullptr, nullptr};
+    int4* cell = nullptr;    // per vertex
+    float4* posf = nullptr;  // per sorted vertex: position rounded to FP32, particle
     int* start = nullptr;
     int* end = nullptr;
     void* temp = nullptr;

@@ -1395,30 +1395,38 @@ __device__ __forceinline__ unsigned cell_hash(const PairCells& g, int cx, int cy
     return ((unsigned)cx * 73856093u ^ (unsigned)cy * 19349663u ^ (unsigned)cz * 83492791u) & g.mask;
 }
 
-// the buckets of the previous step's sort go back to empty
-__global__ void __launch_bounds__(128) k_pp_clear(int nvert, const uint32_t* __restrict__ prev_keys, int* start,
-                                                   int* end) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nvert) return;
-    start[prev_keys[s]] = 0;
-    end[prev_keys[s]] = 0;
-}
-
+// Cell and bucket of every vertex (the cell kept for the search); the buckets of the previous step's
+// sort go back to empty.
 __global__ void __launch_bounds__(128) k_pp_keys(LatticeDesc d, PairCells g, int nvert, const double* __restrict__ pos,
-                                                  uint32_t* __restrict__ keys, uint32_t* __restrict__ ids) {
+                                                  const uint32_t* __restrict__ prev_keys, int* __restrict__ start,
+                                                  int* __restrict__ end, uint32_t* __restrict__ keys,
+                                                  uint32_t* __restrict__ ids, int4* __restrict__ cell) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nvert) return;
+    start[prev_keys[v]] = 0;
+    end[prev_keys[v]] = 0;
     const double* p = pos + 3LL * v;
-    keys[v] = cell_hash(g, pair_cell(d, g, 0, p[0]), pair_cell(d, g, 1, p[1]), pair_cell(d, g, 2, p[2]));
+    const int c[3] = {pair_cell(d, g, 0, p[0]), pair_cell(d, g, 1, p[1]), pair_cell(d, g, 2, p[2])};
+    keys[v] = cell_hash(g, c[0], c[1], c[2]);
     ids[v] = (uint32_t)v;
+    cell[v] = make_int4(c[0], c[1], c[2], 0);
 }
 
-__global__ void __launch_bounds__(128) k_pp_bounds(int nvert, const uint32_t* __restrict__ keys, int* start, int* end) {
+// Bucket bounds, and the sorted vertices' positions in FP32 with their particles for the pre-test of the
+// pairs (a position more than 4 periods out becomes NaN, which the pre-test lets through).
+__global__ void __launch_bounds__(128) k_pp_bounds(LatticeDesc d, int nvert, const uint32_t* __restrict__ keys,
+                                                    const uint32_t* __restrict__ ids, const double* __restrict__ pos,
+                                                    const int* __restrict__ owner, int* __restrict__ start,
+                                                    int* __restrict__ end, float4* __restrict__ posf) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nvert) return;
     const uint32_t k = keys[s];
     if (s == 0 || keys[s - 1] != k) start[k] = s;
     if (s == nvert - 1 || keys[s + 1] != k) end[k] = s + 1;
+    const int v = (int)ids[s];
+    const double x = pos[3LL * v], y = pos[3LL * v + 1], z = pos[3LL * v + 2];
+    const bool far = !(fabs(x) <= 4.0 * d.nx && fabs(y) <= 4.0 * d.ny && fabs(z) <= 4.0 * d.nz);
+    posf[s] = make_float4(far ? nanf("") : (float)x, (float)y, (float)z, __int_as_float(owner[v]));
 }
 
 // Arithmetic1D::min_mod_diff (Periodicity.h:27-35, 96-99) on periodic axes
@@ -1429,61 +1437,76 @@ __device__ __forceinline__ double min_image(const LatticeDesc& d, int a, double 
     return dx - floor(dx * d.inv_n[a] + 0.5) * N;
 }
 
-// One thread per vertex: the sum over partners j of other particles within the cutoff of
-// (-phi(d) / d) (x_j - x_i) (CollisionHandler::handle_collision, CollisionForces.h:187-199),
-// added to the vertex's force.  Every pair is evaluated from both ends, so no atomics.
-__global__ void __launch_bounds__(128) k_pp_forces(LatticeDesc d, Interactions I, PairCells g, int nvert,
-                                                    const double* __restrict__ pos, const int* __restrict__ owner,
-                                                    const uint32_t* __restrict__ ids, const int* __restrict__ start,
-                                                    const int* __restrict__ end, double* __restrict__ force) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nvert) return;
-    const double xi[3] = {pos[3LL * i], pos[3LL * i + 1], pos[3LL * i + 2]};
-    if (!(isfinite(xi[0]) && isfinite(xi[1]) && isfinite(xi[2]))) return;
-    const int oi = owner[i];
-    const int c[3] = {pair_cell(d, g, 0, xi[0]), pair_cell(d, g, 1, xi[1]), pair_cell(d, g, 2, xi[2])};
+__device__ __forceinline__ float min_image_f(int per, float N, float dx) {
+    return per ? dx - floorf(dx / N + 0.5f) * N : dx;
+}
+
+// One warp per vertex, one lane per neighbour cell: the sum over partners j of other particles within
+// the cutoff of (-phi(d) / d) (x_j - x_i) (CollisionHandler::handle_collision, CollisionForces.h:187-199),
+// added to the vertex's force.  Every pair is evaluated from both ends and the lanes are added up in one
+// order, so no atomics.  Pairs pass an FP32 distance test first, with `reach` = the cutoff plus 2^-18 of
+// the longest axis (more than the FP32 positions and differences can be off within 4 periods); the FP64
+// test alone decides the rest.
+// Bound by the latency of the bucket lookups: all 27 of a vertex are in flight at once, over FP32
+// positions in bucket order.  One thread per vertex that walked its 27 cells and formed every distance
+// in FP64 took 156 us for 40 cells of 642 vertices in a 192 x 50 x 50 pipe, whose step went from 274 to
+// 145 us.
+__global__ void __launch_bounds__(128) k_pp_forces(LatticeDesc d, Interactions I, PairCells g, int nvert, float reach,
+                                                    const double* __restrict__ pos, const uint32_t* __restrict__ ids,
+                                                    const int4* __restrict__ cell, const float4* __restrict__ posf,
+                                                    const int* __restrict__ start, const int* __restrict__ end,
+                                                    double* __restrict__ force) {
+    const unsigned FULL = 0xffffffffu;
+    const int slot = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (slot >= nvert) return;  // whole warps
+    const int i = (int)ids[slot];
+    const float4 pi = posf[slot];
+    const int4 c = cell[i];
     const int per[3] = {d.px, d.py, d.pz};
-    const double cut2 = I.pp_cut * I.pp_cut;
+    int n[3] = {c.x + lane % 3 - 1, c.y + (lane / 3) % 3 - 1, c.z + lane / 9 - 1};
+    bool ok = lane < 27;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (n[a] < 0 || n[a] >= g.nc[a]) {
+            if (!per[a]) ok = false;
+            else n[a] = (n[a] + g.nc[a]) % g.nc[a];
+        }
+    const unsigned h = ok ? cell_hash(g, n[0], n[1], n[2]) : 0u;
+    // neighbour cells that share a bucket are visited once, by the first lane that has it
+    const unsigned live = __ballot_sync(FULL, ok), same = __match_any_sync(FULL, h) & live;
+    const bool mine = ok && (same & ((1u << lane) - 1)) == 0;
     double f[3] = {0.0, 0.0, 0.0};
-    unsigned seen[27];
-    int nseen = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-                int n[3] = {c[0] + dx, c[1] + dy, c[2] + dz};
-                bool ok = true;
-                for (int a = 0; a < 3; ++a) {
-                    if (n[a] < 0 || n[a] >= g.nc[a]) {
-                        if (!per[a]) ok = false;
-                        else n[a] = (n[a] + g.nc[a]) % g.nc[a];
-                    }
-                }
-                if (!ok) continue;
-                const unsigned h = cell_hash(g, n[0], n[1], n[2]);
-                bool dup = false;  // neighbour cells that share a bucket are visited once
-                for (int q = 0; q < nseen; ++q) dup = dup || seen[q] == h;
-                if (dup) continue;
-                seen[nseen++] = h;
-                for (int s = start[h]; s < end[h]; ++s) {
-                    const int j = (int)ids[s];
-                    if (owner[j] == oi) continue;
-                    const double dr[3] = {min_image(d, 0, pos[3LL * j] - xi[0]), min_image(d, 1, pos[3LL * j + 1] - xi[1]),
-                                          min_image(d, 2, pos[3LL * j + 2] - xi[2])};
-                    const double dsq = dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2];
-                    if (!(dsq <= cut2)) continue;
-                    const double dist = sqrt(dsq);
-                    for (int k = 0; k < I.npp; ++k) {
-                        if (!(dsq <= I.pp[k].r0 * I.pp[k].r0)) continue;
-                        const double sc = -potential_eval(I.pp[k], dist) / dist;
-                        f[0] += sc * dr[0];
-                        f[1] += sc * dr[1];
-                        f[2] += sc * dr[2];
-                    }
-                }
-            }
-    force[3LL * i] += f[0];
-    force[3LL * i + 1] += f[1];
-    force[3LL * i + 2] += f[2];
+    bool hit = false;
+    const int s1 = mine ? end[h] : 0;
+    for (int s = mine ? start[h] : 0; s < s1; ++s) {
+        const float4 q = posf[s];
+        if (__float_as_int(q.w) == __float_as_int(pi.w)) continue;
+        const float ex = min_image_f(d.px, (float)d.nx, q.x - pi.x), ey = min_image_f(d.py, (float)d.ny, q.y - pi.y),
+                    ez = min_image_f(d.pz, (float)d.nz, q.z - pi.z);
+        if (ex * ex + ey * ey + ez * ez > reach * reach) continue;
+        const double xi[3] = {pos[3LL * i], pos[3LL * i + 1], pos[3LL * i + 2]};
+        if (!(isfinite(xi[0]) && isfinite(xi[1]) && isfinite(xi[2]))) continue;
+        const int j = (int)ids[s];
+        const double dr[3] = {min_image(d, 0, pos[3LL * j] - xi[0]), min_image(d, 1, pos[3LL * j + 1] - xi[1]),
+                              min_image(d, 2, pos[3LL * j + 2] - xi[2])};
+        const double dsq = dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2];
+        if (!(dsq <= I.pp_cut * I.pp_cut)) continue;
+        const double dist = sqrt(dsq);
+        for (int k = 0; k < I.npp; ++k) {
+            if (!(dsq <= I.pp[k].r0 * I.pp[k].r0)) continue;
+            const double sc = -potential_eval(I.pp[k], dist) / dist;
+            f[0] += sc * dr[0];
+            f[1] += sc * dr[1];
+            f[2] += sc * dr[2];
+            hit = true;
+        }
+    }
+    if (!__any_sync(FULL, hit)) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        for (int a = 0; a < 3; ++a) f[a] += __shfl_down_sync(FULL, f[a], o);
+    if (lane == 0)
+        for (int a = 0; a < 3; ++a) force[3LL * i + a] += f[a];
 }
 
 }  // namespace
@@ -1703,13 +1726,13 @@ void launch_pp_forces(const Lattice& L, cudaStream_t s) {
     }
     g.mask = G.table - 1;
     const unsigned b = (L.nvert + 127) / 128;
-    k_pp_clear<<<b, 128, 0, s>>>(L.nvert, G.keys[1], G.start, G.end);
-    k_pp_keys<<<b, 128, 0, s>>>(L.d, g, L.nvert, L.pos[L.pcur], G.keys[0], G.ids[0]);
+    k_pp_keys<<<b, 128, 0, s>>>(L.d, g, L.nvert, L.pos[L.pcur], G.keys[1], G.start, G.end, G.keys[0], G.ids[0], G.cell);
     size_t tb = G.temp_bytes;
     cub::DeviceRadixSort::SortPairs(G.temp, tb, G.keys[0], G.keys[1], G.ids[0], G.ids[1], L.nvert, 0, G.bits, s);
-    k_pp_bounds<<<b, 128, 0, s>>>(L.nvert, G.keys[1], G.start, G.end);
-    k_pp_forces<<<b, 128, 0, s>>>(L.d, L.inter, g, L.nvert, L.pos[L.pcur], L.vert_particle, G.ids[1], G.start, G.end,
-                                  L.force);
+    k_pp_bounds<<<b, 128, 0, s>>>(L.d, L.nvert, G.keys[1], G.ids[1], L.pos[L.pcur], L.vert_particle, G.start, G.end, G.posf);
+    const float reach = (float)(L.inter.pp_cut + std::max(L.d.nx, std::max(L.d.ny, L.d.nz)) / 262144.0);
+    k_pp_forces<<<(unsigned)((32LL * L.nvert + 127) / 128), 128, 0, s>>>(L.d, L.inter, g, L.nvert, reach, L.pos[L.pcur],
+                                                                         G.ids[1], G.cell, G.posf, G.start, G.end, L.force);
 }
 
 void launch_particle_update(const Lattice& L, cudaStream_t s) {
