@@ -2508,6 +2508,38 @@ bib_status ckpt_get_device(bib_ctx* c, CkptFile& F, void* dev, size_t bytes, std
     return BIB_OK;
 }
 
+// A force field in the file's order, one array per component: component by component out of (into) the
+// device's cells of three.
+template <class FT>
+bib_status ckpt_put_force(bib_ctx* c, CkptFile& F, const Lattice& L, const void* dev) {
+    const int64_t stride = L.d.stride, chunk = (int64_t)(kCkptChunk / (3 * sizeof(FT)));
+    std::vector<FT> cells, one;
+    for (int a = 0; a < 3; ++a)
+        for (int64_t k = 0; k < stride; k += chunk) {
+            const int64_t n = std::min(chunk, stride - k);
+            cells.resize((size_t)(3 * n));
+            one.resize((size_t)n);
+            BIB_CUDA(c, cudaMemcpy(cells.data(), static_cast<const FT*>(dev) + 3 * k, 3 * n * sizeof(FT), cudaMemcpyDeviceToHost));
+            for (int64_t i = 0; i < n; ++i) one[(size_t)i] = cells[(size_t)(3 * i + a)];
+            if (!F.put(one.data(), (size_t)n * sizeof(FT))) return fail(c, BIB_EINVAL, "checkpoint write failed");
+        }
+    return BIB_OK;
+}
+
+template <class FT>
+bib_status ckpt_get_force(bib_ctx* c, CkptFile& F, const Lattice& L, void* dev) {
+    const int64_t stride = L.d.stride;
+    std::vector<FT> cells((size_t)(3 * stride)), one((size_t)std::min<int64_t>(stride, kCkptChunk / sizeof(FT)));
+    for (int a = 0; a < 3; ++a)
+        for (int64_t k = 0; k < stride; k += (int64_t)one.size()) {
+            const int64_t n = std::min((int64_t)one.size(), stride - k);
+            if (!F.get(one.data(), (size_t)n * sizeof(FT))) return fail(c, BIB_EINVAL, "checkpoint file is truncated");
+            for (int64_t i = 0; i < n; ++i) cells[(size_t)(3 * (k + i) + a)] = one[(size_t)i];
+        }
+    BIB_CUDA(c, cudaMemcpy(dev, cells.data(), cells.size() * sizeof(FT), cudaMemcpyHostToDevice));
+    return BIB_OK;
+}
+
 size_t wall_bytes(const Lattice& L) {
     return L.d.fd_walls ? pop_bytes(L.storage) * Q * 2 * (size_t)L.d.nx * L.d.nz : 0;
 }
@@ -2566,11 +2598,12 @@ bib_status bib_checkpoint_save(bib_ctx* c, int32_t h, const char* path) {
     if (!F.put(&hd, sizeof(hd))) return fail(c, BIB_EINVAL, "checkpoint write failed");
     std::vector<unsigned char> buf;
     const size_t pb = pop_bytes(L->storage) * Q * (size_t)L->d.stride;
-    const size_t fb = force_bytes(L->storage) * 3 * (size_t)L->d.stride;
     if ((st = ckpt_put_device(c, F, L->f[L->cur], pb, buf))) return st;
     if (L->d.fd_walls && (st = ckpt_put_device(c, F, L->wall, wall_bytes(*L), buf))) return st;
     for (int k = 0; k < 2; ++k)
-        if ((st = ckpt_put_device(c, F, L->F[k], fb, buf))) return st;
+        if ((st = L->storage == BIB_STORAGE_F64 ? ckpt_put_force<double>(c, F, *L, L->F[k])
+                                                : ckpt_put_force<float>(c, F, *L, L->F[k])))
+            return st;
     if (L->phase && (st = ckpt_put_device(c, F, L->phase, (size_t)L->d.stride, buf))) return st;
     if (L->celltype && (st = ckpt_put_device(c, F, L->celltype, (size_t)L->d.n, buf))) return st;
     for (const ParticleHost& ph : L->parts) {
@@ -2665,7 +2698,9 @@ bib_status bib_checkpoint_load(bib_ctx* c, int32_t h, const char* path) {
     if ((st = ckpt_get_device(c, F, L->f[hd.cur], pb, buf))) return st;
     if (L->d.fd_walls && (st = ckpt_get_device(c, F, L->wall, wall_bytes(*L), buf))) return st;
     for (int k = 0; k < 2; ++k)
-        if ((st = ckpt_get_device(c, F, L->F[k], fb, buf))) return st;
+        if ((st = L->storage == BIB_STORAGE_F64 ? ckpt_get_force<double>(c, F, *L, L->F[k])
+                                                : ckpt_get_force<float>(c, F, *L, L->F[k])))
+            return st;
     if (L->phase && (st = ckpt_get_device(c, F, L->phase, (size_t)L->d.stride, buf))) return st;
     if (hd.has_types) {
         std::vector<uint8_t> types((size_t)L->d.n);

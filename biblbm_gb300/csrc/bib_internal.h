@@ -293,7 +293,7 @@ struct Lattice {
     void* f[2] = {nullptr, nullptr};
     int cur = 0;
     void* wall = nullptr;             // 2 sides x nx x nz x 19 populations of FD wall nodes
-    void* F[2] = {nullptr, nullptr};  // force fields (double for F64 storage, float otherwise)
+    void* F[2] = {nullptr, nullptr};  // force fields, F[3 k + a] (double for F64 storage, float otherwise)
     int fe = 0;
     bool target_clean = false;        // F[1-fe] holds the body force, ready to receive spreading
     // Sparse force reset (opt-in; reduced-precision storage, coupled step, no phase field, cell

@@ -70,6 +70,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
     }
     return false;
 }
+// Shared -> global bulk copy, completed by the thread's bulk group; dst, src and bytes are multiples of 16.
+__device__ __forceinline__ void bulk_copy_s2g(void* dst, const void* src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(dst),
+                 "r"(smem_addr(src)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // Global -> shared bulk copy; dst, src and bytes are multiples of 16.
 __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -170,7 +178,7 @@ struct TileOf {
 constexpr int kCplNone = 0, kCplDense = 1, kCplSparse = 2;
 
 // Stage layout (compile-time): 19 population rows, the collision force (BGK + Guo) and,
-// for the dense coupled step, the previous force, each TILE cells long.
+// for the dense coupled step, the previous force (three values per cell), each TILE cells long.
 template <class T, int CPL, int COLL>
 struct StageLayout {
     using FT = typename Store<T>::F;
@@ -183,6 +191,8 @@ struct StageLayout {
     static constexpr unsigned OFF_FCOL = Q * POP;
     static constexpr unsigned OFF_FPREV = OFF_FCOL + (NEED_FCOL ? 3 * FRC : 0);
     static constexpr unsigned BYTES = ((OFF_FPREV + (CPL == kCplDense ? 3 * FRC : 0)) + 127) / 128 * 128;
+    // dense coupling: one tile of the body force in front of the stages, the source of the reset
+    static constexpr unsigned RESET = CPL == kCplDense ? 3 * FRC : 0;
 };
 
 constexpr int kMaxStages = 8;
@@ -230,10 +240,47 @@ __device__ __forceinline__ PopLane pop_lane(int lane) {
     return p;
 }
 
+// The reset of the previous force field to the body force (dense coupling), by one bulk store per tile
+// from a tile of the body force in shared memory, issued by the producer once the tile's stage has been
+// loaded anew (its consumers have handed it back, so the previous force has been read).  Stores from
+// the consumers would touch every third word three times.  After the loads, which the refill of the
+// stage waits for, and from the tile's number: with the run kept per stage in lane registers the FP16
+// kernel at its 56 registers took 168.5 us for 512 x 128 x 128 cells, so 160.8 (162.7 with one force
+// array per component and the reset stored by the consumers).
+template <class FT>
+__device__ __forceinline__ void fill_reset(FT* reset, const double* body, int n, int t, int nthreads) {
+    for (int k = t; k < n; k += nthreads) reset[k] = (FT)body[k % 3];
+    proxy_fence();
+}
+template <class FT>
+__device__ __forceinline__ void reset_tile(const LatticeDesc& d, const StagedGeom& g, int64_t tile, FT* Fprev, const FT* reset) {
+    bulk_copy_s2g(Fprev + 3 * tile_ref(d, g, tile).row0, reset, (unsigned)(3 * g.Ct * sizeof(FT)));
+}
+
+// The batched kernel, whose tiles' lattices would have to be looked up again, keeps the run: lane s of
+// the producer warp that of the tile in stage s (FP32, 32 lattices of 96^3: 1018 us; looked
+// up again or noted in shared memory by lane 0, 1080 to 1110).
+template <class FT>
+struct ResetRun {
+    FT* run = nullptr;
+    unsigned bytes = 0, phase = 0;
+    __device__ __forceinline__ void turn(FT* next, unsigned n, unsigned next_phase, const FT* reset) {
+        if (run) bulk_copy_s2g(run, reset, bytes);
+        run = next;
+        bytes = n;
+        phase = next_phase;
+    }
+    // the last tile of the lane's stage, once it has landed; then every store of the lane
+    __device__ __forceinline__ void finish(uint64_t* full, const FT* reset) {
+        if (run && mbar_wait_bounded(full, phase)) bulk_copy_s2g(run, reset, bytes);
+        run = nullptr;
+        bulk_wait_all();
+    }
+};
 // Copies of one tile into one stage, by the producer warp: lane i < 19 moves population i,
-// lanes 19..21 the collision force, lanes 22..24 the previous force (dense coupling).
+// lane 19 the collision force, lane 20 the previous force (dense coupling).  Returns the tile's first cell.
 template <class T, int CPL, int COLL>
-__device__ __forceinline__ void load_tile(const LatticeDesc& d, const StagedGeom& g, int64_t tile, unsigned char* stage,
+__device__ __forceinline__ int64_t load_tile(const LatticeDesc& d, const StagedGeom& g, int64_t tile, unsigned char* stage,
                                           uint64_t* bar, const T* fin, const T* wall, const typename Store<T>::F* Fcol,
                                           const typename Store<T>::F* Fprev, int lane, const PopLane& pl) {
     using L = StageLayout<T, CPL, COLL>;
@@ -284,16 +331,12 @@ __device__ __forceinline__ void load_tile(const LatticeDesc& d, const StagedGeom
             bulk_copy_g2s(dst + run_at, run, run_len, bar);
         }
     } else {
-        const unsigned fb = (unsigned)(g.Ct * sizeof(FT));
-        if (L::NEED_FCOL && lane < Q + 3) {
-            const int c = lane - Q;
-            bulk_copy_g2s(stage + L::OFF_FCOL + c * L::FRC, Fcol + c * d.stride + t.row0, fb, bar);
-        } else if (CPL == kCplDense && lane >= Q + 3 && lane < Q + 6) {
-            const int c = lane - Q - 3;
-            bulk_copy_g2s(stage + L::OFF_FPREV + c * L::FRC, Fprev + c * d.stride + t.row0, fb, bar);
-        }
+        const unsigned fb = (unsigned)(3 * g.Ct * sizeof(FT));
+        if (L::NEED_FCOL && lane == Q) bulk_copy_g2s(stage + L::OFF_FCOL, Fcol + 3 * t.row0, fb, bar);
+        else if (CPL == kCplDense && lane == Q + 1) bulk_copy_g2s(stage + L::OFF_FPREV, Fprev + 3 * t.row0, fb, bar);
     }
     __syncwarp();
+    return t.row0;
 }
 
 // Consumer side of one tile: the thread's cell of every tile and its x-neighbours (periodic in
@@ -316,24 +359,18 @@ __device__ __forceinline__ TileCell tile_cell(const LatticeDesc& d, int Ct, int 
 // Collision and stores of one cell k of row y whose gathered populations are in f: a
 // BounceBack / NoDynamics node is not collided (zero velocity), every other node collides with
 // the force F; the coupled step writes its velocity (j/rho + Fp/2, or the wall's on
-// finite-difference wall rows) and, with the dense coupling, resets the previous force.
+// finite-difference wall rows).
 template <class T, int CPL, int COLL>
 __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideParams<typename Store<T>::C>& cp,
-                                            T* __restrict__ fout, typename Store<T>::F* __restrict__ Fprev,
-                                            typename Store<T>::U* __restrict__ u_out, const uint8_t* __restrict__ phase,
+                                            T* __restrict__ fout, typename Store<T>::U* __restrict__ u_out, const uint8_t* __restrict__ phase,
                                             const uint8_t* __restrict__ celltype, int64_t k, int y, bool fd,
                                             typename Store<T>::C* f, const typename Store<T>::C* F,
                                             const typename Store<T>::C* Fp) {
     using C = typename Store<T>::C;
-    using FT = typename Store<T>::F;
     using UT = typename Store<T>::U;
     const int ctype = d.has_types ? celltype[k] : BIB_CELL_FLUID;
     if (ctype != BIB_CELL_FLUID) {  // BounceBack / NoDynamics node: no collision, zero velocity
         if (CPL != kCplNone) store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
-        if (CPL == kCplDense) {
-#pragma unroll
-            for (int q = 0; q < 3; ++q) Fprev[q * d.stride + k] = (FT)cp.body[q];
-        }
         if (ctype == BIB_CELL_BOUNCE_BACK) bounce_back_cell(f);
         store_cell<T, C>(fout + k, d.stride, f);
         return;
@@ -342,8 +379,8 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
     if (COLL == BIB_COLLISION_BGK_GUO_VOF && d.use_phase && phase[k]) om = cp.om1;
     const CellMoments<C> m = moments_compact<C>(f, cp.invS);
     if (CPL != kCplNone) {
-        // the velocity and the force reset are stored before the relaxation, so that the
-        // previous force is dead while the relaxation runs
+        // the velocity is stored before the relaxation, so that the previous force is dead while
+        // the relaxation runs
         C u[3];
         if (fd) {
             const int side = y == 0 ? 0 : 1;
@@ -353,10 +390,6 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
             velocity_compact<C>(m, Fp, u);
         }
         store_u_from<UT, C>(u_out, k, u[0], u[1], u[2]);
-        if (CPL == kCplDense) {
-#pragma unroll
-            for (int q = 0; q < 3; ++q) Fprev[q * d.stride + k] = (FT)cp.body[q];
-        }
     }
     staged_relax<C, COLL>(f, F, om, cp.omm, cp.S, m);
     store_cell<T, C>(fout + k, d.stride, f);
@@ -367,8 +400,7 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
 template <class T, int CPL, int COLL>
 __device__ __forceinline__ void consume_cell(const LatticeDesc& d, const StagedGeom& g, int64_t tile, const unsigned char* st,
                                              const CollideParams<typename Store<T>::C>& cp, T* __restrict__ fout,
-                                             typename Store<T>::F* __restrict__ Fprev, typename Store<T>::U* __restrict__ u_out,
-                                             const uint8_t* __restrict__ phase, const uint8_t* __restrict__ celltype,
+                                             typename Store<T>::U* __restrict__ u_out, const uint8_t* __restrict__ phase, const uint8_t* __restrict__ celltype,
                                              const TileCell& cell, uint64_t* empty_s, int lane) {
     using C = typename Store<T>::C;
     using FT = typename Store<T>::F;
@@ -402,11 +434,11 @@ __device__ __forceinline__ void consume_cell(const LatticeDesc& d, const StagedG
         }
         if (L::NEED_FCOL) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) F[q] = (C)SFc[q * TILE + o0];
+            for (int q = 0; q < 3; ++q) F[q] = (C)SFc[3 * o0 + q];
         }
         if (CPL == kCplDense) {
 #pragma unroll
-            for (int q = 0; q < 3; ++q) Fp[q] = (C)SFp[q * TILE + o0];
+            for (int q = 0; q < 3; ++q) Fp[q] = (C)SFp[3 * o0 + q];
         } else if (CPL == kCplSparse) {
 #pragma unroll
             for (int q = 0; q < 3; ++q) Fp[q] = cp.body[q];
@@ -416,17 +448,7 @@ __device__ __forceinline__ void consume_cell(const LatticeDesc& d, const StagedG
     __syncwarp();
     if (lane == 0) mbar_arrive(empty_s);
     if (!active) return;
-    finish_cell<T, CPL, COLL>(d, cp, fout, Fprev, u_out, phase, celltype, t.row0 + o0, y, fd, f, F, Fp);
-}
-
-// The consumer of one tile.
-template <class T, int CPL, int COLL>
-__device__ __forceinline__ void consume_tile(const LatticeDesc& d, const StagedGeom& g, int64_t tile, const unsigned char* st,
-                                             const CollideParams<typename Store<T>::C>& cp, T* __restrict__ fout,
-                                             typename Store<T>::F* __restrict__ Fprev, typename Store<T>::U* __restrict__ u_out,
-                                             const uint8_t* __restrict__ phase, const uint8_t* __restrict__ celltype,
-                                             const TileCell& cell, uint64_t* empty_s, int lane) {
-    consume_cell<T, CPL, COLL>(d, g, tile, st, cp, fout, Fprev, u_out, phase, celltype, cell, empty_s, lane);
+    finish_cell<T, CPL, COLL>(d, cp, fout, u_out, phase, celltype, t.row0 + o0, y, fd, f, F, Fp);
 }
 
 // Warp-specialised persistent kernel: warp 0 produces, warps 1..CONSUMERS collide.  Stage
@@ -455,10 +477,12 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + kMaxStages;
-    unsigned char* stages = smem + 256;
+    FT* reset = reinterpret_cast<FT*>(smem + 256);
+    unsigned char* stages = smem + 256 + L::RESET;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int NS = g.nstages;
     if ((int64_t)blockIdx.x >= g.ntiles) return;
+    if (CPL == kCplDense) fill_reset(reset, d.body, 3 * TILE, tid, L::THREADS);
     if (tid == 0) {
         for (int k = 0; k < NS; ++k) {
             mbar_init(&full[k], 1);
@@ -487,13 +511,17 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
                 continue;
             }
             load_tile<T, CPL, COLL>(d, g, tile, stages + s * L::BYTES, &full[s], fin, wall, Fcol, Fprev, lane, pl);
+            if (CPL == kCplDense && use > 0 && lane == 0) reset_tile(d, g, tile - (int64_t)NS * gridDim.x, Fprev, reset);
         }
         // a copy may still be landing only if the consumers gave up; wait for it so that
-        // no bulk copy writes into the shared memory of a retired CTA (a withheld tile has none)
+        // no bulk copy writes into the shared memory of a retired CTA (a withheld tile has none); the
+        // last tiles' previous force is reset once it has landed
         if (lane == 0) {
             const int issued = it;
             for (int k = issued > NS ? issued - NS : 0; k < issued; ++k)
-                if (k != withheld) mbar_wait_bounded(&full[k % NS], (unsigned)(k / NS) & 1u);
+                if (k != withheld && mbar_wait_bounded(&full[k % NS], (unsigned)(k / NS) & 1u) && CPL == kCplDense)
+                    reset_tile(d, g, blockIdx.x + (int64_t)k * gridDim.x, Fprev, reset);
+            if (CPL == kCplDense) bulk_wait_all();
         }
         return;
     }
@@ -509,8 +537,7 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
             if (lane == 0) atomicExch(wait_err, 1);
             return;
         }
-        consume_tile<T, CPL, COLL>(d, g, tile, stages + s * L::BYTES, cp, fout, Fprev, u_out, phase, celltype, cell,
-                                        &empty[s], lane);
+        consume_cell<T, CPL, COLL>(d, g, tile, stages + s * L::BYTES, cp, fout, u_out, phase, celltype, cell, &empty[s], lane);
     }
 }
 
@@ -571,7 +598,8 @@ __global__ void __launch_bounds__(StageLayout<T, kCplDense, COLL>::THREADS, stag
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + kMaxStages;
-    unsigned char* stages = smem + 256;
+    FT* reset = reinterpret_cast<FT*>(smem + 256);
+    unsigned char* stages = smem + 256 + L::RESET;
     CollideView* pview = reinterpret_cast<CollideView*>(stages + (size_t)NS * L::BYTES);
     CollideView* cview = pview + 1;
     int64_t* tile0 = reinterpret_cast<int64_t*>(cview + 1);
@@ -591,6 +619,8 @@ __global__ void __launch_bounds__(StageLayout<T, kCplDense, COLL>::THREADS, stag
     if (warp == 0) {
         const PopLane pl = pop_lane(lane);
         int it = 0, vi = 0, have = -1;
+        double* body = reinterpret_cast<double*>(empty + kMaxStages);  // in the reset tile (warp 0)
+        ResetRun<FT> last;
         for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
             const int s = it % NS, use = it / NS;
             if (use > 0) {
@@ -605,17 +635,27 @@ __global__ void __launch_bounds__(StageLayout<T, kCplDense, COLL>::THREADS, stag
                 copy_view(pview, views + vi, lane, 32);
                 __syncwarp();
                 have = vi;
+                const double* b = pview->d.body;
+                if (it == 0 || b[0] != body[0] || b[1] != body[1] || b[2] != body[2]) {
+                    // another body force: the tiles in the ring are reset with the one before first
+                    if (lane < NS) last.finish(&full[lane], reset);
+                    __syncwarp();
+                    fill_reset(reset, b, 3 * L::TILE, lane, 32);
+                    if (lane < 3) body[lane] = b[lane];
+                    __syncwarp();
+                }
             }
             const CollideView& V = *pview;
-            load_tile<T, kCplDense, COLL>(V.d, view_geom(V, NS), tile - V.tile0, stages + s * L::BYTES, &full[s],
-                                     static_cast<const T*>(V.fin), static_cast<const T*>(V.wall),
-                                     static_cast<const FT*>(V.Fcol), static_cast<const FT*>(V.Fprev), lane, pl);
+            const int64_t row0 = load_tile<T, kCplDense, COLL>(
+                V.d, view_geom(V, NS), tile - V.tile0, stages + s * L::BYTES, &full[s], static_cast<const T*>(V.fin),
+                static_cast<const T*>(V.wall), static_cast<const FT*>(V.Fcol), static_cast<const FT*>(V.Fprev), lane, pl);
+            if (lane == s)
+                last.turn(static_cast<FT*>(V.Fprev) + 3 * row0, (unsigned)(3 * V.Ct * sizeof(FT)), (unsigned)use & 1u, reset);
         }
-        if (lane == 0) {
-            const int issued = it;
-            for (int k = issued > NS ? issued - NS : 0; k < issued; ++k)
-                mbar_wait_bounded(&full[k % NS], (unsigned)(k / NS) & 1u);
-        }
+        if (lane == 0)
+            for (int k = it > NS ? it - NS : 0; k < it; ++k) mbar_wait_bounded(&full[k % NS], (unsigned)(k / NS) & 1u);
+        __syncwarp();
+        if (lane < NS) last.finish(&full[lane], reset);
         return;
     }
     int it = 0, cur_view = -1, vi = 0;
@@ -638,10 +678,9 @@ __global__ void __launch_bounds__(StageLayout<T, kCplDense, COLL>::THREADS, stag
             cur_view = vi;
         }
         const CollideView& V = *cview;
-        consume_tile<T, kCplDense, COLL>(V.d, view_geom(V, NS), tile - V.tile0, stages + s * L::BYTES,
-                                    *reinterpret_cast<const CollideParams<C>*>(V.cp), static_cast<T*>(V.fout),
-                                    static_cast<FT*>(V.Fprev), static_cast<typename Store<T>::U*>(V.u), V.phase, V.celltype, cell,
-                                    &empty[s], lane);
+        consume_cell<T, kCplDense, COLL>(V.d, view_geom(V, NS), tile - V.tile0, stages + s * L::BYTES,
+                                         *reinterpret_cast<const CollideParams<C>*>(V.cp), static_cast<T*>(V.fout),
+                                         static_cast<typename Store<T>::U*>(V.u), V.phase, V.celltype, cell, &empty[s], lane);
     }
 }
 
@@ -662,7 +701,7 @@ int optin_smem() {
 
 template <class T, int CPL, int COLL>
 size_t staged_smem(int nstages) {
-    return 256 + (size_t)nstages * StageLayout<T, CPL, COLL>::BYTES;
+    return 256 + StageLayout<T, CPL, COLL>::RESET + (size_t)nstages * StageLayout<T, CPL, COLL>::BYTES;
 }
 
 // Pipeline depth: the tuning value, else as many stages as fit the resident CTAs of an SM

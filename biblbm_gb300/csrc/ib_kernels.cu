@@ -69,26 +69,6 @@ __device__ __forceinline__ int64_t axis_weights(double x, W* w) {
     return lo;
 }
 
-// Windows of up to four consecutive cells of one x-row of one force component, added with
-// one or two aligned float4 atomics (the field rows start 16-byte aligned: the component
-// stride is a multiple of 128 cells).  Slots outside the window add zero.
-__device__ __forceinline__ float window_select(const float* x, int j, int o, int s) {
-    float r = 0.0f;
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-        if (m < s && j - o == m) r = x[m];
-    return r;
-}
-__device__ __forceinline__ void red_window(float* row, int64_t k0, const float* v, int s) {
-    const int64_t kq = k0 & ~(int64_t)3;
-    const int o = (int)(k0 - kq);
-    float4* q = reinterpret_cast<float4*>(row + kq);
-    atomicAdd(q, make_float4(window_select(v, 0, o, s), window_select(v, 1, o, s), window_select(v, 2, o, s),
-                             window_select(v, 3, o, s)));
-    if (o + s > 4)
-        atomicAdd(q + 1, make_float4(window_select(v, 4, o, s), window_select(v, 5, o, s), window_select(v, 6, o, s),
-                                     window_select(v, 7, o, s)));
-}
 // One cell of the velocity field ((ux, uy, uz, 0) per cell), one or two vector loads.
 template <class C>
 struct U3 {
@@ -182,10 +162,10 @@ __device__ __forceinline__ void tophat_spread(const LatticeDesc& d, const IbDesc
                 const int gz = remap_global(d.pz, d.nz, lo[2] + c, off);
                 if (gz < 0) continue;
                 const FT wt = wxy * w[2][c];
-                FT* q = F + gx + (int64_t)d.nx * (gy + (int64_t)d.ny * gz);
+                FT* q = F + 3 * (gx + (int64_t)d.nx * (gy + (int64_t)d.ny * gz));
                 atomicAdd(q, wt * fv[0]);
-                atomicAdd(q + d.stride, wt * fv[1]);
-                atomicAdd(q + 2 * d.stride, wt * fv[2]);
+                atomicAdd(q + 1, wt * fv[1]);
+                atomicAdd(q + 2, wt * fv[2]);
             }
         }
     }
@@ -281,9 +261,9 @@ __device__ __forceinline__ void interpolate_move_vertex(const IbView& V, int v) 
                     acc[2] += wt * uc.z;
                     if (FOLD && !fd_row) {
                         const int64_t k = col + zo[c];
-                        facc[0] += wt * (__ldg(Fo + k) - body[0]);
-                        facc[1] += wt * (__ldg(Fo + d.stride + k) - body[1]);
-                        facc[2] += wt * (__ldg(Fo + 2 * d.stride + k) - body[2]);
+                        facc[0] += wt * (__ldg(Fo + 3 * k) - body[0]);
+                        facc[1] += wt * (__ldg(Fo + 3 * k + 1) - body[1]);
+                        facc[2] += wt * (__ldg(Fo + 3 * k + 2) - body[2]);
                     }
                 }
             }
@@ -342,11 +322,13 @@ __global__ void __launch_bounds__(128) k_force_clear(LatticeDesc d, IbDesc ib, i
     const int gx0 = remap_global(d.px, d.nx, (int64_t)l.x, off);
     const int gxl = remap_global(d.px, d.nx, (int64_t)l.x + S - 1, off);
     if (gx0 >= 0 && gxl == gx0 + S - 1) {
-        // the row's nodes are contiguous: the float4 words from gx0 down to 4 to gxl
-        const int64_t k0 = (row + gx0) & ~(int64_t)3, k1 = (row + gxl) & ~(int64_t)3;
-        for (int q = 0; q < 3; ++q) {
-            float4* p = reinterpret_cast<float4*>(F + q * d.stride);
-            for (int64_t k = k0; k <= k1; k += 4) p[k >> 2] = make_float4(b[q], b[q], b[q], b[q]);
+        // the row's values are contiguous: the float4 words around them, component (index mod 3)
+        const int64_t k0 = (3 * (row + gx0)) & ~(int64_t)3, k1 = (3 * (row + gxl) + 2) & ~(int64_t)3;
+        int c = (int)(k0 % 3);
+        for (int64_t k = k0; k <= k1; k += 4) {
+            const int c1 = c == 2 ? 0 : c + 1, c2 = c1 == 2 ? 0 : c1 + 1;
+            reinterpret_cast<float4*>(F)[k >> 2] = make_float4(b[c], b[c1], b[c2], b[c]);
+            c = c1;  // 4 values on is one component on
         }
         return;
     }
@@ -354,181 +336,149 @@ __global__ void __launch_bounds__(128) k_force_clear(LatticeDesc d, IbDesc ib, i
     for (int m = 0; m < S; ++m) {
         const int gx = remap_global(d.px, d.nx, (int64_t)l.x + m, off);
         if (gx < 0) continue;
-        for (int q = 0; q < 3; ++q) F[q * d.stride + row + gx] = b[q];
+        for (int q = 0; q < 3; ++q) F[3 * (row + gx) + q] = b[q];
     }
 }
 
 // ---------------------------------------------------------------- spreading
+// The whole share of one vertex by one thread, node by node: with the near-wall blend of a pipe boundary,
+// and with a positive field offset, where the periodic remap leaves nodes out.
 template <class FT, int S>
-__device__ __forceinline__ void spread_vertex(const IbView& V, int v) {
-    static_assert(S == 3 || S == 4, "Roma (3) or Peskin (4) support");
+__device__ __noinline__ void spread_vertex_nodes(const IbView& V, const double* p, const double* force) {
     const LatticeDesc& d = V.d;
     const IbDesc& ib = V.ib;
-    const double* __restrict__ pos = V.pos;
-    const double* __restrict__ force = V.force;
-    FT* __restrict__ F = static_cast<FT*>(V.F);
-    const double p[3] = {pos[3 * v], pos[3 * v + 1], pos[3 * v + 2]};
-    if (!inside_envelope(d, ib.dirac, p)) {
-        if (V.spread_lo) V.spread_lo[v] = make_int4(0, 0, 0, 0);
-        return;
-    }
     const int off = (int)ib.offset;
-    constexpr int s = S;
-    if (V.spread_lo) {
-        constexpr double h = S == 4 ? 2.0 : 1.5;
-        V.spread_lo[v] = make_int4(record_lo(d.px, d.nx, (int64_t)ceil(p[0] - ib.offset - h), off),
-                                   record_lo(d.py, d.ny, (int64_t)ceil(p[1] - ib.offset - h), off),
-                                   record_lo(d.pz, d.nz, (int64_t)ceil(p[2] - ib.offset - h), off), 1);
-    }
-    FT fscale = FT(1);
-    if (ib.has_pipe) {
-        const double wp = pipe_weight(ib, p, S == 4 ? 2.0 : 1.5);
-        if (wp < 1) {  // near the wall: the TopHat takes the share 1 - w of the force
-            FT* Fw = static_cast<FT*>(V.F);
-            const FT ft[3] = {(FT)(force[3 * v] * (wp <= 0 ? 1.0 : 1. - wp)),
-                              (FT)(force[3 * v + 1] * (wp <= 0 ? 1.0 : 1. - wp)),
-                              (FT)(force[3 * v + 2] * (wp <= 0 ? 1.0 : 1. - wp))};
-            tophat_spread<FT>(d, ib, p, ft, Fw);
-            if (wp <= 0) return;
-            fscale = (FT)wp;
-        }
+    FT* F = static_cast<FT*>(V.F);
+    const double wp = ib.has_pipe ? pipe_weight(ib, p, S == 4 ? 2.0 : 1.5) : 1.0;
+    double share = 1.0;
+    if (wp < 1) {  // near the wall: the TopHat takes the share 1 - w of the force
+        const double st = wp <= 0 ? 1.0 : 1. - wp;
+        const FT ft[3] = {(FT)(force[0] * st), (FT)(force[1] * st), (FT)(force[2] * st)};
+        tophat_spread<FT>(d, ib, p, ft, F);
+        if (wp <= 0) return;
+        share = (double)(FT)wp;
     }
     int64_t lo[3];
     FT w[3][4];
     for (int a = 0; a < 3; ++a) lo[a] = axis_weights<FT, S>(p[a] - ib.offset, w[a]);
-    int gx[4], gy[4], gz[4];
-#pragma unroll
-    for (int m = 0; m < s; ++m) {
-        gx[m] = remap_global(d.px, d.nx, lo[0] + m, off);
-        gy[m] = remap_global(d.py, d.ny, lo[1] + m, off);
-        gz[m] = remap_global(d.pz, d.nz, lo[2] + m, off);
-    }
-    int64_t yo[4], zo[4];
-#pragma unroll
-    for (int m = 0; m < s; ++m) {
-        yo[m] = (int64_t)gy[m] * d.nx;
-        zo[m] = (int64_t)gz[m] * d.ny * d.nx;
-    }
-    const FT fv[3] = {fscale == FT(1) ? (FT)force[3 * v] : (FT)(force[3 * v] * (double)fscale),
-                      fscale == FT(1) ? (FT)force[3 * v + 1] : (FT)(force[3 * v + 1] * (double)fscale),
-                      fscale == FT(1) ? (FT)force[3 * v + 2] : (FT)(force[3 * v + 2] * (double)fscale)};
-    if (sizeof(FT) == sizeof(float) && gx[s - 1] == gx[0] + s - 1) {
-        // FP32 field and no periodic wrap along x inside the support: each (y, z) row of
-        // each component receives one window of s values through one or two float4 atomics
-        float* Ff = reinterpret_cast<float*>(F);
-#pragma unroll
-        for (int b = 0; b < s; ++b) {
-            if (gy[b] < 0) continue;
-#pragma unroll
-            for (int c = 0; c < s; ++c) {
-                if (gz[c] < 0) continue;
-                const FT wyz = w[1][b] * w[2][c];
-                const int64_t k0 = gx[0] + yo[b] + zo[c];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    float vals[4];
-                    for (int m = 0; m < 4; ++m) vals[m] = m < s ? (float)((w[0][m] * wyz) * fv[q]) : 0.0f;
-                    red_window(Ff + q * d.stride, k0, vals, s);
-                }
-            }
-        }
-        return;
-    }
-#pragma unroll
-    for (int a = 0; a < s; ++a) {
-        if (gx[a] < 0) continue;
-#pragma unroll
-        for (int b = 0; b < s; ++b) {
-            if (gy[b] < 0) continue;
-            const FT wxy = w[0][a] * w[1][b];
-            FT* col = F + gx[a] + yo[b];
-#pragma unroll
-            for (int c = 0; c < s; ++c) {
-                if (gz[c] < 0) continue;
-                const FT wt = wxy * w[2][c];
-                FT* q = col + zo[c];
-                atomicAdd(q, wt * fv[0]);
-                atomicAdd(q + d.stride, wt * fv[1]);
-                atomicAdd(q + 2 * d.stride, wt * fv[2]);
+    const FT fv[3] = {(FT)(force[0] * share), (FT)(force[1] * share), (FT)(force[2] * share)};
+    for (int a = 0; a < S; ++a) {
+        const int gx = remap_global(d.px, d.nx, lo[0] + a, off);
+        for (int b = 0; b < S; ++b) {
+            const int gy = remap_global(d.py, d.ny, lo[1] + b, off);
+            for (int c = 0; c < S; ++c) {
+                const int gz = remap_global(d.pz, d.nz, lo[2] + c, off);
+                if (gx < 0 || gy < 0 || gz < 0) continue;
+                const FT wt = w[0][a] * w[1][b] * w[2][c];
+                FT* q = F + 3 * (gx + (int64_t)d.nx * (gy + (int64_t)d.ny * gz));
+                for (int k = 0; k < 3; ++k) atomicAdd(q + k, wt * fv[k]);
             }
         }
     }
 }
+
+// Spreading by rows.  A row of a vertex's support, S cells of three components, is one contiguous run
+// of 3 S values of the force field.  The first warp of a CTA prepares 32 vertices in shared memory (the
+// products of x-weight and force, the y and z weights, the row offsets); then all threads take the
+// (vertex, row, word) items in order, neighbouring lanes the neighbouring words of a row.  FP32 fields
+// are added to in aligned float4 words (S = 3: three words cover a run at any offset, S = 4: four; values
+// outside the run add zero), FP64 fields value by value.
+// Bound by the count of its L2 reductions.  With one array per component a vertex had 27 runs of 3 values;
+// with the components of a cell together it has 9 of 9 values, 1.25 lines each: 256,800 vertices (Roma) of
+// the 400-cell channel 79.5 -> 40.9 us, 128,400 (Peskin) of a 240 x 96 x 90 channel 80 -> 39 us.  64 vertices
+// per CTA were slower (40.6 against 36.8 us alone: the adding threads wait longer for the first warp).
+constexpr int kSpreadVerts = 32, kSpreadThreads = 128;
+template <class FT, int S>
+struct SpreadVertex {
+    static constexpr int WORDS = sizeof(FT) == 4 ? (S == 3 ? 3 : 4) : 3 * S;  // per row
+    static constexpr int ITEMS = S * S * WORDS;
+    FT p[3 * S];  // x-weight times force
+    FT wy[S], wz[S];
+    int yo[S], zo[S];  // row offsets in cells of one z-plane / in rows, -1: behind a wall
+    int gx;            // first cell along x (its run wraps if gx + S > nx), -1: nothing to add
+    int inst;          // batch: the lattice
+};
 
 template <class FT, int S, bool BATCH>
-__global__ void __launch_bounds__(128) k_spread(IbView v1, const IbView* __restrict__ views, const int* __restrict__ vinst,
-                                                 int nvert) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= nvert) return;
-    const IbView& V = BATCH ? views[vinst[g]] : v1;
-    spread_vertex<FT, S>(V, BATCH ? g - V.vbase : g);
-}
-
-// Two lanes per vertex (FP32 field, Roma support, no pipe, no wrap along x inside the support):
-// the lanes of a pair add the two float4 words of a window that straddles a 16-byte boundary in
-// the same instruction, so that both words go out in one request when they share a 128-byte line
-// (the spreading is bound by the count of its requests: 0.0950 -> 0.0835 ms on the 400-cell
-// channel against one lane issuing both words).  Same products as spread_vertex.
-__device__ __forceinline__ void spread_vertex_pair(const IbView& V, int v, int half) {
-    const LatticeDesc& d = V.d;
-    const IbDesc& ib = V.ib;
-    const double p[3] = {V.pos[3 * v], V.pos[3 * v + 1], V.pos[3 * v + 2]};
-    if (!inside_envelope(d, ib.dirac, p)) {
-        if (V.spread_lo && half == 0) V.spread_lo[v] = make_int4(0, 0, 0, 0);
-        return;
-    }
-    const int off = (int)ib.offset;
-    int64_t lo[3];
-    float w[3][4];
+__global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const IbView* __restrict__ views,
+                                                                const int* __restrict__ vinst, int nvert) {
+    using SV = SpreadVertex<FT, S>;
+    __shared__ SV sv[kSpreadVerts];
+    const int g0 = blockIdx.x * kSpreadVerts;
+    if (threadIdx.x < kSpreadVerts) {
+        SV& s = sv[threadIdx.x];
+        const int g = g0 + threadIdx.x;
+        s.gx = -1;
+        if (g < nvert) {
+            s.inst = BATCH ? vinst[g] : 0;
+            const IbView& V = BATCH ? views[s.inst] : v1;
+            const LatticeDesc& d = V.d;
+            const int v = BATCH ? g - V.vbase : g;
+            const double p[3] = {V.pos[3 * v], V.pos[3 * v + 1], V.pos[3 * v + 2]};
+            const double force[3] = {V.force[3 * v], V.force[3 * v + 1], V.force[3 * v + 2]};
+            const bool inside = inside_envelope(d, V.ib.dirac, p);
+            const int off = (int)V.ib.offset;
+            if (inside) {
+                if (V.ib.has_pipe || off > 0) {
+                    spread_vertex_nodes<FT, S>(V, p, force);
+                } else {
+                    FT wx[S];
+                    const int64_t lx = axis_weights<FT, S>(p[0] - V.ib.offset, wx);
+                    const int64_t ly = axis_weights<FT, S>(p[1] - V.ib.offset, s.wy);
+                    const int64_t lz = axis_weights<FT, S>(p[2] - V.ib.offset, s.wz);
+                    s.gx = remap_global(d.px, d.nx, lx, off);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) lo[a] = axis_weights<float, 3>(p[a] - ib.offset, w[a]);
-    int gx[3], gy[3], gz[3];
+                    for (int m = 0; m < S; ++m) {
+                        s.yo[m] = remap_global(d.py, d.ny, ly + m, off);
+                        s.zo[m] = remap_global(d.pz, d.nz, lz + m, off);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        gx[m] = remap_global(d.px, d.nx, lo[0] + m, off);
-        gy[m] = remap_global(d.py, d.ny, lo[1] + m, off);
-        gz[m] = remap_global(d.pz, d.nz, lo[2] + m, off);
-    }
-    if (ib.has_pipe || gx[2] != gx[0] + 2) {
-        if (half == 0) spread_vertex<float, 3>(V, v);
-        return;
-    }
-    if (V.spread_lo && half == 0)
-        V.spread_lo[v] = make_int4(record_lo(d.px, d.nx, (int64_t)ceil(p[0] - ib.offset - 1.5), off),
-                                   record_lo(d.py, d.ny, (int64_t)ceil(p[1] - ib.offset - 1.5), off),
-                                   record_lo(d.pz, d.nz, (int64_t)ceil(p[2] - ib.offset - 1.5), off), 1);
-    const float fv[3] = {(float)V.force[3 * v], (float)V.force[3 * v + 1], (float)V.force[3 * v + 2]};
-    float* F = static_cast<float*>(V.F);
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-        if (gy[b] < 0) continue;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            if (gz[c] < 0) continue;
-            const float wyz = w[1][b] * w[2][c];
-            const int64_t k0 = gx[0] + (int64_t)gy[b] * d.nx + (int64_t)gz[c] * d.ny * d.nx;
-            const int64_t kq = k0 & ~(int64_t)3;
-            const int o = (int)(k0 - kq);
-            const bool go = half == 0 || o + 3 > 4;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                float vals[4];
-#pragma unroll
-                for (int m = 0; m < 4; ++m) vals[m] = m < 3 ? (float)((w[0][m] * wyz) * fv[q]) : 0.0f;
-                const int j = half * 4;
-                const float4 val = make_float4(window_select(vals, j, o, 3), window_select(vals, j + 1, o, 3),
-                                               window_select(vals, j + 2, o, 3), window_select(vals, j + 3, o, 3));
-                if (go) atomicAdd(reinterpret_cast<float4*>(F + q * d.stride + kq) + half, val);
+                        for (int q = 0; q < 3; ++q) s.p[3 * m + q] = wx[m] * (FT)force[q];
+                    }
+                }
+            }
+            if (V.spread_lo) {
+                constexpr double h = S == 4 ? 2.0 : 1.5;
+                V.spread_lo[v] = inside ? make_int4(record_lo(d.px, d.nx, (int64_t)ceil(p[0] - V.ib.offset - h), off),
+                                                    record_lo(d.py, d.ny, (int64_t)ceil(p[1] - V.ib.offset - h), off),
+                                                    record_lo(d.pz, d.nz, (int64_t)ceil(p[2] - V.ib.offset - h), off), 1)
+                                        : make_int4(0, 0, 0, 0);
             }
         }
     }
-}
-
-__global__ void __launch_bounds__(128) k_spread_pairs(IbView v1, int nvert) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const int v = g >> 1;
-    if (v >= nvert) return;
-    spread_vertex_pair(v1, v, g & 1);
+    __syncthreads();
+    for (int it = threadIdx.x; it < kSpreadVerts * SV::ITEMS; it += kSpreadThreads) {
+        const int t = it / SV::ITEMS, r = it - t * SV::ITEMS, row = r / SV::WORDS, j = r - row * SV::WORDS;
+        const SV& s = sv[t];
+        if (s.gx < 0) continue;
+        const int y = s.yo[row / S], z = s.zo[row % S];
+        if (y < 0 || z < 0) continue;
+        const IbView& V = BATCH ? views[s.inst] : v1;
+        const int nx = V.d.nx;
+        const FT wyz = s.wy[row / S] * s.wz[row % S];
+        const int64_t cell0 = (int64_t)nx * (y + (int64_t)V.d.ny * z);
+        FT* F = static_cast<FT*>(V.F);
+        if (s.gx + S <= nx) {
+            const int64_t e0 = 3 * (cell0 + s.gx);
+            if constexpr (sizeof(FT) == 4) {
+                const int o = (int)(e0 & 3);
+                float v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int e = 4 * j + k - o;
+                    v[k] = e >= 0 && e < 3 * S ? s.p[e] * wyz : 0.0f;
+                }
+                if (4 * j - o < 3 * S) atomicAdd(reinterpret_cast<float4*>(F + (e0 - o)) + j, make_float4(v[0], v[1], v[2], v[3]));
+            } else {
+                atomicAdd(F + e0 + j, s.p[j] * wyz);
+            }
+        } else {  // the run wraps periodically along x: value by value
+            const int e0 = sizeof(FT) == 4 ? 4 * j : j, e1 = min(sizeof(FT) == 4 ? e0 + 4 : e0 + 1, 3 * S);
+            for (int e = e0; e < e1; ++e) {
+                const int x = (s.gx + e / 3) % nx;
+                atomicAdd(F + 3 * (cell0 + x) + e % 3, s.p[e] * wyz);
+            }
+        }
+    }
 }
 
 // Deterministic spreading.  Every (vertex, stencil node) pair becomes an entry keyed by its
@@ -574,14 +524,15 @@ template <class FT>
 __global__ void __launch_bounds__(128) k_spread_reduce(LatticeDesc d, IbDesc ib, int64_t nentries,
                                                         const uint32_t* __restrict__ keys, const uint32_t* __restrict__ ids,
                                                         const double* __restrict__ pos, const double* __restrict__ force,
-                                                        FT* __restrict__ F) {
+                                                        FT* __restrict__ F, int64_t cell, int64_t comp) {
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= nentries) return;
     const uint32_t key = keys[p];
     if (key == (uint32_t)d.n || (p > 0 && keys[p - 1] == key)) return;  // not the head of a cell's run
     const int s = support(ib.dirac), s3 = s * s * s;
     const double h = half_support(ib.dirac);
-    FT acc[3] = {F[key], F[d.stride + key], F[2 * d.stride + key]};
+    FT* out = F + cell * key;  // component q of a cell at out[q * comp]
+    FT acc[3] = {out[0], out[comp], out[2 * comp]};
     for (int64_t q = p; q < nentries && keys[q] == key; ++q) {
         const uint32_t e = ids[q];
         const int v = (int)(e / s3), m = (int)(e % s3);
@@ -598,9 +549,9 @@ __global__ void __launch_bounds__(128) k_spread_reduce(LatticeDesc d, IbDesc ib,
         acc[1] += wt * (FT)force[3 * v + 1];
         acc[2] += wt * (FT)force[3 * v + 2];
     }
-    F[key] = acc[0];
-    F[d.stride + key] = acc[1];
-    F[2 * d.stride + key] = acc[2];
+    out[0] = acc[0];
+    out[comp] = acc[1];
+    out[2 * comp] = acc[2];
 }
 
 // ---------------------------------------------------------------- interaction forces
@@ -1541,9 +1492,9 @@ cudaError_t launch_spread_sorted(const LatticeDesc& d, const IbDesc& ib, bool f6
     if (e != cudaSuccess) return e;
     const unsigned ge = (unsigned)((ne + 127) / 128);
     if (f64_field)
-        k_spread_reduce<double><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (double*)field);
+        k_spread_reduce<double><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (double*)field, 1, d.stride);
     else
-        k_spread_reduce<float><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (float*)field);
+        k_spread_reduce<float><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (float*)field, 1, d.stride);
     return cudaGetLastError();
 }
 
@@ -1602,15 +1553,14 @@ void interpolate_any(int storage, int dirac, const IbView& v1, const IbView* vie
 template <bool BATCH>
 void spread_any(int storage, int dirac, const IbView& v1, const IbView* views, const int* vinst, int nvert,
                 cudaStream_t s) {
-    const unsigned g = (nvert + 127) / 128;
+    const unsigned g = (nvert + kSpreadVerts - 1) / kSpreadVerts;
     const bool peskin = dirac == BIB_DIRAC_PESKIN;
     if (storage == BIB_STORAGE_F64) {
-        if (peskin) k_spread<double, 4, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
-        else k_spread<double, 3, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
+        if (peskin) k_spread_rows<double, 4, BATCH><<<g, kSpreadThreads, 0, s>>>(v1, views, vinst, nvert);
+        else k_spread_rows<double, 3, BATCH><<<g, kSpreadThreads, 0, s>>>(v1, views, vinst, nvert);
     } else {
-        if (peskin) k_spread<float, 4, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
-        else if (!BATCH) k_spread_pairs<<<(unsigned)((2LL * nvert + 127) / 128), 128, 0, s>>>(v1, nvert);
-        else k_spread<float, 3, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
+        if (peskin) k_spread_rows<float, 4, BATCH><<<g, kSpreadThreads, 0, s>>>(v1, views, vinst, nvert);
+        else k_spread_rows<float, 3, BATCH><<<g, kSpreadThreads, 0, s>>>(v1, views, vinst, nvert);
     }
 }
 
@@ -1788,9 +1738,9 @@ void launch_spread(const Lattice& L, int fbuf, cudaStream_t s, bool record) {
                                         (int)ne, 0, key_bits(L.d.n), s);
         const unsigned ge = (unsigned)((ne + 127) / 128);
         if (L.storage == BIB_STORAGE_F64)
-            k_spread_reduce<double><<<ge, 128, 0, s>>>(L.d, L.ib, ne, L.sort_keys[1], L.sort_ids[1], pos, L.force, (double*)L.F[fbuf]);
+            k_spread_reduce<double><<<ge, 128, 0, s>>>(L.d, L.ib, ne, L.sort_keys[1], L.sort_ids[1], pos, L.force, (double*)L.F[fbuf], 3, 1);
         else
-            k_spread_reduce<float><<<ge, 128, 0, s>>>(L.d, L.ib, ne, L.sort_keys[1], L.sort_ids[1], pos, L.force, (float*)L.F[fbuf]);
+            k_spread_reduce<float><<<ge, 128, 0, s>>>(L.d, L.ib, ne, L.sort_keys[1], L.sort_ids[1], pos, L.force, (float*)L.F[fbuf], 3, 1);
         return;
     }
     IbView v = single_view(L, fbuf);

@@ -171,6 +171,21 @@ __device__ __forceinline__ void store2<double>(double* p, double a, double b) {
     *reinterpret_cast<double2*>(p) = make_double2(a, b);
 }
 
+// The force field keeps the three components of a cell together, F[3 k + a]: a row of a vertex's
+// support is one contiguous run.  Two neighbouring cells (k even) as three vector accesses.
+template <class FT>
+__device__ __forceinline__ void load_force2(const FT* F, int64_t k, FT* a, FT* b) {
+    load2<FT>(F + 3 * k, a[0], a[1]);
+    load2<FT>(F + 3 * k + 2, a[2], b[0]);
+    load2<FT>(F + 3 * k + 4, b[1], b[2]);
+}
+template <class FT>
+__device__ __forceinline__ void store_force2(FT* F, int64_t k, const double* v) {
+    store2<FT>(F + 3 * k, (FT)v[0], (FT)v[1]);
+    store2<FT>(F + 3 * k + 2, (FT)v[2], (FT)v[0]);
+    store2<FT>(F + 3 * k + 4, (FT)v[1], (FT)v[2]);
+}
+
 // ---------------------------------------------------------------- delta-function supports
 __device__ __forceinline__ double half_support(int dirac) { return dirac == BIB_DIRAC_PESKIN ? 2.0 : 1.5; }
 __device__ __forceinline__ int support(int dirac) { return dirac == BIB_DIRAC_PESKIN ? 4 : 3; }

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) k_collide_stream(LatticeDesc d, const T* 
         if (COUPLED) {
             store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
             if (Fprev)
-                for (int c = 0; c < 3; ++c) Fprev[c * d.stride + k] = (FT)d.body[c];
+                for (int c = 0; c < 3; ++c) Fprev[3 * k + c] = (FT)d.body[c];
         }
         if (ctype == BIB_CELL_BOUNCE_BACK) bounce_back_cell(f);
 #pragma unroll
@@ -95,20 +95,16 @@ __global__ void __launch_bounds__(256) k_collide_stream(LatticeDesc d, const T* 
         } else {
             C Fp[3] = {(C)d.body[0], (C)d.body[1], (C)d.body[2]};
             if (Fprev) {
-                Fp[0] = (C)Fprev[k];
-                Fp[1] = (C)Fprev[d.stride + k];
-                Fp[2] = (C)Fprev[2 * d.stride + k];
+                for (int c = 0; c < 3; ++c) Fp[c] = (C)Fprev[3 * k + c];
             }
             velocity_with_force(f, Fp, u);
         }
         store_u<UT>(u_out, k, (UT)u[0], (UT)u[1], (UT)u[2]);
         if (Fprev) {
-            Fprev[k] = (FT)d.body[0];
-            Fprev[d.stride + k] = (FT)d.body[1];
-            Fprev[2 * d.stride + k] = (FT)d.body[2];
+            for (int c = 0; c < 3; ++c) Fprev[3 * k + c] = (FT)d.body[c];
         }
     }
-    C Fc[3] = {(C)__ldg(Fcol + k), (C)__ldg(Fcol + d.stride + k), (C)__ldg(Fcol + 2 * d.stride + k)};
+    C Fc[3] = {(C)__ldg(Fcol + 3 * k), (C)__ldg(Fcol + 3 * k + 1), (C)__ldg(Fcol + 3 * k + 2)};
     if (coll == BIB_COLLISION_BGK_GUO_VOF) {
         C omega = (C)d.omega_c0;
         if (d.use_phase && phase[k]) omega = (C)d.omega_c1;
@@ -199,10 +195,10 @@ __global__ void __launch_bounds__(256) k_collide_stream_rows(LatticeDesc d, cons
         }
     }
     if (active) {
-        for (int c = 0; c < 3; ++c) load2<FT>(Fcol + c * d.stride + k0, fca[c], fcb[c]);
+        load_force2<FT>(Fcol, k0, fca, fcb);
         if (COUPLED && !wallrow) {
             if (Fprev) {
-                for (int c = 0; c < 3; ++c) load2<FT>(Fprev + c * d.stride + k0, fpa[c], fpb[c]);
+                load_force2<FT>(Fprev, k0, fpa, fpb);
             } else {  // sparse force reset: the velocity field takes the body force only
                 for (int c = 0; c < 3; ++c) fpa[c] = fpb[c] = (FT)d.body[c];
             }
@@ -259,7 +255,7 @@ __global__ void __launch_bounds__(256) k_collide_stream_rows(LatticeDesc d, cons
         store_u<UT>(u_out, k0, (UT)u0[0], (UT)u0[1], (UT)u0[2]);
         store_u<UT>(u_out, k0 + 1, (UT)u1[0], (UT)u1[1], (UT)u1[2]);
         if (Fprev)
-            for (int c = 0; c < 3; ++c) store2<FT>(Fprev + c * d.stride + k0, (FT)d.body[c], (FT)d.body[c]);
+            store_force2<FT>(Fprev, k0, d.body);
     }
     C Fa[3] = {(C)fca[0], (C)fca[1], (C)fca[2]}, Fb[3] = {(C)fcb[0], (C)fcb[1], (C)fcb[2]};
     C om0 = (C)d.omega, om1 = (C)d.omega, omm = C(0);
@@ -380,8 +376,8 @@ __device__ __forceinline__ void fd_wall_cell(const LatticeDesc& d, const T* __re
         fc[i] = s >= 0 ? Store<T>::load(f + i * d.stride + s, d.inv_scale) : C(0);  // unknown ones are not used
     }
     gather<T>(d, f, wall, x, y1, z, k1, f1);
-    const C Fy = (C)F[d.stride + k];
-    C F1[3] = {(C)F[k1], (C)F[d.stride + k1], (C)F[2 * d.stride + k1]};
+    const C Fy = (C)F[3 * k + 1];
+    C F1[3] = {(C)F[3 * k1], (C)F[3 * k1 + 1], (C)F[3 * k1 + 2]};
     const C uw[3] = {(C)d.wall_u[side][0], (C)d.wall_u[side][1], (C)d.wall_u[side][2]};
     C rhoOnWall = 0, rhoNormal = 0;
 #pragma unroll
@@ -441,7 +437,7 @@ __device__ __forceinline__ void cell_velocity(const LatticeDesc& d, const T* __r
     } else {
         C fc[Q];
         gather<T>(d, f, wall, x, y, z, k, fc);
-        C Fc[3] = {(C)F[k], (C)F[d.stride + k], (C)F[2 * d.stride + k]};
+        C Fc[3] = {(C)F[3 * k], (C)F[3 * k + 1], (C)F[3 * k + 2]};
         velocity_with_force(fc, Fc, uc);
     }
 }
@@ -599,7 +595,7 @@ __global__ void __launch_bounds__(kWireX * kWireZ) k_import_aos(LatticeDesc d, T
 #pragma unroll
     for (int i = 0; i < Q; ++i) scatter_canonical<T>(d, f, wall, i, x, t.y, z, k, c[i]);
     if (PER == Q + 4) {
-        for (int a = 0; a < 3; ++a) F[a * d.stride + k] = (typename Store<T>::F)c[Q + a];
+        for (int a = 0; a < 3; ++a) F[3 * k + a] = (typename Store<T>::F)c[Q + a];
         if (phase) phase[k] = c[Q + 3] >= 0.5 ? 1 : 0;
     }
 }
@@ -623,7 +619,7 @@ __global__ void __launch_bounds__(kWireX * kWireZ) k_export_aos(LatticeDesc d, c
 #pragma unroll
         for (int i = 0; i < Q; ++i) c[i] = (double)fc[i];
         if (PER == Q + 4) {
-            for (int a = 0; a < 3; ++a) c[Q + a] = (double)F[a * d.stride + k];
+            for (int a = 0; a < 3; ++a) c[Q + a] = (double)F[3 * k + a];
             c[Q + 3] = phase && phase[k] ? 1.0 : 0.0;
         }
     }
@@ -642,23 +638,21 @@ template <class FT>
 __global__ void k_force_import(LatticeDesc d, FT* __restrict__ F, const double* __restrict__ src) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= d.n) return;
-    for (int a = 0; a < 3; ++a) F[a * d.stride + k] = (FT)src[a * d.n + k];
+    for (int a = 0; a < 3; ++a) F[3 * k + a] = (FT)src[a * d.n + k];
 }
 
 template <class FT>
 __global__ void k_force_export(LatticeDesc d, const FT* __restrict__ F, double* __restrict__ dst) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= d.n) return;
-    for (int a = 0; a < 3; ++a) dst[a * d.n + k] = (double)F[a * d.stride + k];
+    for (int a = 0; a < 3; ++a) dst[a * d.n + k] = (double)F[3 * k + a];
 }
 
 template <class FT>
 __global__ void k_force_fill(LatticeDesc d, FT* __restrict__ F) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= d.stride) return;
-    F[k] = (FT)d.body[0];
-    F[d.stride + k] = (FT)d.body[1];
-    F[2 * d.stride + k] = (FT)d.body[2];
+    for (int a = 0; a < 3; ++a) F[3 * k + a] = (FT)d.body[a];
 }
 
 __global__ void k_phase_import(LatticeDesc d, uint8_t* __restrict__ ph, const double* __restrict__ src) {
