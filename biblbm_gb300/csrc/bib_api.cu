@@ -393,6 +393,8 @@ void free_particles(Lattice& L) {
     cudaFree(L.sort_temp);
     L.sort_temp = nullptr;
     L.sort_temp_bytes = 0;
+    cudaFree(L.spread_rec);
+    L.spread_rec = nullptr;
     for (int k = 0; k < 2; ++k) {
         cudaFree(L.pgrid.keys[k]);
         cudaFree(L.pgrid.ids[k]);
@@ -497,6 +499,7 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
             BIB_ALLOC(c, (void**)&L.sort_keys[k], ne * sizeof(uint32_t));
             BIB_ALLOC(c, (void**)&L.sort_ids[k], ne * sizeof(uint32_t));
         }
+        BIB_ALLOC(c, &L.spread_rec, (size_t)L.nvert * 3 * (sup + 1) * force_bytes(L.storage));
         L.sort_temp_bytes = spread_sort_temp_bytes(ne);
         BIB_ALLOC(c, &L.sort_temp, L.sort_temp_bytes);
     }

