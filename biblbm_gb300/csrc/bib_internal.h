@@ -365,6 +365,8 @@ enum class Coupling {
 void launch_collide_stream(const Lattice& L, Coupling mode, cudaStream_t s);
 // shared-memory staged variant (collide_staged.cu); false if the lattice shape does not fit it
 bool launch_collide_stream_staged(const Lattice& L, Coupling mode, cudaStream_t s);
+// linear tiles, for rows the row tiles do not take (FP16 / FP32); false: not for this lattice
+bool launch_collide_stream_linear(const Lattice& L, Coupling mode, cudaStream_t s);
 bool collide_staged_fits(const Lattice& L);  // both step kinds fit the staged kernel
 void launch_fd_walls(const Lattice& L, int buf, int fbuf, cudaStream_t s);
 void launch_velocity_field(const Lattice& L, cudaStream_t s);  // u from the current state and F[fe]

@@ -15,187 +15,11 @@
 // Per lattice update the kernel moves exactly the algorithmic bytes: 19 populations read
 // and written once, the spread force read, the velocity field written (coupled step) and, with
 // the dense coupling only, the previous force read and reset to the body force.
-#include <algorithm>
-#include <cstring>
-#include <mutex>
-#include <unordered_map>
-
-#include "lattice_common.cuh"
+#include "staged_common.cuh"
 
 namespace bib {
 
 namespace {
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-// One potentially blocking test of a barrier phase: a thread whose phase is not complete is
-// suspended until it completes or about kSuspendNs pass (the suspend-time hint), so that waiting
-// warps do not spin through issue slots the working warps need.
-constexpr uint32_t kSuspendNs = 20000;
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity), "r"(kSuspendNs)
-        : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-// Bounded wait for one phase of a stage barrier: gives up after limit_ns (2 s by default; a
-// copy of a tile takes microseconds) or 2^26 polls, so that a lost completion can never hang
-// the GPU.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity, uint64_t limit_ns = kDefaultWaitNs) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
-    for (uint32_t it = 0; it < (1u << 26); ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 255u) == 0 && global_ns() - t0 > limit_ns) break;
-    }
-    return false;
-}
-// Shared -> global bulk copy, completed by the thread's bulk group; dst, src and bytes are multiples of 16.
-__device__ __forceinline__ void bulk_copy_s2g(void* dst, const void* src, unsigned bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(dst),
-                 "r"(smem_addr(src)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// Global -> shared bulk copy; dst, src and bytes are multiples of 16.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
-// Values of a staged population row as the compute type, in storage units (FP16 keeps the
-// scaled f-bar; the scale is folded into the collision).
-template <class T>
-struct Staged;
-template <>
-struct Staged<__half> {
-    static __device__ __forceinline__ float one(const __half* p) { return __half2float(*p); }
-    static __device__ __forceinline__ void two(const __half* p, float& a, float& b) {
-        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(p));
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store(__half* p, float a, float b) {
-        *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
-    }
-    static __device__ __forceinline__ void put(__half* p, float a) { *p = __float2half_rn(a); }
-};
-template <>
-struct Staged<float> {
-    static __device__ __forceinline__ float one(const float* p) { return *p; }
-    static __device__ __forceinline__ void two(const float* p, float& a, float& b) {
-        const float2 v = *reinterpret_cast<const float2*>(p);
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store(float* p, float a, float b) {
-        *reinterpret_cast<float2*>(p) = make_float2(a, b);
-    }
-    static __device__ __forceinline__ void put(float* p, float a) { *p = a; }
-};
-template <>
-struct Staged<double> {
-    static __device__ __forceinline__ double one(const double* p) { return *p; }
-    static __device__ __forceinline__ void two(const double* p, double& a, double& b) {
-        const double2 v = *reinterpret_cast<const double2*>(p);
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store(double* p, double a, double b) {
-        *reinterpret_cast<double2*>(p) = make_double2(a, b);
-    }
-    static __device__ __forceinline__ void put(double* p, double a) { *p = a; }
-};
-
-// The 19 post-collision values of one cell to their arrays (stride apart); FP16 converts two
-// values per instruction (same rounding; measured on the 400-cell channel: the collide-and-stream
-// 0.1763 -> 0.1748 ms, the lattice-only TRT kernel 56,680 -> 57,370 MLUPS at 384^3).
-template <class T, class C>
-__device__ __forceinline__ void store_cell(T* o, int64_t stride, const C* f) {
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        Staged<T>::put(o, f[i]);
-        o += stride;
-    }
-}
-template <>
-__device__ __forceinline__ void store_cell<__half, float>(__half* o, int64_t stride, const float* f) {
-#pragma unroll
-    for (int i = 0; i + 1 < Q; i += 2) {
-        const __half2 h = __floats2half2_rn(f[i], f[i + 1]);
-        o[0] = __low2half(h);
-        o[stride] = __high2half(h);
-        o += 2 * stride;
-    }
-    *o = __float2half_rn(f[Q - 1]);
-}
-
-// Collision of one cell in storage units: the compact pairwise forms (BGK + Guo, BGK, TRT) in the
-// compute type.  With u non-null the velocity j/rho + Fp/2 of the incoming state is returned.
-template <class C, int COLL>
-__device__ __forceinline__ void staged_relax(C* f, const C* F, C om, C omm, C S, const CellMoments<C>& m) {
-    if constexpr (COLL == BIB_COLLISION_TRT) {
-        const C Fm[3] = {omm, C(0), C(0)};  // the TRT branch takes omega_minus in F[0]
-        relax_compact<C, COLL>(f, Fm, om, S, m);
-    } else {
-        relax_compact<C, COLL>(f, F, om, S, m);
-    }
-}
-
-// Tile pitch in cells: the shared-memory row of one population holds up to TILE cells, so
-// every staged address is a per-thread base plus a compile-time offset.
-template <class T>
-struct TileOf {
-    static constexpr int value = sizeof(T) == 8 ? 256 : 512;
-};
-
-// Coupling of a staged launch: lattice only; dense (the velocity field with the previous force,
-// which is read and reset to the body force); sparse (the velocity field with the body force,
-// the previous force left to the sparse reset).
-constexpr int kCplNone = 0, kCplDense = 1, kCplSparse = 2;
-
-// Stage layout (compile-time): 19 population rows, the collision force (BGK + Guo) and,
-// for the dense coupled step, the previous force (three values per cell), each TILE cells long.
-template <class T, int CPL, int COLL>
-struct StageLayout {
-    using FT = typename Store<T>::F;
-    static constexpr int TILE = TileOf<T>::value;
-    static constexpr int CONSUMERS = TILE / 32;  // consumer warps: one cell per thread and tile
-    static constexpr int THREADS = 32 * (CONSUMERS + 1);
-    static constexpr bool NEED_FCOL = COLL == BIB_COLLISION_BGK_GUO_VOF;
-    static constexpr unsigned POP = TILE * sizeof(T);
-    static constexpr unsigned FRC = TILE * sizeof(FT);
-    static constexpr unsigned OFF_FCOL = Q * POP;
-    static constexpr unsigned OFF_FPREV = OFF_FCOL + (NEED_FCOL ? 3 * FRC : 0);
-    static constexpr unsigned BYTES = ((OFF_FPREV + (CPL == kCplDense ? 3 * FRC : 0)) + 127) / 128 * 128;
-    // dense coupling: one tile of the body force in front of the stages, the source of the reset
-    static constexpr unsigned RESET = CPL == kCplDense ? 3 * FRC : 0;
-};
-
-constexpr int kMaxStages = 8;
 
 struct StagedGeom {
     int R;            // rows per tile (divides ny)
@@ -247,11 +71,6 @@ __device__ __forceinline__ PopLane pop_lane(int lane) {
 // stage waits for, and from the tile's number: with the run kept per stage in lane registers the FP16
 // kernel at its 56 registers took 168.5 us for 512 x 128 x 128 cells, so 160.8 (162.7 with one force
 // array per component and the reset stored by the consumers).
-template <class FT>
-__device__ __forceinline__ void fill_reset(FT* reset, const double* body, int n, int t, int nthreads) {
-    for (int k = t; k < n; k += nthreads) reset[k] = (FT)body[k % 3];
-    proxy_fence();
-}
 template <class FT>
 __device__ __forceinline__ void reset_tile(const LatticeDesc& d, const StagedGeom& g, int64_t tile, FT* Fprev, const FT* reset) {
     bulk_copy_s2g(Fprev + 3 * tile_ref(d, g, tile).row0, reset, (unsigned)(3 * g.Ct * sizeof(FT)));
@@ -356,45 +175,6 @@ __device__ __forceinline__ TileCell tile_cell(const LatticeDesc& d, int Ct, int 
     return c;
 }
 
-// Collision and stores of one cell k of row y whose gathered populations are in f: a
-// BounceBack / NoDynamics node is not collided (zero velocity), every other node collides with
-// the force F; the coupled step writes its velocity (j/rho + Fp/2, or the wall's on
-// finite-difference wall rows).
-template <class T, int CPL, int COLL>
-__device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideParams<typename Store<T>::C>& cp,
-                                            T* __restrict__ fout, typename Store<T>::U* __restrict__ u_out, const uint8_t* __restrict__ phase,
-                                            const uint8_t* __restrict__ celltype, int64_t k, int y, bool fd,
-                                            typename Store<T>::C* f, const typename Store<T>::C* F,
-                                            const typename Store<T>::C* Fp) {
-    using C = typename Store<T>::C;
-    using UT = typename Store<T>::U;
-    const int ctype = d.has_types ? celltype[k] : BIB_CELL_FLUID;
-    if (ctype != BIB_CELL_FLUID) {  // BounceBack / NoDynamics node: no collision, zero velocity
-        if (CPL != kCplNone) store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
-        if (ctype == BIB_CELL_BOUNCE_BACK) bounce_back_cell(f);
-        store_cell<T, C>(fout + k, d.stride, f);
-        return;
-    }
-    C om = cp.om0;
-    if (COLL == BIB_COLLISION_BGK_GUO_VOF && d.use_phase && phase[k]) om = cp.om1;
-    const CellMoments<C> m = moments_compact<C>(f, cp.invS);
-    if (CPL != kCplNone) {
-        // the velocity is stored before the relaxation, so that the previous force is dead while
-        // the relaxation runs
-        C u[3];
-        if (fd) {
-            const int side = y == 0 ? 0 : 1;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) u[q] = cp.wall_u[side][q];
-        } else {
-            velocity_compact<C>(m, Fp, u);
-        }
-        store_u_from<UT, C>(u_out, k, u[0], u[1], u[2]);
-    }
-    staged_relax<C, COLL>(f, F, om, cp.omm, cp.S, m);
-    store_cell<T, C>(fout + k, d.stride, f);
-}
-
 // One cell per consumer thread: read the thread's cell from the stage, release the stage,
 // collide and store.
 template <class T, int CPL, int COLL>
@@ -456,13 +236,6 @@ __device__ __forceinline__ void consume_cell(const LatticeDesc& d, const StagedG
 // landed, empty[s] when every consumer warp is done reading it.  Consumers never wait for
 // each other, and the producer refills a stage as soon as it is released, so up to NS - 1
 // tiles of loads are in flight per CTA.  Results go straight from registers to HBM.
-// Resident CTAs per SM the kernel is built for: FP16 needs two (32 consumer warps) to hide
-// the latency of its arithmetic; FP32 and FP64 run one CTA with a deeper pipeline.
-template <class T>
-constexpr int staged_ctas_per_sm() {
-    return sizeof(T) == 2 ? 2 : 1;
-}
-
 template <class T, int CPL, int COLL>
 __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_ctas_per_sm<T>())
     k_collide_stream_staged(
@@ -692,13 +465,6 @@ int staged_rows(const LatticeDesc& d, int target) {
     return R;
 }
 
-int optin_smem() {
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    return optin;
-}
-
 template <class T, int CPL, int COLL>
 size_t staged_smem(int nstages) {
     return 256 + StageLayout<T, CPL, COLL>::RESET + (size_t)nstages * StageLayout<T, CPL, COLL>::BYTES;
@@ -714,29 +480,6 @@ int staged_stages(const Lattice& L) {
     for (int ns = 2; ns <= kMaxStages; ++ns)
         if (staged_smem<T, CPL, COLL>(ns) <= limit) best = ns;
     return best;
-}
-
-template <class C>
-CollideParams<C> collide_params(const LatticeDesc& d, int storage) {
-    CollideParams<C> cp{};
-    const bool phase_omega = d.collision == BIB_COLLISION_BGK_GUO_VOF;
-    cp.om0 = (C)(phase_omega ? d.omega_c0 : d.omega);
-    cp.om1 = (C)(phase_omega ? d.omega_c1 : d.omega);
-    cp.omm = (C)(1.0 / (d.trt_magic / (1.0 / d.omega - 0.5) + 0.5));
-    const double S = storage == BIB_STORAGE_F16 ? (double)d.scale : 1.0;
-    cp.S = (C)S;
-    cp.invS = (C)(storage == BIB_STORAGE_F16 ? (double)d.inv_scale : 1.0);
-    for (int q = 0; q < 3; ++q) {
-        cp.body[q] = (C)d.body[q];
-        cp.wall_u[0][q] = (C)d.wall_u[0][q];
-        cp.wall_u[1][q] = (C)d.wall_u[1][q];
-    }
-    for (int face = 0; face < 4; ++face)
-        for (int i = 0; i < Q; ++i) {
-            const double cu = cx(i) * d.wall_u[face][0] + cy(i) * d.wall_u[face][1] + cz(i) * d.wall_u[face][2];
-            cp.mw[face][i] = (C)((C)(6.0 * weight<double>(i) * cu) * (C)S);
-        }
-    return cp;
 }
 
 template <class T, int CPL, int COLL>

@@ -680,7 +680,8 @@ inline unsigned lin_grid(int64_t n, int b) { return (unsigned)((n + b - 1) / b);
 template <class T>
 void collide_stream_t(const Lattice& L, Coupling mode, cudaStream_t s) {
     using FT = typename Store<T>::F;
-    if (L.collide_kernel != BIB_KERNEL_ROWS && launch_collide_stream_staged(L, mode, s)) return;
+    if (L.collide_kernel != BIB_KERNEL_ROWS && (launch_collide_stream_staged(L, mode, s) || launch_collide_stream_linear(L, mode, s)))
+        return;
     const bool coupled = mode != Coupling::kNone;
     // the previous force, read for the velocity and reset (dense coupling only)
     FT* Fprev = mode == Coupling::kDense ? (FT*)L.F[L.fe] : nullptr;
