@@ -195,18 +195,43 @@ __device__ __forceinline__ void pipe_move(const IbDesc& ib, const double* old, c
     for (int k = 0; k < 3; ++k) x[k] += (v[k] - s2 * n[k]) * (1. - t);
 }
 
+// Velocity and move of a vertex in a pipe from the interpolated velocity u3: near the wall blended with
+// (or switched to) the TopHat kernel, and a step that crosses the wall reflected.
+template <class UT, int S, class C>
+__device__ __noinline__ void move_near_pipe(const IbView& V, int v, const C* u3) {
+    const double p[3] = {V.pos[3 * v], V.pos[3 * v + 1], V.pos[3 * v + 2]};
+    double out[3] = {(double)u3[0], (double)u3[1], (double)u3[2]};
+    if (inside_envelope(V.d, V.ib.dirac, p)) {
+        const double w = pipe_weight(V.ib, p, S == 4 ? 2.0 : 1.5);
+        if (w < 1) {
+            C t[3] = {C(0), C(0), C(0)};
+            tophat_interp<C, UT>(V.d, V.ib, p, static_cast<const UT*>(V.u), t);
+            for (int k = 0; k < 3; ++k) out[k] = w <= 0 ? (double)t[k] : (1. - w) * (double)t[k] + w * out[k];
+        }
+    }
+    double xn[3] = {p[0] + out[0], p[1] + out[1], p[2] + out[2]};
+    pipe_move(V.ib, p, out, xn);
+    for (int k = 0; k < 3; ++k) {
+        V.vel[3 * v + k] = out[k];
+        V.pos_next[3 * v + k] = xn[k];
+    }
+}
+
 // ---------------------------------------------------------------- interpolation
 // Interpolation of the velocity field (written by the collide-and-stream kernel or the
 // velocity kernel) to every vertex, followed by the explicit Euler move
 // X_{n+1} = X_n + U_n (DeformableParticle3D::move_vertices, DeformableParticle3D.hh:26-51).
 // Classes and index arithmetic follow interpolate_impl with the Bulk / General
 // interpolators, ImmersedBoundaryDynamics_interpolation.hh:13-153.
-// One thread per vertex.  BATCH: the vertex numbering runs over the lattices of a batch and
-// each thread looks its lattice's view up through vinst; otherwise v1 is the lattice.
+// BATCH: the vertex numbering runs over the lattices of a batch and each vertex looks its lattice's view
+// up through vinst; otherwise v1 is the lattice.
 // FOLD (sparse force reset): the velocity field holds j/rho + body/2, and the vertex velocity
 // adds the share of the previous step's force, sum of w (Fold - body) / 2 over the support
 // nodes off the finite-difference wall rows (whose velocity is the wall's); the sum of the two
 // is the interpolation of j/rho + Fold/2, the reference's computeVelocity field.
+//
+//
+// Many vertices: one thread per vertex.
 template <class UT, int S, bool FOLD = false>
 __device__ __forceinline__ void interpolate_move_vertex(const IbView& V, int v) {
     using C = typename InterpC<UT>::type;  // also the force field's type
@@ -272,33 +297,138 @@ __device__ __forceinline__ void interpolate_move_vertex(const IbView& V, int v) 
         out[1] = (double)(FOLD ? acc[1] + C(0.5) * facc[1] : acc[1]);
         out[2] = (double)(FOLD ? acc[2] + C(0.5) * facc[2] : acc[2]);
     }
-    if (ib.has_pipe && inside_envelope(d, ib.dirac, p)) {
-        const double w = pipe_weight(ib, p, S == 4 ? 2.0 : 1.5);
-        if (w < 1) {  // near the wall: blend with (or switch to) the TopHat kernel
-            C t[3] = {C(0), C(0), C(0)};
-            tophat_interp<C, UT>(d, ib, p, u, t);
-            for (int k = 0; k < 3; ++k) out[k] = w <= 0 ? (double)t[k] : (1. - w) * (double)t[k] + w * out[k];
-        }
+    if (ib.has_pipe) {
+        const C u3[3] = {(C)out[0], (C)out[1], (C)out[2]};
+        move_near_pipe<UT, S>(V, v, u3);
+        return;
     }
     vel[3 * v] = out[0];
     vel[3 * v + 1] = out[1];
     vel[3 * v + 2] = out[2];
-    double xn[3] = {p[0] + out[0], p[1] + out[1], p[2] + out[2]};
-    if (ib.has_pipe) pipe_move(ib, p, out, xn);
-    pos_next[3 * v] = xn[0];
-    pos_next[3 * v + 1] = xn[1];
-    pos_next[3 * v + 2] = xn[2];
+    pos_next[3 * v] = p[0] + out[0];
+    pos_next[3 * v + 1] = p[1] + out[1];
+    pos_next[3 * v + 2] = p[2] + out[2];
 }
 
 // 9 CTAs of 128 threads per SM (at most 56 registers): measured 2 % faster than 8 on the
 // 400-cell channel (the kernel waits on its gathers; more warps hide more of that)
 template <class UT, int S, bool BATCH, bool FOLD = false>
-__global__ void __launch_bounds__(128, 9) k_interpolate_move(IbView v1, const IbView* __restrict__ views,
+__global__ void __launch_bounds__(128, 9) k_interpolate_vertices(IbView v1, const IbView* __restrict__ views,
                                                            const int* __restrict__ vinst, int nvert) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nvert) return;
     const IbView& V = BATCH ? views[vinst[g]] : v1;
     interpolate_move_vertex<UT, S, FOLD>(V, BATCH ? g - V.vbase : (V.order ? V.order[g] : g));
+}
+
+// Few vertices: a CTA takes 32; three warps prepare one axis each (nodes and weights, the FP64 part), then warp r
+// gathers row r of every support (one vertex per lane) and 96 threads add the rows up in order and move
+// one coordinate each.  Bound by the latency of the gathers and by the FP64 pipe (about 9 operations per
+// coordinate); with tens of thousands of vertices the CTAs' barriers cost more than the threads of the
+// kernel above wait.  Measured, interpolation and update of a step in 256 x 64 x 64, 32 vertices per CTA against
+// one thread per vertex: FP32 Roma 18.7 / 24.4 us at 2,568 vertices, 23.0 / 25.1 at 20,544, 27.2 / 26.2 at 41,088,
+// 57 / 35 at 164,352; FP64 Peskin 28.7 / 55.5, 63 / 66, 100 / 88, 319 / 221; the line is between those.
+constexpr int kGatherMax = 24576;
+constexpr int kGatherVerts = 32;
+template <class C, int S>
+struct GatherTile {
+    int vert[kGatherVerts];         // vertex, -1: none
+    int inst[kGatherVerts];         // batch: the lattice
+    int node[3][S][kGatherVerts];   // support nodes, -1: none
+    C w[3][S][kGatherVerts];
+    C part[S * S][3][kGatherVerts];  // of each row
+};
+
+template <class UT, int S, bool BATCH, bool FOLD = false>
+__global__ void __launch_bounds__(32 * S * S) k_interpolate_move(IbView v1, const IbView* __restrict__ views,
+                                                                const int* __restrict__ vinst, int nvert) {
+    using C = typename InterpC<UT>::type;  // also the force field's type
+    static_assert(S == 3 || S == 4, "Roma (3) or Peskin (4) support");
+    constexpr int dirac = S == 4 ? BIB_DIRAC_PESKIN : BIB_DIRAC_ROMA;
+    __shared__ GatherTile<C, S> sm;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 3) {
+        const int g = blockIdx.x * kGatherVerts + lane, a = warp;
+        int v = -1, inst = 0;
+        if (g < nvert) {
+            if (BATCH) inst = vinst[g];
+            const IbView& V = BATCH ? views[inst] : v1;
+            v = BATCH ? g - V.vbase : (V.order ? V.order[g] : g);
+            const LatticeDesc& d = V.d;
+            const int off = (int)V.ib.offset, per = a == 0 ? d.px : (a == 1 ? d.py : d.pz);
+            const int N = a == 0 ? d.nx : (a == 1 ? d.ny : d.nz);
+            const double p = V.pos[3 * v + a];
+            const bool in = inside_axis(per, N, dirac, p);
+            const double x = p - V.ib.offset;
+            const int64_t lo = (int64_t)ceil(x - half_support(dirac));
+#pragma unroll
+            for (int m = 0; m < S; ++m) {
+                sm.node[a][m][lane] = in ? remap_global(per, N, lo + m, off) : -1;
+                sm.w[a][m][lane] = axis_weight<C>(dirac, lo, x, m);
+            }
+        }
+        if (a == 0) {
+            sm.vert[lane] = v;
+            sm.inst[lane] = inst;
+        }
+    }
+    __syncthreads();
+    const int v = sm.vert[lane];
+    if (v >= 0) {
+        const IbView& V = BATCH ? views[sm.inst[lane]] : v1;
+        const LatticeDesc& d = V.d;
+        const UT* __restrict__ u = static_cast<const UT*>(V.u);
+        const int b = warp / S, c = warp % S;
+        const int gy = sm.node[1][b][lane], gz = sm.node[2][c][lane];
+        C acc[3] = {C(0), C(0), C(0)};
+        if (gy >= 0 && gz >= 0) {
+            const int64_t row = (int64_t)d.nx * (gy + (int64_t)d.ny * gz);
+            const bool fold = FOLD && !fd_wall_node(d, gy);
+#pragma unroll
+            for (int m = 0; m < S; ++m) {
+                const int gx = sm.node[0][m][lane];
+                if (gx < 0) continue;
+                const C w = sm.w[0][m][lane];
+                const U3<C> uc = load_u(u, row + gx);
+                acc[0] += w * uc.x;
+                acc[1] += w * uc.y;
+                acc[2] += w * uc.z;
+                if (fold) {
+                    const C* __restrict__ Fo = static_cast<const C*>(V.Fold) + 3 * (row + gx);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) acc[q] += C(0.5) * (w * (__ldg(Fo + q) - (C)d.body[q]));
+                }
+            }
+            const C wyz = sm.w[1][b][lane] * sm.w[2][c][lane];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) acc[q] *= wyz;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) sm.part[warp][q][lane] = acc[q];
+    }
+    __syncthreads();
+    // one coordinate per thread, neighbouring threads the coordinates of a vertex
+    const int t = threadIdx.x / 3, q = threadIdx.x - 3 * t;
+    if (threadIdx.x >= 3 * kGatherVerts || sm.vert[t] < 0) return;
+    const IbView& V = BATCH ? views[sm.inst[t]] : v1;
+    const int64_t e = 3LL * sm.vert[t] + q;
+    C sum = sm.part[0][q][t];
+#pragma unroll
+    for (int r = 1; r < S * S; ++r) sum += sm.part[r][q][t];
+    if (V.ib.has_pipe) {  // the near-wall blend and the reflection need the whole vector
+        if (q == 0) {
+            C u3[3] = {sum, sm.part[0][1][t], sm.part[0][2][t]};
+#pragma unroll
+            for (int r = 1; r < S * S; ++r) {
+                u3[1] += sm.part[r][1][t];
+                u3[2] += sm.part[r][2][t];
+            }
+            move_near_pipe<UT, S>(V, sm.vert[t], u3);
+        }
+        return;
+    }
+    V.vel[e] = (double)sum;
+    V.pos_next[e] = V.pos[e] + (double)sum;
 }
 
 // Sparse force reset: F := body force at the support nodes the last spreading into F recorded
@@ -378,15 +508,15 @@ __device__ __noinline__ void spread_vertex_nodes(const IbView& V, const double* 
 }
 
 // Spreading by rows.  A row of a vertex's support, S cells of three components, is one contiguous run
-// of 3 S values of the force field.  The first warp of a CTA prepares 32 vertices in shared memory (the
-// products of x-weight and force, the y and z weights, the row offsets); then all threads take the
+// of 3 S values of the force field.  Three warps of a CTA prepare 32 vertices in shared memory, one axis each
+// (the products of x-weight and force, the y and z weights, the rows); then all threads take the
 // (vertex, row, word) items in order, neighbouring lanes the neighbouring words of a row.  FP32 fields
 // are added to in aligned float4 words (S = 3: three words cover a run at any offset, S = 4: four; values
 // outside the run add zero), FP64 fields value by value.
 // Bound by the count of its L2 reductions.  With one array per component a vertex had 27 runs of 3 values;
 // with the components of a cell together it has 9 of 9 values, 1.25 lines each: 256,800 vertices (Roma) of
-// the 400-cell channel 79.5 -> 40.9 us, 128,400 (Peskin) of a 240 x 96 x 90 channel 80 -> 39 us.  64 vertices
-// per CTA were slower (40.6 against 36.8 us alone: the adding threads wait longer for the first warp).
+// the 400-cell channel 79.5 -> 37.4 us, 128,400 (Peskin) of a 240 x 96 x 90 channel 80 -> 35 us (40.9 and 38 with
+// all axes of a vertex prepared by one thread).  64 vertices per CTA were slower (40.6 against 36.8 us alone).
 constexpr int kSpreadVerts = 32, kSpreadThreads = 128;
 template <class FT, int S>
 struct SpreadVertex {
@@ -394,7 +524,7 @@ struct SpreadVertex {
     static constexpr int ITEMS = S * S * WORDS;
     FT p[3 * S];  // x-weight times force
     FT wy[S], wz[S];
-    int yo[S], zo[S];  // row offsets in cells of one z-plane / in rows, -1: behind a wall
+    int yo[S], zo[S];  // rows and planes, -1: behind a wall
     int gx;            // first cell along x (its run wraps if gx + S > nx), -1: nothing to add
     int inst;          // batch: the lattice
 };
@@ -404,46 +534,59 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const
                                                                 const int* __restrict__ vinst, int nvert) {
     using SV = SpreadVertex<FT, S>;
     __shared__ SV sv[kSpreadVerts];
-    const int g0 = blockIdx.x * kSpreadVerts;
-    if (threadIdx.x < kSpreadVerts) {
-        SV& s = sv[threadIdx.x];
-        const int g = g0 + threadIdx.x;
-        s.gx = -1;
+    __shared__ int lo_rec[3][kSpreadVerts];  // first support node per axis for the sparse reset
+    __shared__ unsigned inside_m[3];         // vertices inside the envelope, per axis
+    const int a = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.x * kSpreadVerts + lane;
+    int v = 0, inst = 0;
+    if (a < 3) {  // warp a prepares axis a of the 32 vertices
+        constexpr int dirac = S == 4 ? BIB_DIRAC_PESKIN : BIB_DIRAC_ROMA;
+        bool in = false;
         if (g < nvert) {
-            s.inst = BATCH ? vinst[g] : 0;
-            const IbView& V = BATCH ? views[s.inst] : v1;
+            inst = BATCH ? vinst[g] : 0;
+            const IbView& V = BATCH ? views[inst] : v1;
+            v = BATCH ? g - V.vbase : g;
+            SV& s = sv[lane];
             const LatticeDesc& d = V.d;
-            const int v = BATCH ? g - V.vbase : g;
-            const double p[3] = {V.pos[3 * v], V.pos[3 * v + 1], V.pos[3 * v + 2]};
-            const double force[3] = {V.force[3 * v], V.force[3 * v + 1], V.force[3 * v + 2]};
-            const bool inside = inside_envelope(d, V.ib.dirac, p);
-            const int off = (int)V.ib.offset;
-            if (inside) {
-                if (V.ib.has_pipe || off > 0) {
-                    spread_vertex_nodes<FT, S>(V, p, force);
-                } else {
-                    FT wx[S];
-                    const int64_t lx = axis_weights<FT, S>(p[0] - V.ib.offset, wx);
-                    const int64_t ly = axis_weights<FT, S>(p[1] - V.ib.offset, s.wy);
-                    const int64_t lz = axis_weights<FT, S>(p[2] - V.ib.offset, s.wz);
-                    s.gx = remap_global(d.px, d.nx, lx, off);
+            const int off = (int)V.ib.offset, per = a == 0 ? d.px : (a == 1 ? d.py : d.pz);
+            const int N = a == 0 ? d.nx : (a == 1 ? d.ny : d.nz);
+            const double p = V.pos[3 * v + a];
+            in = inside_axis(per, N, dirac, p);
+            const double x = p - V.ib.offset;
+            const int64_t lo = (int64_t)ceil(x - half_support(dirac));
+            lo_rec[a][lane] = in ? record_lo(per, N, lo, off) : 0;
+            if (a == 0) {
+                s.inst = inst;
+                s.gx = in ? remap_global(per, N, lo, off) : -1;
+                const FT f[3] = {(FT)V.force[3 * v], (FT)V.force[3 * v + 1], (FT)V.force[3 * v + 2]};
 #pragma unroll
-                    for (int m = 0; m < S; ++m) {
-                        s.yo[m] = remap_global(d.py, d.ny, ly + m, off);
-                        s.zo[m] = remap_global(d.pz, d.nz, lz + m, off);
+                for (int m = 0; m < S; ++m) {
+                    const FT w = axis_weight<FT>(dirac, lo, x, m);
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) s.p[3 * m + q] = wx[m] * (FT)force[q];
-                    }
+                    for (int q = 0; q < 3; ++q) s.p[3 * m + q] = w * f[q];
+                }
+            } else {
+                int* node = a == 1 ? s.yo : s.zo;
+                FT* w = a == 1 ? s.wy : s.wz;
+#pragma unroll
+                for (int m = 0; m < S; ++m) {
+                    node[m] = in ? remap_global(per, N, lo + m, off) : -1;
+                    w[m] = axis_weight<FT>(dirac, lo, x, m);
                 }
             }
-            if (V.spread_lo) {
-                constexpr double h = S == 4 ? 2.0 : 1.5;
-                V.spread_lo[v] = inside ? make_int4(record_lo(d.px, d.nx, (int64_t)ceil(p[0] - V.ib.offset - h), off),
-                                                    record_lo(d.py, d.ny, (int64_t)ceil(p[1] - V.ib.offset - h), off),
-                                                    record_lo(d.pz, d.nz, (int64_t)ceil(p[2] - V.ib.offset - h), off), 1)
-                                        : make_int4(0, 0, 0, 0);
-            }
         }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) inside_m[a] = m;
+    }
+    __syncthreads();
+    const unsigned inside = inside_m[0] & inside_m[1] & inside_m[2];
+    if (a == 0) {
+        const bool in = (inside >> lane) & 1u;
+        const IbView& V = BATCH ? views[inst] : v1;
+        const bool nodewise = g < nvert && (V.ib.has_pipe || (int)V.ib.offset > 0);
+        if (!in || nodewise) sv[lane].gx = -1;
+        if (g < nvert && V.spread_lo)
+            V.spread_lo[v] = in ? make_int4(lo_rec[0][lane], lo_rec[1][lane], lo_rec[2][lane], 1) : make_int4(0, 0, 0, 0);
+        if (in && nodewise) spread_vertex_nodes<FT, S>(V, V.pos + 3LL * v, V.force + 3LL * v);
     }
     __syncthreads();
     for (int it = threadIdx.x; it < kSpreadVerts * SV::ITEMS; it += kSpreadThreads) {
@@ -1606,20 +1749,28 @@ IbView single_view(const Lattice& L, int fbuf) {
 
 namespace {
 
+template <class UT, int S, bool BATCH, bool FOLD = false>
+void interpolate_inst(const IbView& v1, const IbView* views, const int* vinst, int nvert, cudaStream_t s) {
+    if (nvert <= kGatherMax)
+        k_interpolate_move<UT, S, BATCH, FOLD>
+            <<<(nvert + kGatherVerts - 1) / kGatherVerts, 32 * S * S, 0, s>>>(v1, views, vinst, nvert);
+    else
+        k_interpolate_vertices<UT, S, BATCH, FOLD><<<(nvert + 127) / 128, 128, 0, s>>>(v1, views, vinst, nvert);
+}
+
 template <bool BATCH>
 void interpolate_any(int storage, int dirac, const IbView& v1, const IbView* views, const int* vinst, int nvert,
                      cudaStream_t s) {
-    const unsigned g = (nvert + 127) / 128;
     const bool peskin = dirac == BIB_DIRAC_PESKIN;
     if (storage == BIB_STORAGE_F64) {
-        if (peskin) k_interpolate_move<double, 4, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
-        else k_interpolate_move<double, 3, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
+        if (peskin) interpolate_inst<double, 4, BATCH>(v1, views, vinst, nvert, s);
+        else interpolate_inst<double, 3, BATCH>(v1, views, vinst, nvert, s);
     } else if (storage == BIB_STORAGE_F32) {
-        if (peskin) k_interpolate_move<float, 4, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
-        else k_interpolate_move<float, 3, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
+        if (peskin) interpolate_inst<float, 4, BATCH>(v1, views, vinst, nvert, s);
+        else interpolate_inst<float, 3, BATCH>(v1, views, vinst, nvert, s);
     } else {
-        if (peskin) k_interpolate_move<__half, 4, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
-        else k_interpolate_move<__half, 3, BATCH><<<g, 128, 0, s>>>(v1, views, vinst, nvert);
+        if (peskin) interpolate_inst<__half, 4, BATCH>(v1, views, vinst, nvert, s);
+        else interpolate_inst<__half, 3, BATCH>(v1, views, vinst, nvert, s);
     }
 }
 
@@ -1661,14 +1812,13 @@ void launch_interpolate_move(const Lattice& L, cudaStream_t s, int fold) {
     }
     IbView v = single_view(L, -1);
     v.Fold = L.F[fold];
-    const unsigned g = (L.nvert + 127) / 128;
     const bool peskin = L.ib.dirac == BIB_DIRAC_PESKIN;
     if (L.storage == BIB_STORAGE_F32) {
-        if (peskin) k_interpolate_move<float, 4, false, true><<<g, 128, 0, s>>>(v, nullptr, nullptr, L.nvert);
-        else k_interpolate_move<float, 3, false, true><<<g, 128, 0, s>>>(v, nullptr, nullptr, L.nvert);
+        if (peskin) interpolate_inst<float, 4, false, true>(v, nullptr, nullptr, L.nvert, s);
+        else interpolate_inst<float, 3, false, true>(v, nullptr, nullptr, L.nvert, s);
     } else {
-        if (peskin) k_interpolate_move<__half, 4, false, true><<<g, 128, 0, s>>>(v, nullptr, nullptr, L.nvert);
-        else k_interpolate_move<__half, 3, false, true><<<g, 128, 0, s>>>(v, nullptr, nullptr, L.nvert);
+        if (peskin) interpolate_inst<__half, 4, false, true>(v, nullptr, nullptr, L.nvert, s);
+        else interpolate_inst<__half, 3, false, true>(v, nullptr, nullptr, L.nvert, s);
     }
 }
 

@@ -196,21 +196,15 @@ __device__ __forceinline__ int support(int dirac) { return dirac == BIB_DIRAC_PE
 // selects between two interpolators with the same result here).  On a periodic axis the
 // min-mod distance is at most N/2 < (N - 1)/2 + h, so only walled axes can put a vertex
 // outside.  Non-finite positions are outside.
+__device__ __forceinline__ bool inside_axis(int per, int N, int dirac, double p) {
+    if (per) return isfinite(p);
+    const double h = half_support(dirac), top = (double)(N - 1);
+    const double elo = 0.0 - h, ehi = top + h;
+    return fabs(0.5 * (elo + ehi) - p) < 0.5 * (ehi - elo);
+}
 __device__ __forceinline__ bool inside_envelope(const LatticeDesc& d, int dirac, const double* p) {
-    const double h = half_support(dirac);
-    const int N[3] = {d.nx, d.ny, d.nz};
-    const int per[3] = {d.px, d.py, d.pz};
-    bool in = true;
-    for (int a = 0; a < 3; ++a) {
-        if (per[a]) {
-            in = in && isfinite(p[a]);
-        } else {
-            const double top = (double)(N[a] - 1);
-            const double elo = 0.0 - h, ehi = top + h;
-            in = in && fabs(0.5 * (elo + ehi) - p[a]) < 0.5 * (ehi - elo);
-        }
-    }
-    return in;
+    return inside_axis(d.px, d.nx, dirac, p[0]) && inside_axis(d.py, d.ny, dirac, p[1]) &&
+           inside_axis(d.pz, d.nz, dirac, p[2]);
 }
 
 // Positive remainder of x modulo N; the division is only taken more than a period away.
