@@ -341,84 +341,93 @@ __global__ void __launch_bounds__(128) k_guo_walls(LatticeDesc d, T* __restrict_
                              (w.nodyn ? C(0) : bgk_equilibrium<C>(i, rbw, invRho, jw, jsq)) + fw[i]);
 }
 
+// grid: blocks of wall nodes, two sides
+constexpr int kWallBlock = 64;
 template <class T>
-__global__ void k_fd_walls(LatticeDesc d, const T* __restrict__ f, T* __restrict__ wall,
-                           const typename Store<T>::F* __restrict__ F) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= d.nx) return;
-    fd_wall_cell<T>(d, f, wall, F, x, blockIdx.y, blockIdx.z);
+__global__ void __launch_bounds__(kWallBlock) k_fd_walls(LatticeDesc d, const T* __restrict__ f, T* __restrict__ wall,
+                                                         const typename Store<T>::F* __restrict__ F) {
+    const uint32_t t = blockIdx.x * kWallBlock + threadIdx.x, nx = (uint32_t)d.nx;
+    if (t >= nx * (uint32_t)d.nz) return;
+    fd_wall_cell<T>(d, f, wall, F, (int)(t % nx), (int)(t / nx), blockIdx.y);
 }
 
-// Batched: grid.z = 2 sides x lattices; each lattice's view of the state after the swap.
+// Batched: grid.z = lattices; each lattice's view of the state after the swap.
 template <class T>
-__global__ void k_fd_walls_batch(const CollideView* __restrict__ views) {
-    const CollideView& V = views[blockIdx.z >> 1];
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.y;
-    if (!V.d.fd_walls || x >= V.d.nx || z >= V.d.nz) return;
+__global__ void __launch_bounds__(kWallBlock) k_fd_walls_batch(const CollideView* __restrict__ views) {
+    const CollideView& V = views[blockIdx.z];
+    const uint32_t t = blockIdx.x * kWallBlock + threadIdx.x, nx = (uint32_t)V.d.nx;
+    if (!V.d.fd_walls || t >= nx * (uint32_t)V.d.nz) return;
     fd_wall_cell<T>(V.d, static_cast<const T*>(V.fin), static_cast<T*>(const_cast<void*>(V.wall)),
-                    static_cast<const typename Store<T>::F*>(V.Fprev), x, z, blockIdx.z & 1);
+                    static_cast<const typename Store<T>::F*>(V.Fprev), (int)(t % nx), (int)(t / nx), blockIdx.y);
 }
 
-template <class T>
-__device__ __forceinline__ void fd_wall_cell(const LatticeDesc& d, const T* __restrict__ f, T* __restrict__ wall,
-                                             const typename Store<T>::F* __restrict__ F, int x, int z, int side) {
+// With a uniform wall velocity the stress has three entries (xy, yy, yz), and a wall row and its
+// neighbour gather from rows inside the domain (three rows at least, periodic x and z).  One thread per
+// wall node; bound by latency, in FP64 by the FP64 pipe: with all six entries, multiplications by zero
+// lattice components and the general gather 18.1 us (64 x 64 nodes on two sides, FP64; 8.6 us FP32 128 x 64),
+// now 11.4 and 5.0; 64 lattices in one launch 68 -> 25 us, whose rows of 32 to 96 nodes left lanes idle.
+template <class T, int SIDE>
+__device__ __forceinline__ void fd_wall_node_rebuild(const LatticeDesc& d, const T* __restrict__ f, T* __restrict__ wall,
+                                                     const typename Store<T>::F* __restrict__ F, int x, int z) {
     using C = typename Store<T>::C;
-    const int y = side == 0 ? 0 : d.ny - 1;
-    const int orientation = side == 0 ? -1 : 1;
-    const int64_t k = x + (int64_t)d.nx * (y + (int64_t)d.ny * z);
-    const int y1 = y - orientation;
-    const int64_t k1 = x + (int64_t)d.nx * (y1 + (int64_t)d.ny * z);
+    constexpr int O = SIDE == 0 ? -1 : 1;  // outward normal
+    const int y = SIDE == 0 ? 0 : d.ny - 1, y1 = y - O;
+    const int64_t plane = (int64_t)d.nx * d.ny;
+    // source offsets along x and z of c = -1, 0, 1
+    const int xo[3] = {x + 1 == d.nx ? 0 : x + 1, x, x == 0 ? d.nx - 1 : x - 1};
+    const int64_t zo[3] = {(z + 1 == d.nz ? 0 : z + 1) * plane, z * plane, (z == 0 ? d.nz - 1 : z - 1) * plane};
     C fc[Q], f1[Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
-        int face;
-        const int64_t s = source_cell(d, i, x, y, z, face);
-        fc[i] = s >= 0 ? Store<T>::load(f + i * d.stride + s, d.inv_scale) : C(0);  // unknown ones are not used
+        const T* p = f + i * d.stride + xo[cx(i) + 1] + zo[cz(i) + 1];
+        f1[i] = Store<T>::load(p + (int64_t)d.nx * (y1 - cy(i)), d.inv_scale);
+        fc[i] = cy(i) == -O ? C(0) : Store<T>::load(p + (int64_t)d.nx * (y - cy(i)), d.inv_scale);  // unknown ones are not used
     }
-    gather<T>(d, f, wall, x, y1, z, k1, f1);
+    const int64_t k = x + (int64_t)d.nx * y + z * plane, k1 = x + (int64_t)d.nx * y1 + z * plane;
     const C Fy = (C)F[3 * k + 1];
     C F1[3] = {(C)F[3 * k1], (C)F[3 * k1 + 1], (C)F[3 * k1 + 2]};
-    const C uw[3] = {(C)d.wall_u[side][0], (C)d.wall_u[side][1], (C)d.wall_u[side][2]};
+    const C uw[3] = {(C)d.wall_u[SIDE][0], (C)d.wall_u[SIDE][1], (C)d.wall_u[SIDE][2]};
     C rhoOnWall = 0, rhoNormal = 0;
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
         if (cy(i) == 0) rhoOnWall += fc[i];
+        if (cy(i) == O) rhoNormal += fc[i];
     }
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        if (cy(i) == orientation) rhoNormal += fc[i];
-    }
-    const C velNormal = C(orientation) * (uw[1] - C(0.5) * Fy);
+    const C velNormal = C(O) * (uw[1] - C(0.5) * Fy);
     const C rhoBarW = (C(2) * rhoNormal + rhoOnWall - velNormal) / (C(1) + velNormal);
     const C rho = rhoBarW + C(1);
     C u1[3];
     velocity_with_force(f1, F1, u1);
-    C dy_u[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) dy_u[a] = C(-orientation) * (u1[a] - uw[a]);
+    // one-sided normal derivative of the velocity times -rho / (3 omega), fromPiToFneq
+    // (src/latticeBoltzmann/offEquilibriumTemplates.h:91-115) times 4.5 and the multiplicities
     const C sToPi = -rho / C(3) / (C)d.omega;
-    // pi: xx, xy, xz, yy, yz, zz with the tangential derivatives equal to zero
-    const C pi[6] = {C(0), dy_u[0] * sToPi, C(0), C(2) * dy_u[1] * sToPi, dy_u[2] * sToPi, C(0)};
-    C j[3] = {rho * uw[0], rho * uw[1], rho * uw[2]};
-    const C jSqr = j[0] * j[0] + j[1] * j[1] + j[2] * j[2];
-    const C rhoBar = rho - C(1);
-    const C invRho = C(1) / (rhoBar + C(1));
-    const int64_t wk = wall_index(d, side, x, z), ws = wall_stride(d);
+    const C pxy = C(9) * C(-O) * (u1[0] - uw[0]) * sToPi, pyy = C(9) * C(-O) * (u1[1] - uw[1]) * sToPi,
+            pyz = C(9) * C(-O) * (u1[2] - uw[2]) * sToPi;
+    const C j[3] = {rho * uw[0], rho * uw[1], rho * uw[2]};
+    const C rhoBar = rho - C(1), invRho = C(1) / rho;
+    // bgk_equilibrium (d3q19.cuh) with the terms of a pair gathered
+    const C base = rhoBar - C(1.5) * invRho * (j[0] * j[0] + j[1] * j[1] + j[2] * j[2]);
+    const C h = C(4.5) * invRho, third = pyy * (C(1) / C(3));
+    const int64_t wk = wall_index(d, SIDE, x, z), ws = wall_stride(d);
+    Store<T>::store(wall + wk, weight<C>(0) * (base - third), d.scale);
 #pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        // fromPiToFneq, src/latticeBoltzmann/offEquilibriumTemplates.h:91-115
-        const C c0 = C(cx(i)), c1 = C(cy(i)), c2 = C(cz(i));
-        const C cs2 = C(1) / C(3);
-        C fneq = C(0);
-        fneq += pi[0] * (c0 * c0 - cs2);
-        fneq += pi[1] * C(2) * c0 * c1;
-        fneq += pi[2] * C(2) * c0 * c2;
-        fneq += pi[3] * (c1 * c1 - cs2);
-        fneq += pi[4] * C(2) * c1 * c2;
-        fneq += pi[5] * (c2 * c2 - cs2);
-        fneq *= weight<C>(i) * C(3) * C(3) / C(2);
-        Store<T>::store(wall + i * ws + wk, bgk_equilibrium<C>(i, rhoBar, invRho, j, jSqr) + fneq, d.scale);
+    for (int i = 1; i < 10; ++i) {
+        const C cj = cdot<C>(i, j[0], j[1], j[2]);
+        C even = fmac(h * cj, cj, base) - third;
+        if (cy(i) != 0) {
+            even += pyy;
+            if (cx(i) != 0) even += C(cx(i) * cy(i)) * pxy;
+            if (cz(i) != 0) even += C(cy(i) * cz(i)) * pyz;
+        }
+        Store<T>::store(wall + i * ws + wk, weight<C>(i) * fmac(C(3), cj, even), d.scale);
+        Store<T>::store(wall + (i + 9) * ws + wk, weight<C>(i) * fmac(C(-3), cj, even), d.scale);
     }
+}
+template <class T>
+__device__ __forceinline__ void fd_wall_cell(const LatticeDesc& d, const T* __restrict__ f, T* __restrict__ wall,
+                                             const typename Store<T>::F* __restrict__ F, int x, int z, int side) {
+    if (side == 0) fd_wall_node_rebuild<T, 0>(d, f, wall, F, x, z);
+    else fd_wall_node_rebuild<T, 1>(d, f, wall, F, x, z);
 }
 
 // computeVelocity of one cell of the current state with the current external force F (wall nodes give
@@ -717,17 +726,14 @@ void collide_stream_t(const Lattice& L, Coupling mode, cudaStream_t s) {
 
 template <class T>
 void fd_walls_batch_t(const BatchLaunch& B, cudaStream_t s) {
-    const int bx = B.nx_max >= 128 ? 128 : 64;
-    dim3 g((B.nx_max + bx - 1) / bx, B.nz_max, 2 * B.n);
-    k_fd_walls_batch<T><<<g, bx, 0, s>>>(B.wviews);
+    k_fd_walls_batch<T><<<dim3(lin_grid((int64_t)B.nx_max * B.nz_max, kWallBlock), 2, B.n), kWallBlock, 0, s>>>(B.wviews);
 }
 
 template <class T>
 void fd_walls_t(const Lattice& L, int buf, int fbuf, cudaStream_t s) {
     using FT = typename Store<T>::F;
-    const int bx = row_block(L.d);
-    dim3 g((L.d.nx + bx - 1) / bx, L.d.nz, 2);
-    k_fd_walls<T><<<g, bx, 0, s>>>(L.d, (const T*)L.f[buf], (T*)L.wall, (const FT*)L.F[fbuf]);
+    k_fd_walls<T><<<dim3(lin_grid((int64_t)L.d.nx * L.d.nz, kWallBlock), 2), kWallBlock, 0, s>>>(
+        L.d, (const T*)L.f[buf], (T*)L.wall, (const FT*)L.F[fbuf]);
 }
 
 #define BIB_DISPATCH(storage, FN, ...)                          \
