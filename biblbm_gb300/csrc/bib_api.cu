@@ -123,6 +123,110 @@ inline double dt(V3d a, V3d b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 inline double nrm(V3d a) { return std::sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
 inline V3d scl(V3d a, double s) { return {a.x / s, a.y / s, a.z / s}; }
 
+// Patches of the shape (ShapeDev): chunks of 32 vertices along a Morton curve over the shape's box, and
+// per triangle edge the neighbour and the rest angle from the adjacent-triangle pairs (edge_of[p]: the two
+// triangles of pair p).  A pair (q0, q1, q2, q3) of triangles at q1 and q3 with the common edge q0 q2 is
+// seen from both sides alike with (q2, q3, q0, q1) from the second.  Left out (npatch 0) where a patch would
+// not fit.
+void build_patches(ShapeHost& S, const std::vector<std::pair<int, int>>& edge_of) {
+    const int nv = (int)S.rest.size() / 3, nt = (int)S.tri_area.size();
+    std::vector<int> nb(3 * (size_t)nt, -1), flip(3 * (size_t)nt, 0);
+    std::vector<float> bend(6 * (size_t)nt, 0.0f);
+    for (size_t p = 0; p < edge_of.size(); ++p)
+        for (int side = 0; side < 2; ++side) {
+            const int* q = &S.pairs[4 * p];
+            const int t = side ? edge_of[p].second : edge_of[p].first;
+            const int v0 = side ? q[2] : q[0], own = side ? q[3] : q[1], v2 = side ? q[0] : q[2];
+            for (int k = 0; k < 3; ++k) {
+                if (S.tri[3 * t + k] != own) continue;
+                nb[3 * t + k] = side ? q[1] : q[3];
+                flip[3 * t + k] = !(S.tri[3 * t + (k + 2) % 3] == v0 && S.tri[3 * t + (k + 1) % 3] == v2);
+                bend[6 * (size_t)t + 2 * k] = (float)S.pair_cs[2 * p];
+                bend[6 * (size_t)t + 2 * k + 1] = (float)S.pair_cs[2 * p + 1];
+            }
+        }
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) lo[a] = hi[a] = S.rest[a];
+    for (int v = 0; v < nv; ++v)
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = std::min(lo[a], S.rest[3 * v + a]);
+            hi[a] = std::max(hi[a], S.rest[3 * v + a]);
+        }
+    const double span = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
+    std::vector<std::pair<uint64_t, int>> code((size_t)nv);
+    for (int v = 0; v < nv; ++v) {
+        uint64_t m = 0;
+        for (int a = 0; a < 3; ++a) {
+            const uint64_t q = span > 0 ? (uint64_t)(1023.0 * (S.rest[3 * v + a] - lo[a]) / span) : 0;
+            for (int b = 0; b < 10; ++b) m |= ((q >> b) & 1u) << (3 * b + a);
+        }
+        code[(size_t)v] = {m, v};
+    }
+    std::sort(code.begin(), code.end());
+    std::vector<int> local((size_t)nv, -1), tri_local((size_t)nt, -1);
+    for (int first = 0; first < nv; first += kPatchOwn) {
+        PatchDev P{};
+        P.own = std::min(kPatchOwn, nv - first);
+        P.verts0 = (int)S.pverts.size(), P.tris0 = (int)S.ptris.size(), P.inc0 = (int)S.pinc.size();
+        auto add = [&](int v) {
+            if (local[(size_t)v] < 0) {
+                local[(size_t)v] = P.all++;
+                S.pverts.push_back(v);
+            }
+            return local[(size_t)v];
+        };
+        for (int k = 0; k < P.own; ++k) add(code[(size_t)(first + k)].second);
+        std::vector<int> tris;
+        for (int k = 0; k < P.own; ++k) {
+            const int v = code[(size_t)(first + k)].second;
+            for (int e = S.inc_off[v]; e < S.inc_off[v + 1]; ++e)
+                if ((S.inc[e] >> 29) == 1) tris.push_back(S.inc[e] & ((1 << 29) - 1));
+        }
+        std::sort(tris.begin(), tris.end());
+        tris.erase(std::unique(tris.begin(), tris.end()), tris.end());
+        P.tris = (int)tris.size();
+        bool fits = 3 * tris.size() < 65535;
+        for (int i = 0; i < P.tris && fits; ++i) {
+            const int t = tris[(size_t)i];
+            tri_local[(size_t)t] = i;
+            PatchTri pt{};
+            for (int k = 0; k < 3; ++k) {
+                pt.corner[k] = (uint16_t)add(S.tri[3 * t + k]);
+                pt.nb[k] = nb[3 * t + k] < 0 ? kNoNb : (uint16_t)add(nb[3 * t + k]);
+                if (flip[3 * t + k]) pt.flip |= 1u << k;
+            }
+            std::copy_n(&S.tri_rest_f[4 * (size_t)t], 4, pt.rest);
+            std::copy_n(&bend[6 * (size_t)t], 6, pt.bend);
+            pt.area = S.tri_area_f[(size_t)t];
+            S.ptris.push_back(pt);
+        }
+        if (!fits || P.all >= 65535) {
+            S.patches.clear();
+            return;
+        }
+        for (int k = 0; k < P.own; ++k) {
+            const int v = code[(size_t)(first + k)].second;
+            S.pinc_off.push_back((uint16_t)((int)S.pinc.size() - P.inc0));
+            for (int e = S.inc_off[v]; e < S.inc_off[v + 1]; ++e) {
+                if ((S.inc[e] >> 29) != 1) continue;
+                const int t = S.inc[e] & ((1 << 29) - 1);
+                for (int c = 0; c < 3; ++c)
+                    if (S.tri[3 * t + c] == v) S.pinc.push_back((uint16_t)(3 * tri_local[(size_t)t] + c));
+            }
+        }
+        for (int k = P.own; k <= kPatchOwn; ++k) S.pinc_off.push_back((uint16_t)((int)S.pinc.size() - P.inc0));
+        for (size_t i = (size_t)P.verts0; i < S.pverts.size(); ++i) local[(size_t)S.pverts[i]] = -1;
+        P.incs = (int)S.pinc.size() - P.inc0;
+        const size_t smem = patch_smem_bytes(P.all, P.tris, P.incs);
+        if (smem > kMaxPatchSmem) {
+            S.patches.clear();
+            return;
+        }
+        S.patch_smem = std::max(S.patch_smem, smem);
+        S.patches.push_back(P);
+    }
+}
+
 bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv, int64_t nt, std::string& why) {
     S.rest.assign(xyz, xyz + 3 * nv);
     S.tri.resize(3 * nt);
@@ -172,6 +276,7 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
     S.link_len.clear();
     S.pairs.clear();
     S.pair_cs.clear();
+    std::vector<std::pair<int, int>> edge_of;  // the triangles of each pair
     for (auto& kv : links) {
         const int i0 = kv.first.first, i1 = kv.first.second;
         S.links.push_back(i0);
@@ -188,6 +293,7 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
         }
         const int q[4] = {a[0], a[1], a[2], b[2]};
         for (int k = 0; k < 4; ++k) S.pairs.push_back(q[k]);
+        edge_of.emplace_back(kv.second.t1, kv.second.t2);
         V3d p0 = P(q[0]), p1 = P(q[1]), p2 = P(q[2]), p3 = P(q[3]);
         V3d n1 = crs(sub(p1, p0), sub(p2, p0));
         n1 = scl(n1, nrm(n1));
@@ -249,6 +355,7 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
     });
     S.order.resize((size_t)nv);
     for (int64_t v = 0; v < nv; ++v) S.order[(size_t)v] = code[(size_t)v].second;
+    build_patches(S, edge_of);
     return true;
 }
 
@@ -381,6 +488,11 @@ void free_particles(Lattice& L) {
     cudaFree(L.pdev);
     cudaFree(L.vert_particle);
     cudaFree(L.visit_order);
+    cudaFree(L.patch_jobs);
+    L.patch_jobs = nullptr;
+    L.patch_jobs_host.clear();
+    L.npatch = 0;
+    L.patch_smem = 0;
     L.visit_order = nullptr;
     L.vel = L.force = L.stats = nullptr;
     L.pdev = nullptr;
@@ -483,6 +595,12 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
         d.tri4 = S.dev.tri4;
         d.tri_area_f = S.dev.tri_area_f;
         d.pair_cs_f = S.dev.pair_cs_f;
+        d.pf[0] = (float)ph.prm[BIB_P_G];
+        d.pf[1] = (float)ph.prm[BIB_P_C];
+        d.pf[2] = (float)ph.prm[BIB_P_K_BEND];
+        d.pf[3] = (float)ph.prm[BIB_P_K_AREA_LOCAL];
+        d.ka_a0 = ph.prm[BIB_P_K_AREA_GLOBAL] / S.area;
+        d.kv_vd = ph.prm[BIB_P_K_VOLUME] / ph.prm[BIB_P_VOL_DESIRED];
         d.inst = 0;
         d.lpid = p;
         d.A0 = S.area;
@@ -490,6 +608,32 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
         L.max_nv = std::max(L.max_nv, ph.nv);
         L.max_elems = std::max(L.max_elems, std::max(d.nt, std::max(d.nl, d.np)));
         L.max_nt = std::max(L.max_nt, d.nt);
+    }
+    // reduced precision: the membranes by patches, unless one has link springs or a shape has no patches
+    if (L.storage != BIB_STORAGE_F64) {
+        bool patched = true;
+        for (const ParticleHost& ph : L.parts)
+            patched = patched && ph.model != BIB_MODEL_RBC_WLCPOW && !c->shapes[ph.shape]->patches.empty();
+        for (int p = 0; p < np && patched; ++p) {
+            const ShapeHost& S = *c->shapes[L.parts[p].shape];
+            for (int k = 0; k < (int)S.patches.size(); ++k) {
+                const PatchDev& P = S.patches[(size_t)k];
+                PatchJob j{};
+                j.verts = S.dev.pverts + P.verts0;
+                j.tris = S.dev.ptris + P.tris0;
+                j.inc_off = S.dev.pinc_off + (kPatchOwn + 1) * k;
+                j.inc = S.dev.pinc + P.inc0;
+                j.part = p, j.v0 = L.parts[p].v0, j.inst = 0, j.lpid = p;
+                j.own = (uint16_t)P.own, j.all = (uint16_t)P.all, j.ntris = (uint16_t)P.tris, j.nincs = (uint16_t)P.incs;
+                L.patch_jobs_host.push_back(j);
+            }
+            L.patch_smem = std::max(L.patch_smem, S.patch_smem);
+        }
+        if (patched) {
+            L.npatch = (int)L.patch_jobs_host.size();
+            BIB_ALLOC(c, (void**)&L.patch_jobs, L.npatch * sizeof(PatchJob));
+            BIB_CUDA(c, cudaMemcpy(L.patch_jobs, L.patch_jobs_host.data(), L.npatch * sizeof(PatchJob), cudaMemcpyHostToDevice));
+        }
     }
     if (L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) {
         const int sup = L.ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
@@ -602,6 +746,18 @@ void record(bib_ctx* c, int idx) {
 }
 
 
+// Membrane and interaction forces at X_n and their spreading into F[fbuf], in one launch where the lattice
+// allows it (with profiling on always in separate ones, for the times of both).
+void membrane_and_spread(bib_ctx* c, Lattice& L, int fbuf, bool record_nodes, bool ib = true) {
+    cudaStream_t s = c->stream;
+    if (ib && !c->profiling && launch_membrane_spread(L, fbuf, s, record_nodes)) return;
+    if (ib) launch_membrane_forces(L, s);
+    if (ib) launch_pp_forces(L, s);
+    record(c, 1);
+    if (ib) launch_spread(L, fbuf, s, record_nodes);
+    record(c, 2);
+}
+
 // One coupled step.  The reference's driver order (progs/capsule_in_shear/capsule_in_shear.cpp:
 // 187-227) is computeVelocity -> setExternalVector -> [interpolate, compute + spread forces,
 // move] -> collideAndStream -> wall processors.  Forces at X_n do not depend on the velocity,
@@ -621,11 +777,7 @@ void enqueue_step(bib_ctx* c, Lattice& L, bool with_ib, bool with_lbm) {
     if (with_ib && with_lbm && ib && L.phase) {
         if (!L.target_clean) launch_force_fill(L, 1 - L.fe, s);
         record(c, 0);
-        launch_membrane_forces(L, s);
-        launch_pp_forces(L, s);
-        record(c, 1);
-        launch_spread(L, 1 - L.fe, s);
-        record(c, 2);
+        membrane_and_spread(c, L, 1 - L.fe, false);
         launch_velocity_field(L, s);
         launch_interpolate_move(L, s);
         launch_particle_update(L, s);
@@ -650,13 +802,9 @@ void enqueue_step(bib_ctx* c, Lattice& L, bool with_ib, bool with_lbm) {
         const bool sparse = ib && sparse_coupling(L);
         if (!L.target_clean) launch_force_fill(L, 1 - L.fe, s);
         record(c, 0);
-        if (ib) launch_membrane_forces(L, s);
-        if (ib) launch_pp_forces(L, s);
-        record(c, 1);
-        if (ib) launch_spread(L, 1 - L.fe, s, sparse);
+        membrane_and_spread(c, L, 1 - L.fe, sparse, ib);
         if (sparse) L.sparse_ok[1 - L.fe] = true;  // a clean target plus the recorded nodes
         else forces_touched(L);
-        record(c, 2);
         // dense: u of this state, collision with F[1-fe], F[fe] := body
         launch_collide_stream(L, sparse ? Coupling::kSparse : Coupling::kDense, s);
         record(c, 3);
@@ -687,11 +835,7 @@ void enqueue_step(bib_ctx* c, Lattice& L, bool with_ib, bool with_lbm) {
         launch_force_fill(L, L.fe, s);
         L.target_clean = false;
         forces_touched(L);
-        if (ib) launch_membrane_forces(L, s);
-        if (ib) launch_pp_forces(L, s);
-        record(c, 1);
-        if (ib) launch_spread(L, L.fe, s);
-        record(c, 2);
+        membrane_and_spread(c, L, L.fe, false, ib);
         record(c, 3);
         record(c, 4);
         if (ib) {
@@ -1017,6 +1161,9 @@ struct Batch {
     int* vinst = nullptr;
     int nparts = 0, nvert = 0, max_nv = 0;
     size_t membrane_smem = 0;
+    PatchJob* patch_jobs = nullptr;     // every patch of every particle, when all lattices are patched
+    int npatch = 0;
+    size_t patch_smem = 0;
     int64_t ntiles = 0;
     int any_fd = 0, nx_max = 0, nz_max = 0;
     int any_phase = 0;                  // a lattice voxelizes its particles into a phase field
@@ -1037,6 +1184,10 @@ struct Batch {
         }
         cudaFree(parts);
         cudaFree(vinst);
+        cudaFree(patch_jobs);
+        patch_jobs = nullptr;
+        npatch = 0;
+        patch_smem = 0;
         parts = nullptr;
         vinst = nullptr;
         built = false;
@@ -1063,6 +1214,8 @@ bib_status build_batch(bib_ctx* c, Batch& B) {
     std::vector<CollideView> cv[2];
     std::vector<ParticleDev> parts;
     std::vector<int> vinst;
+    std::vector<PatchJob> jobs;
+    bool patched = true;
     B.versions.assign(n, 0);
     B.state0.assign(n, 0);
     B.max_nv = 0;
@@ -1118,6 +1271,13 @@ bib_status build_batch(bib_ctx* c, Batch& B) {
         B.any_phase |= (L.phase && L.nvert) ? 1 : 0;
         B.nx_max = std::max(B.nx_max, L.d.nx);
         B.nz_max = std::max(B.nz_max, L.d.nz);
+        patched = patched && (L.nvert == 0 || L.npatch > 0);
+        B.patch_smem = std::max(B.patch_smem, L.patch_smem);
+        for (PatchJob j : L.patch_jobs_host) {
+            j.part += (int)parts.size();
+            j.inst = i;
+            jobs.push_back(j);
+        }
         for (size_t k = 0; k < L.pdev_host.size(); ++k) {
             ParticleDev d = L.pdev_host[k];
             d.inst = i;
@@ -1135,6 +1295,10 @@ bib_status build_batch(bib_ctx* c, Batch& B) {
     for (int p = 0; p < 2; ++p)
         if ((st = upload(c, &B.views[p], iv[p])) || (st = upload(c, &B.cviews[p], cv[p]))) return st;
     if ((st = upload(c, &B.parts, parts)) || (st = upload(c, &B.vinst, vinst))) return st;
+    if (patched && !jobs.empty()) {
+        if ((st = upload(c, &B.patch_jobs, jobs))) return st;
+        B.npatch = (int)jobs.size();
+    }
     B.phase = 0;
     B.built = true;
     return BIB_OK;
@@ -1188,6 +1352,9 @@ BatchLaunch batch_launch(bib_ctx* c, const Batch& B, int phase) {
     bl.nvert = B.nvert;
     bl.max_nv = B.max_nv;
     bl.membrane_smem = B.membrane_smem;
+    bl.patch_jobs = B.patch_jobs;
+    bl.npatch = B.npatch;
+    bl.patch_smem = B.patch_smem;
     bl.ntiles = B.ntiles;
     bl.stages = B.stages;
     bl.any_fd = B.any_fd;
@@ -1203,8 +1370,10 @@ BatchLaunch batch_launch(bib_ctx* c, const Batch& B, int phase) {
 // moved membranes), then collide-and-stream.  The interpolated velocity is the same either way.
 bib_status enqueue_batch_step(bib_ctx* c, Batch& B) {
     const BatchLaunch bl = batch_launch(c, B, B.phase);
-    launch_membrane_batch(bl, B.membrane_block, c->stream);
-    launch_spread_batch(bl, c->stream);
+    if (!launch_membrane_spread_batch(bl, c->stream)) {
+        launch_membrane_batch(bl, B.membrane_block, c->stream);
+        launch_spread_batch(bl, c->stream);
+    }
     if (B.any_phase) {
         for (int32_t h : B.handles) {
             Lattice& L = *get_lattice(c, h);
@@ -1381,6 +1550,11 @@ void bib_destroy(bib_ctx* c) {
         cudaFree(S->dev.tri4);
         cudaFree(S->dev.tri_area_f);
         cudaFree(S->dev.pair_cs_f);
+        cudaFree(S->dev.pverts);
+        cudaFree(S->dev.ptris);
+        cudaFree(S->dev.pinc_off);
+        cudaFree(S->dev.pinc);
+
     }
     for (int k = 0; k < 6; ++k)
         if (c->ev[k]) cudaEventDestroy(c->ev[k]);
@@ -1991,7 +2165,8 @@ bib_status bib_shape_store(bib_ctx* c, const double* xyz, const int64_t* tri, in
         (st = upload(c, &S->dev.pair_cs, S->pair_cs)) || (st = upload(c, &S->dev.inc_off, S->inc_off)) ||
         (st = upload(c, &S->dev.inc, S->inc)) || (st = upload(c, &S->dev.tri_rest_f, S->tri_rest_f)) ||
         (st = upload(c, &S->dev.tri_area_f, S->tri_area_f)) || (st = upload(c, &S->dev.pair_cs_f, S->pair_cs_f)) ||
-        (st = upload(c, &S->dev.tri4, S->tri4)))
+        (st = upload(c, &S->dev.tri4, S->tri4)) || (st = upload(c, &S->dev.pverts, S->pverts)) || (st = upload(c, &S->dev.ptris, S->ptris)) ||
+        (st = upload(c, &S->dev.pinc_off, S->pinc_off)) || (st = upload(c, &S->dev.pinc, S->pinc)))
         return st;
     S->dev.nv = (int)nv;
     S->dev.nt = (int)nt;

@@ -46,6 +46,42 @@ struct IbDesc {
     double pipe_y0 = 0.0, pipe_z0 = 0.0, pipe_r = 0.0;
 };
 
+// Patches of a shape for the reduced-precision membrane forces: up to 32 owned vertices each, the
+// vertices their triangles and those triangles' neighbours touch, and the triangles at the owned
+// vertices.  All indices are local to the patch; its vertices start with the owned ones.
+constexpr int kPatchOwn = 32;
+struct PatchDev {
+    int own, all, tris, incs;    // owned vertices, vertices, triangles, entries of their vertices' runs
+    int verts0, tris0, inc0;     // first entry in pverts, ptris, pinc
+};
+struct alignas(16) PatchTri {
+    uint16_t corner[3];          // vertices of the triangle
+    uint16_t nb[3];              // vertex of the neighbour across the edge opposite each corner (kNoNb: none)
+    uint32_t flip;               // bit k: the adjacent-triangle pair across the edge opposite corner k runs the other way
+    float rest[4];               // l0, l0', cos(phi0), sin(phi0)
+    float bend[6];               // cosine and sine of the rest angle across the edge opposite each corner
+    float area, pad;
+};
+static_assert(sizeof(PatchTri) == 64, "loaded as four 16-byte words");
+constexpr uint16_t kNoNb = 0xffff;
+// A patch of a particle, as its CTA needs it: one 64-byte load away from everything else.
+struct alignas(16) PatchJob {
+    const int* verts;
+    const PatchTri* tris;
+    const uint16_t* inc_off;
+    const uint16_t* inc;
+    int part, v0;                // particle, its first vertex
+    int inst, lpid;              // its lattice within a batch, its index there
+    uint16_t own, all, ntris, nincs;
+    int pad[2];
+};
+static_assert(sizeof(PatchJob) == 64, "loaded as four 16-byte words");
+// shared memory of a patch: relative positions and the triangles' corner forces
+constexpr size_t kMaxPatchSmem = 40 * 1024;
+inline size_t patch_smem_bytes(int all, int tris, int incs) {
+    return (3 * (size_t)all + 9 * (size_t)tris) * sizeof(float) + ((size_t)incs + 1) / 2 * 4;
+}
+
 // Geometry of one reference shape, device resident.
 struct ShapeDev {
     int nv, nt, nl, np;
@@ -64,6 +100,11 @@ struct ShapeDev {
     float* tri_rest_f;    // 4*nt: rest l0, l0', cos(phi0), sin(phi0) of each triangle
     float* tri_area_f;    // nt
     float* pair_cs_f;     // 2*np
+    // patches
+    int* pverts;
+    PatchTri* ptris;
+    uint16_t* pinc_off;   // kPatchOwn + 1 per patch: the owned vertices' runs in pinc
+    uint16_t* pinc;       // 3 * triangle + corner, in triangle order
 };
 
 // One particle as the device kernels see it.
@@ -84,6 +125,8 @@ struct ParticleDev {
     const float* tri_rest_f;
     const float* tri_area_f;
     const float* pair_cs_f;
+    float pf[4];          // G, C, bending modulus, local area modulus in FP32
+    double ka_a0, kv_vd;  // k_area_global / A0, k_volume / vol_desired
     int inst;             // lattice of the particle within a batch (0 for a single lattice)
     int lpid;             // particle index within its lattice
     double A0;
@@ -262,6 +305,11 @@ struct ShapeHost {
     std::vector<int> tri, tri4, links, pairs, inc_off, inc;
     std::vector<int> order;  // vertices in a spatially clustered order (Morton order of the rest shape)
     std::vector<float> tri_rest_f, tri_area_f, pair_cs_f;
+    std::vector<PatchDev> patches;
+    std::vector<int> pverts;
+    std::vector<PatchTri> ptris;
+    std::vector<uint16_t> pinc_off, pinc;
+    size_t patch_smem = 0;  // the largest patch's
     double area = 0, volume = 0;
     std::string tag;  // ParticleShape tag (ParticleShape.h:64), the shape's name in text output
     ShapeDev dev{};
@@ -329,6 +377,10 @@ struct Lattice {
     int max_nv = 0;
     int max_elems = 0;            // most triangles, links or pairs of one particle
     int max_nt = 0;               // most triangles of one particle
+    PatchJob* patch_jobs = nullptr;  // every patch of every particle; null: the membranes are not patched
+    std::vector<PatchJob> patch_jobs_host;
+    int npatch = 0;
+    size_t patch_smem = 0;
     double* upd_partial = nullptr;  // partial sums of the split update (particles x 64 x 5)
     bool particles_dirty = true;  // host copies below are authoritative until uploaded
     std::vector<double> host_pos;    // concatenated vertex positions
@@ -390,6 +442,9 @@ void launch_copy_f64(double* dst, const double* src, size_t n, cudaStream_t s);
 
 // ---- kernel launchers (ib_kernels.cu) ----
 void launch_membrane_forces(const Lattice& L, cudaStream_t s);
+// membrane forces and their spreading into F[fbuf] in one launch; false: not for this lattice (nothing done)
+bool launch_membrane_spread(const Lattice& L, int fbuf, cudaStream_t s, bool record = false);
+
 // spreading into F[fbuf]; with `record` the support nodes go to spread_lo[fbuf]
 void launch_spread(const Lattice& L, int fbuf, cudaStream_t s, bool record = false);
 // vel and pos[1-pcur] = pos + vel; fold >= 0: the velocity field is the sparse-reset form and
@@ -432,12 +487,16 @@ struct BatchLaunch {
     int nvert = 0;
     int max_nv = 0;
     size_t membrane_smem = 0;
+    const PatchJob* patch_jobs = nullptr;  // every patch of every particle, when all lattices are patched
+    int npatch = 0;
+    size_t patch_smem = 0;
     int64_t ntiles = 0;                 // staged tiles over all lattices
     int stages = 0;                     // staged pipeline depth (0 = automatic)
     int any_fd = 0;                     // some lattice has finite-difference walls
     int nx_max = 0, nz_max = 0;
     int* wait_err = nullptr;            // device word of the bounded waits
 };
+bool launch_membrane_spread_batch(const BatchLaunch& B, cudaStream_t s);  // false: not patched, nothing done
 IbView single_view(const Lattice& L, int fbuf);  // parities of L; fbuf < 0: no spreading target
 void launch_membrane_batch(const BatchLaunch& B, int block, cudaStream_t s);
 void launch_spread_batch(const BatchLaunch& B, cudaStream_t s);

@@ -529,23 +529,25 @@ struct SpreadVertex {
     int inst;          // batch: the lattice
 };
 
-template <class FT, int S, bool BATCH>
-__global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const IbView* __restrict__ views,
-                                                                const int* __restrict__ vinst, int nvert) {
+template <class FT, int S>
+struct SpreadTile {
+    SpreadVertex<FT, S> sv[kSpreadVerts];
+    int lo_rec[3][kSpreadVerts];  // first support node per axis for the sparse reset
+    unsigned inside[3];           // vertices inside the envelope, per axis
+};
+
+// The spreading of 32 vertices by a CTA of kSpreadThreads threads: lane l of the first three warps gives
+// vertex l of the tile, v (-1: none) of lattice `inst`, and its force; view(inst) is the lattice.
+template <class FT, int S, class View>
+__device__ __forceinline__ void spread_tile(SpreadTile<FT, S>& T, const View& view, int v, int inst, const FT* f) {
     using SV = SpreadVertex<FT, S>;
-    __shared__ SV sv[kSpreadVerts];
-    __shared__ int lo_rec[3][kSpreadVerts];  // first support node per axis for the sparse reset
-    __shared__ unsigned inside_m[3];         // vertices inside the envelope, per axis
-    const int a = threadIdx.x >> 5, lane = threadIdx.x & 31, g = blockIdx.x * kSpreadVerts + lane;
-    int v = 0, inst = 0;
+    const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (a < 3) {  // warp a prepares axis a of the 32 vertices
         constexpr int dirac = S == 4 ? BIB_DIRAC_PESKIN : BIB_DIRAC_ROMA;
         bool in = false;
-        if (g < nvert) {
-            inst = BATCH ? vinst[g] : 0;
-            const IbView& V = BATCH ? views[inst] : v1;
-            v = BATCH ? g - V.vbase : g;
-            SV& s = sv[lane];
+        if (v >= 0) {
+            const IbView& V = view(inst);
+            SV& s = T.sv[lane];
             const LatticeDesc& d = V.d;
             const int off = (int)V.ib.offset, per = a == 0 ? d.px : (a == 1 ? d.py : d.pz);
             const int N = a == 0 ? d.nx : (a == 1 ? d.ny : d.nz);
@@ -553,11 +555,10 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const
             in = inside_axis(per, N, dirac, p);
             const double x = p - V.ib.offset;
             const int64_t lo = (int64_t)ceil(x - half_support(dirac));
-            lo_rec[a][lane] = in ? record_lo(per, N, lo, off) : 0;
+            T.lo_rec[a][lane] = in ? record_lo(per, N, lo, off) : 0;
             if (a == 0) {
                 s.inst = inst;
                 s.gx = in ? remap_global(per, N, lo, off) : -1;
-                const FT f[3] = {(FT)V.force[3 * v], (FT)V.force[3 * v + 1], (FT)V.force[3 * v + 2]};
 #pragma unroll
                 for (int m = 0; m < S; ++m) {
                     const FT w = axis_weight<FT>(dirac, lo, x, m);
@@ -575,27 +576,26 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (lane == 0) inside_m[a] = m;
+        if (lane == 0) T.inside[a] = m;
     }
     __syncthreads();
-    const unsigned inside = inside_m[0] & inside_m[1] & inside_m[2];
     if (a == 0) {
-        const bool in = (inside >> lane) & 1u;
-        const IbView& V = BATCH ? views[inst] : v1;
-        const bool nodewise = g < nvert && (V.ib.has_pipe || (int)V.ib.offset > 0);
-        if (!in || nodewise) sv[lane].gx = -1;
-        if (g < nvert && V.spread_lo)
-            V.spread_lo[v] = in ? make_int4(lo_rec[0][lane], lo_rec[1][lane], lo_rec[2][lane], 1) : make_int4(0, 0, 0, 0);
+        const bool in = ((T.inside[0] & T.inside[1] & T.inside[2]) >> lane) & 1u;
+        const IbView& V = view(inst);
+        const bool nodewise = v >= 0 && (V.ib.has_pipe || (int)V.ib.offset > 0);
+        if (!in || nodewise) T.sv[lane].gx = -1;
+        if (v >= 0 && V.spread_lo)
+            V.spread_lo[v] = in ? make_int4(T.lo_rec[0][lane], T.lo_rec[1][lane], T.lo_rec[2][lane], 1) : make_int4(0, 0, 0, 0);
         if (in && nodewise) spread_vertex_nodes<FT, S>(V, V.pos + 3LL * v, V.force + 3LL * v);
     }
     __syncthreads();
     for (int it = threadIdx.x; it < kSpreadVerts * SV::ITEMS; it += kSpreadThreads) {
         const int t = it / SV::ITEMS, r = it - t * SV::ITEMS, row = r / SV::WORDS, j = r - row * SV::WORDS;
-        const SV& s = sv[t];
+        const SV& s = T.sv[t];
         if (s.gx < 0) continue;
         const int y = s.yo[row / S], z = s.zo[row % S];
         if (y < 0 || z < 0) continue;
-        const IbView& V = BATCH ? views[s.inst] : v1;
+        const IbView& V = view(s.inst);
         const int nx = V.d.nx;
         const FT wyz = s.wy[row / S] * s.wz[row % S];
         const int64_t cell0 = (int64_t)nx * (y + (int64_t)V.d.ny * z);
@@ -604,13 +604,13 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const
             const int64_t e0 = 3 * (cell0 + s.gx);
             if constexpr (sizeof(FT) == 4) {
                 const int o = (int)(e0 & 3);
-                float v[4];
+                float w[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int e = 4 * j + k - o;
-                    v[k] = e >= 0 && e < 3 * S ? s.p[e] * wyz : 0.0f;
+                    w[k] = e >= 0 && e < 3 * S ? s.p[e] * wyz : 0.0f;
                 }
-                if (4 * j - o < 3 * S) atomicAdd(reinterpret_cast<float4*>(F + (e0 - o)) + j, make_float4(v[0], v[1], v[2], v[3]));
+                if (4 * j - o < 3 * S) atomicAdd(reinterpret_cast<float4*>(F + (e0 - o)) + j, make_float4(w[0], w[1], w[2], w[3]));
             } else {
                 atomicAdd(F + e0 + j, s.p[j] * wyz);
             }
@@ -622,6 +622,24 @@ __global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const
             }
         }
     }
+}
+
+template <class FT, int S, bool BATCH>
+__global__ void __launch_bounds__(kSpreadThreads) k_spread_rows(IbView v1, const IbView* __restrict__ views,
+                                                                const int* __restrict__ vinst, int nvert) {
+    __shared__ SpreadTile<FT, S> T;
+    const int g = blockIdx.x * kSpreadVerts + (threadIdx.x & 31);
+    auto view = [&](int inst) -> const IbView& { return BATCH ? views[inst] : v1; };
+    int v = -1, inst = 0;
+    FT f[3] = {FT(0), FT(0), FT(0)};
+    if (threadIdx.x < 96 && g < nvert) {
+        if (BATCH) inst = vinst[g];
+        const IbView& V = view(inst);
+        v = BATCH ? g - V.vbase : g;
+        if (threadIdx.x < 32)
+            for (int q = 0; q < 3; ++q) f[q] = (FT)V.force[3 * v + q];
+    }
+    spread_tile<FT, S>(T, view, v, inst, f);
 }
 
 // Deterministic spreading.  Every (vertex, stencil node) pair becomes an entry keyed by its
@@ -903,6 +921,17 @@ __device__ __forceinline__ MemCoef<M> mem_coef(const ParticleDev& P, double area
     k.df_vol6 = (M)(P.prm[BIB_P_K_VOLUME] * (P.prm[BIB_P_VOL_DESIRED] - volume) / P.prm[BIB_P_VOL_DESIRED]) / M(6);
     return k;
 }
+// Rest state of one triangle at hand (the patch kernel), in place of the particle's tables.
+struct TriRest {
+    float4 rest;
+    float area;
+};
+__device__ __forceinline__ float4 rest_of(const ParticleDev& P, int t) { return reinterpret_cast<const float4*>(P.tri_rest_f)[t]; }
+__device__ __forceinline__ float4 rest_of(const TriRest& R, int) { return R.rest; }
+template <class M>
+__device__ __forceinline__ M tri_area_of(const TriRest& R, int) {
+    return R.area;
+}
 template <class M>
 __device__ __forceinline__ M tri_area_of(const ParticleDev& P, int t) {
     return sizeof(M) == sizeof(double) ? (M)P.tri_area[t] : (M)P.tri_area_f[t];
@@ -915,15 +944,15 @@ __device__ __forceinline__ M pair_c(const ParticleDev& P, int p, int k) {
 // DeformableCapsuleParticle::compute_forces for one triangle, src/fsi/DeformableCapsule.hh:68-148
 // (with the reference's c = l' sin(phi) / (l' sin(phi0)), line 96).  The rest-state lengths
 // and angle come from the FP64 rest mesh (M = double) or its FP32 copies.
-template <class M, class PS, class Sink>
-__device__ void capsule_triangle(const ParticleDev& P, int t, int4 ti, const PS& ps, int skalak, const MemCoef<M>& k,
+template <class M, class PD, class PS, class Sink>
+__device__ void capsule_triangle(const PD& P, int t, int4 ti, const PS& ps, int skalak, const MemCoef<M>& k,
                                  Sink& sk) {
     const int i0 = ti.x, i1 = ti.y, i2 = ti.z;
     const int id[3] = {i0, i1, i2};
     const V3<M> p0 = ps(i0), p1 = ps(i1), p2 = ps(i2);
     const V3<M> e0 = p1 - p0, e1 = p2 - p0;
     M l0, l0p, sin_phi_0, cos_phi_0;
-    if (sizeof(M) == sizeof(double)) {
+    if constexpr (sizeof(M) == sizeof(double)) {
         const V3<M> e0_0 = mk3<M>((M)(P.rest[3 * i1] - P.rest[3 * i0]), (M)(P.rest[3 * i1 + 1] - P.rest[3 * i0 + 1]),
                                   (M)(P.rest[3 * i1 + 2] - P.rest[3 * i0 + 2]));
         const V3<M> e1_0 = mk3<M>((M)(P.rest[3 * i2] - P.rest[3 * i0]), (M)(P.rest[3 * i2 + 1] - P.rest[3 * i0 + 1]),
@@ -933,7 +962,7 @@ __device__ void capsule_triangle(const ParticleDev& P, int t, int4 ti, const PS&
         sin_phi_0 = norm3(cross3(e0_0, e1_0)) / (l0 * l0p);
         cos_phi_0 = dot3(e0_0, e1_0) / (l0 * l0p);
     } else {
-        const float4 r = reinterpret_cast<const float4*>(P.tri_rest_f)[t];
+        const float4 r = rest_of(P, t);
         l0 = (M)r.x;
         l0p = (M)r.y;
         cos_phi_0 = (M)r.z;
@@ -1050,8 +1079,8 @@ __device__ void rbc_link(const ParticleDev& P, int l, const PS& ps, Sink& sk) {
 // src/fsi/RBCParticle.hh:175-213 with tri::triangle_area_and_gradient and
 // tri::grad_signed_volume (TriangleUtils.h:58-120).  The volume gradient is
 // translation invariant on a closed surface, so it is taken relative to the centre.
-template <class M, class PS, class Sink>
-__device__ void rbc_triangle(const ParticleDev& P, int t, int4 ti, const PS& ps, const MemCoef<M>& k, Sink& sk) {
+template <class M, class PD, class PS, class Sink>
+__device__ void rbc_triangle(const PD& P, int t, int4 ti, const PS& ps, const MemCoef<M>& k, Sink& sk) {
     const int i0 = ti.x, i1 = ti.y, i2 = ti.z;
     const V3<M> v0 = ps(i0), v1 = ps(i1), v2 = ps(i2);
     const M v01v11 = v0.y - v1.y, v02v22 = v0.z - v2.z, v02v12 = v0.z - v1.z;
@@ -1215,6 +1244,151 @@ __global__ void __launch_bounds__(512) k_membrane(const ParticleDev* __restrict_
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const ParticleDev& P = parts[blockIdx.x];
     membrane_block<M>(P, BATCH ? views[P.inst] : v1, smem_raw);
+}
+
+// Bending across one edge of a triangle, its share on the triangle's own corners: v1 is the corner
+// opposite the edge v0 v2, v3 the neighbour's vertex across it, n1 = (v1 - v0) x (v2 - v0) with its length
+// n1n.  The forces are along n1 (rbc_pair: the terms of n1u), as factors of its unit vector on v0, v1, v2.
+template <class M>
+__device__ __forceinline__ void bend_side(V3<M> v0, V3<M> v1, V3<M> v2, V3<M> v3, V3<M> n1, M n1n, V3<M> n1u, M kb, M c0, M c1,
+                                          M* s) {
+    const V3<M> e0 = v1 - v0, e1 = v2 - v0, e2 = v3 - v0;
+    const M e1n = norm3(e1);
+    const V3<M> e1u = div3(e1, e1n);
+    const V3<M> n2 = cross3(e1, e2);
+    const V3<M> n2u = div3(n2, norm3(n2));
+    const M cos_t = dot3(n1u, n2u);
+    const M sin_t = (dot3(n1 - n2, v1 - v3) > M(0) ? M(1) : M(-1)) * norm3(cross3(n1u, n2u));
+    const M pref = fast_div(kb * (-c0 * sin_t + c1 * cos_t), n1n);
+    s[0] = pref * dot3(e1u, e1 - e0);
+    s[1] = pref * -e1n;
+    s[2] = pref * dot3(e1u, e0);
+}
+
+// Membrane forces by patches (reduced precision), one CTA per patch of 32 owned vertices.  The CTA stages
+// the positions that the patch's triangles and their neighbours need, evaluates every triangle at an owned
+// vertex once (capsule law, area and volume penalties, and the triangle's own share of the bending across
+// its three edges) into shared memory, and adds up the corners of each owned vertex in triangle order:
+// no atomics, the same bits on every run.  SPREAD: the forces go straight on into the force field.
+// Bound by instruction issue, and by the FP64 pipe for the staging and the delta offsets.  A triangle on a
+// patch boundary is evaluated by each of its patches (1.5 evaluations per triangle).  One CTA per particle
+// with a shared-memory float atomic for each corner of each triangle and adjacent-triangle pair: 400 cells
+// of 642 vertices 45.8 us plus 37.4 us of spreading, in one launch here 81.8; 200 cells with the 4-point kernel
+// 41.2 + 34.8, here 55.7; one of 2562 vertices 20.8 + 2.3 (seeding) + 6.4, here 10.8.  One thread per vertex evaluating
+// all its elements (the deterministic mode): 260 cells 199 us, here 34.5.  At 59 % of the issue slots with 7 CTAs
+// per SM; 5 take 95 us for the 400 cells, 8 (64 registers, spills) the same.
+template <int S, bool BATCH, bool SPREAD>
+__global__ void __launch_bounds__(kSpreadThreads, 7) k_membrane_patch(const PatchJob* __restrict__ jobs,
+                                                                      const ParticleDev* __restrict__ parts, IbView v1,
+                                                                      const IbView* __restrict__ views) {
+    static_assert(kPatchOwn == kSpreadVerts, "a patch is a tile of the spreading");
+    extern __shared__ __align__(16) float dyn[];
+    __shared__ SpreadTile<float, S> T;
+    __shared__ float wall[3][kPatchOwn];
+    __shared__ MemCoef<float> kc;
+    __shared__ float own_f[3][kPatchOwn];
+    __shared__ uint16_t inc_off[kPatchOwn + 1];
+    const PatchJob& J = jobs[blockIdx.x];
+    const ParticleDev& P = parts[J.part];
+    const IbView& V = BATCH ? views[J.inst] : v1;
+    const double* st = V.stats + STATS * J.lpid;
+    const double* pos = V.pos + 3LL * J.v0;
+    const int* verts = J.verts;
+    const int own = J.own, all = J.all, ntris = J.ntris;
+    float* sp = dyn;
+    float* tf = dyn + 3 * all;
+    uint16_t* inc = reinterpret_cast<uint16_t*>(tf + 9 * ntris);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the thread's first triangle is loaded along with the positions
+    uint4 raw[4];
+    auto load_tri = [&](int i) {
+        const uint4* q = reinterpret_cast<const uint4*>(J.tris + i);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) raw[w] = __ldg(q + w);
+    };
+    if ((int)threadIdx.x < ntris) load_tri(threadIdx.x);
+    for (int i = threadIdx.x; i < J.nincs; i += kSpreadThreads) inc[i] = J.inc[i];
+    if (threadIdx.x <= kPatchOwn) inc_off[threadIdx.x] = J.inc_off[threadIdx.x];
+    // positions relative to the centre of mass: exact FP64 subtraction, then rounding
+    for (int i = threadIdx.x; i < all; i += kSpreadThreads) {
+        const double* p = pos + 3LL * verts[i];
+        sp[3 * i] = (float)(p[0] - st[2]);
+        sp[3 * i + 1] = (float)(p[1] - st[3]);
+        sp[3 * i + 2] = (float)(p[2] - st[4]);
+    }
+    if (threadIdx.x == 0) {
+        kc.G = P.pf[0];
+        kc.C = P.pf[1];
+        kc.kb = P.pf[2];
+        kc.k_area_local = P.pf[3];
+        kc.df_area_global = (float)(P.ka_a0 * (P.A0 - st[0]));
+        kc.df_vol6 = (float)(P.kv_vd * (P.prm[BIB_P_VOL_DESIRED] - st[1])) / 6.0f;
+    }
+    // the force decorators come first (ImmersedBoundaryDynamics_forces.hh:293-296)
+    if (warp == 3 && V.inter.nwall > 0 && lane < own) {
+        double fw[3];
+        wall_force(V.inter, pos + 3LL * verts[lane], fw);
+        for (int q = 0; q < 3; ++q) wall[q][lane] = (float)fw[q];
+    }
+    const int skalak = P.model != BIB_MODEL_CAPSULE_NEOHOOKEAN;
+    const bool rbc_terms = P.model == BIB_MODEL_SKALAK_BENDING;
+    const int v = warp < 3 && lane < own ? J.v0 + verts[lane] : -1;
+    __syncthreads();
+    const MemCoef<float> k = kc;
+    const SharedPos<float> ps{sp};
+    for (int i = threadIdx.x; i < ntris; i += kSpreadThreads) {
+        if (i >= kSpreadThreads) load_tri(i);
+        const int c[3] = {(int)(raw[0].x & 0xffffu), (int)(raw[0].x >> 16), (int)(raw[0].y & 0xffffu)};
+        const int nb[3] = {(int)(raw[0].y >> 16), (int)(raw[0].z & 0xffffu), (int)(raw[0].z >> 16)};
+        const TriRest R{make_float4(__uint_as_float(raw[1].x), __uint_as_float(raw[1].y), __uint_as_float(raw[1].z),
+                                    __uint_as_float(raw[1].w)),
+                        __uint_as_float(raw[3].z)};
+        const float bend[6] = {__uint_as_float(raw[2].x), __uint_as_float(raw[2].y), __uint_as_float(raw[2].z),
+                               __uint_as_float(raw[2].w), __uint_as_float(raw[3].x), __uint_as_float(raw[3].y)};
+        const V3<float> z = mk3<float>(0, 0, 0);
+        CornerSink<float> cs{{c[0], c[1], c[2]}, {z, z, z}};
+        const int4 ti = make_int4(c[0], c[1], c[2], 0);
+        capsule_triangle<float>(R, 0, ti, ps, skalak, k, cs);
+        if (rbc_terms) {
+            rbc_triangle<float>(R, 0, ti, ps, k, cs);
+            const V3<float> p[3] = {ps(c[0]), ps(c[1]), ps(c[2])};
+            const V3<float> n = cross3(p[1] - p[0], p[2] - p[0]);
+            const float nn = norm3(n);
+            const V3<float> nu = div3(n, nn);
+            float along[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                if (nb[e] == kNoNb) continue;
+                const bool flip = (raw[0].w >> e) & 1u;  // the pair runs against the triangle: n1 turns over
+                const V3<float> a = p[(e + 2) % 3], b = p[(e + 1) % 3];
+                const V3<float> v0 = flip ? b : a, v2 = flip ? a : b;
+                const float sign = flip ? -1.0f : 1.0f;
+                float s[3];
+                bend_side<float>(v0, p[e], v2, ps(nb[e]), sign * n, nn, sign * nu, k.kb, bend[2 * e], bend[2 * e + 1], s);
+                along[e] += sign * s[1];
+                along[(e + 2) % 3] += sign * (flip ? s[2] : s[0]);
+                along[(e + 1) % 3] += sign * (flip ? s[0] : s[2]);
+            }
+            for (int e = 0; e < 3; ++e) cs.f[e] = cs.f[e] + along[e] * nu;
+        }
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            tf[9 * i + 3 * e] = cs.f[e].x;
+            tf[9 * i + 3 * e + 1] = cs.f[e].y;
+            tf[9 * i + 3 * e + 2] = cs.f[e].z;
+        }
+    }
+    __syncthreads();
+    if (v >= 0) {  // one component of an owned vertex per thread
+        float sum = V.inter.nwall > 0 ? wall[warp][lane] : 0.0f;
+        for (int e = inc_off[lane]; e < inc_off[lane + 1]; ++e) sum += tf[3 * inc[e] + warp];
+        V.force[3LL * v + warp] = (double)sum;
+        own_f[warp][lane] = sum;
+    }
+    if (!SPREAD) return;
+    __syncthreads();
+    const float f[3] = {own_f[0][lane], own_f[1][lane], own_f[2][lane]};
+    spread_tile<float, S>(T, [&](int) -> const IbView& { return V; }, v, 0, f);
 }
 
 // Deterministic membrane forces: one thread per vertex sums the contributions of its
@@ -1847,9 +2021,36 @@ int membrane_split(int np, int max_elems, int block) {
     return std::max(1, std::min(want, most));
 }
 
+namespace {
+template <bool SPREAD, bool BATCH>
+void patch_launch(int dirac, const PatchJob* jobs, const ParticleDev* parts, int npatch, size_t smem, const IbView& v,
+                  const IbView* views, cudaStream_t s) {
+    if (dirac == BIB_DIRAC_PESKIN) k_membrane_patch<4, BATCH, SPREAD><<<npatch, kSpreadThreads, smem, s>>>(jobs, parts, v, views);
+    else k_membrane_patch<3, BATCH, SPREAD><<<npatch, kSpreadThreads, smem, s>>>(jobs, parts, v, views);
+}
+}  // namespace
+
+bool launch_membrane_spread(const Lattice& L, int fbuf, cudaStream_t s, bool record) {
+    if (L.npatch == 0 || L.inter.npp > 0 || L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) return false;
+    IbView v = single_view(L, fbuf);
+    v.spread_lo = record ? L.spread_lo[fbuf] : nullptr;
+    patch_launch<true, false>(L.ib.dirac, L.patch_jobs, L.pdev, L.npatch, L.patch_smem, v, nullptr, s);
+    return true;
+}
+
+bool launch_membrane_spread_batch(const BatchLaunch& B, cudaStream_t s) {
+    if (B.npatch == 0) return false;
+    patch_launch<true, true>(B.dirac, B.patch_jobs, B.parts, B.npatch, B.patch_smem, IbView{}, B.views, s);
+    return true;
+}
+
 void launch_membrane_forces(const Lattice& L, cudaStream_t s) {
     const int np = (int)L.parts.size();
     if (np == 0) return;
+    if (L.npatch > 0) {
+        patch_launch<false, false>(L.ib.dirac, L.patch_jobs, L.pdev, L.npatch, L.patch_smem, single_view(L, -1), nullptr, s);
+        return;
+    }
     if (L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) {
         const unsigned g = (L.nvert + 127) / 128;
         if (L.storage == BIB_STORAGE_F64)
