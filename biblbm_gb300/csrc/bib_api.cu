@@ -163,7 +163,10 @@ void build_patches(ShapeHost& S, const std::vector<std::pair<int, int>>& edge_of
         code[(size_t)v] = {m, v};
     }
     std::sort(code.begin(), code.end());
-    std::vector<int> local((size_t)nv, -1), tri_local((size_t)nt, -1);
+    std::vector<int> local((size_t)nv, -1), seen((size_t)nt, -1), tri_local((size_t)nt, -1), tris;
+    S.ptris.reserve(2 * (size_t)nt);
+    S.pverts.reserve(4 * (size_t)nv);
+    S.pinc.reserve(3 * (size_t)nt);
     for (int first = 0; first < nv; first += kPatchOwn) {
         PatchDev P{};
         P.own = std::min(kPatchOwn, nv - first);
@@ -176,14 +179,17 @@ void build_patches(ShapeHost& S, const std::vector<std::pair<int, int>>& edge_of
             return local[(size_t)v];
         };
         for (int k = 0; k < P.own; ++k) add(code[(size_t)(first + k)].second);
-        std::vector<int> tris;
+        tris.clear();
         for (int k = 0; k < P.own; ++k) {
             const int v = code[(size_t)(first + k)].second;
-            for (int e = S.inc_off[v]; e < S.inc_off[v + 1]; ++e)
-                if ((S.inc[e] >> 29) == 1) tris.push_back(S.inc[e] & ((1 << 29) - 1));
+            for (int e = S.inc_off[v]; e < S.inc_off[v + 1]; ++e) {
+                const int t = S.inc[e] & ((1 << 29) - 1);
+                if ((S.inc[e] >> 29) != 1 || seen[(size_t)t] == first) continue;
+                seen[(size_t)t] = first;
+                tris.push_back(t);
+            }
         }
         std::sort(tris.begin(), tris.end());
-        tris.erase(std::unique(tris.begin(), tris.end()), tris.end());
         P.tris = (int)tris.size();
         bool fits = 3 * tris.size() < 65535;
         for (int i = 0; i < P.tris && fits; ++i) {
@@ -302,19 +308,20 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
         S.pair_cs.push_back(dt(n1, n2));
         S.pair_cs.push_back((dt(sub(n1, n2), sub(p1, p3)) > 0 ? 1.0 : -1.0) * nrm(crs(n1, n2)));
     }
-    // FP32 copies of the rest-state constants for the reduced-precision element kernels
-    S.tri_rest_f.resize(4 * nt);
-    S.tri_area_f.resize(nt);
+    // rest lengths and angle of every triangle, and FP32 copies of the rest-state constants for the
+    // reduced-precision element kernels
+    S.tri_rest.resize(4 * nt);
     for (int64_t t = 0; t < nt; ++t) {
         const V3d a = P(S.tri[3 * t]), b = P(S.tri[3 * t + 1]), c = P(S.tri[3 * t + 2]);
         const V3d e0 = sub(b, a), e1 = sub(c, a);
         const double l0 = nrm(e0), l0p = nrm(e1);
-        S.tri_rest_f[4 * t] = (float)l0;
-        S.tri_rest_f[4 * t + 1] = (float)l0p;
-        S.tri_rest_f[4 * t + 2] = (float)(dt(e0, e1) / (l0 * l0p));
-        S.tri_rest_f[4 * t + 3] = (float)(nrm(crs(e0, e1)) / (l0 * l0p));
-        S.tri_area_f[t] = (float)S.tri_area[t];
+        S.tri_rest[4 * t] = l0;
+        S.tri_rest[4 * t + 1] = l0p;
+        S.tri_rest[4 * t + 2] = dt(e0, e1) / (l0 * l0p);
+        S.tri_rest[4 * t + 3] = nrm(crs(e0, e1)) / (l0 * l0p);
     }
+    S.tri_rest_f.assign(S.tri_rest.begin(), S.tri_rest.end());
+    S.tri_area_f.assign(S.tri_area.begin(), S.tri_area.end());
     S.pair_cs_f.assign(S.pair_cs.begin(), S.pair_cs.end());
     S.tri4.assign(4 * nt, 0);
     for (int64_t t = 0; t < nt; ++t)
@@ -369,6 +376,42 @@ bib_status upload(bib_ctx* c, T** dptr, const std::vector<T>& v) {
 }
 
 // DeformableParticle3D::update (DeformableParticle3D.hh:54-82) on the host, FP64.
+// The tables of a shape in one allocation (S.dev.base).
+bib_status upload_shape(bib_ctx* c, ShapeHost& S) {
+    std::vector<unsigned char> all;
+    std::vector<std::pair<void**, size_t>> at;
+    auto put = [&](auto** dptr, const auto& v) {
+        *dptr = nullptr;
+        if (v.empty()) return;
+        all.resize((all.size() + 255) / 256 * 256);
+        at.emplace_back(reinterpret_cast<void**>(dptr), all.size());
+        const unsigned char* p = reinterpret_cast<const unsigned char*>(v.data());
+        all.insert(all.end(), p, p + v.size() * sizeof(v[0]));
+    };
+    ShapeDev& d = S.dev;
+    put(&d.tri, S.tri);
+    put(&d.tri4, S.tri4);
+    put(&d.tri_area, S.tri_area);
+    put(&d.links, S.links);
+    put(&d.link_len, S.link_len);
+    put(&d.pairs, S.pairs);
+    put(&d.pair_cs, S.pair_cs);
+    put(&d.inc_off, S.inc_off);
+    put(&d.inc, S.inc);
+    put(&d.tri_rest, S.tri_rest);
+    put(&d.tri_rest_f, S.tri_rest_f);
+    put(&d.tri_area_f, S.tri_area_f);
+    put(&d.pair_cs_f, S.pair_cs_f);
+    put(&d.ptris, S.ptris);
+    put(&d.pverts, S.pverts);
+    put(&d.pinc_off, S.pinc_off);
+    put(&d.pinc, S.pinc);
+    bib_status st = upload(c, &d.base, all);
+    if (st) return st;
+    for (auto& f : at) *f.first = d.base + f.second;
+    return BIB_OK;
+}
+
 void particle_update(const ShapeHost& S, const double* pos, double* st) {
     double area = 0, vol = 0, cx = 0, cy = 0, cz = 0;
     const int nt = (int)S.tri_area.size();
@@ -488,8 +531,7 @@ void free_particles(Lattice& L) {
     cudaFree(L.pdev);
     cudaFree(L.vert_particle);
     cudaFree(L.visit_order);
-    cudaFree(L.patch_jobs);
-    L.patch_jobs = nullptr;
+    L.patch_jobs = nullptr;  // within pdev
     L.patch_jobs_host.clear();
     L.npatch = 0;
     L.patch_smem = 0;
@@ -582,7 +624,6 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
         d.nt = (int)S.tri_area.size();
         d.nl = (int)S.link_len.size();
         d.np = (int)S.pair_cs.size() / 2;
-        d.rest = S.dev.rest;
         d.tri = S.dev.tri;
         d.tri_area = S.dev.tri_area;
         d.links = S.dev.links;
@@ -591,6 +632,7 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
         d.pair_cs = S.dev.pair_cs;
         d.inc_off = S.dev.inc_off;
         d.inc = S.dev.inc;
+        d.tri_rest = S.dev.tri_rest;
         d.tri_rest_f = S.dev.tri_rest_f;
         d.tri4 = S.dev.tri4;
         d.tri_area_f = S.dev.tri_area_f;
@@ -631,8 +673,6 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
         }
         if (patched) {
             L.npatch = (int)L.patch_jobs_host.size();
-            BIB_ALLOC(c, (void**)&L.patch_jobs, L.npatch * sizeof(PatchJob));
-            BIB_CUDA(c, cudaMemcpy(L.patch_jobs, L.patch_jobs_host.data(), L.npatch * sizeof(PatchJob), cudaMemcpyHostToDevice));
         }
     }
     if (L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) {
@@ -661,8 +701,15 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
         BIB_ALLOC(c, (void**)&L.visit_order, L.nvert * sizeof(int));
         BIB_CUDA(c, cudaMemcpy(L.visit_order, vp.data(), L.nvert * sizeof(int), cudaMemcpyHostToDevice));
     }
-    BIB_ALLOC(c, (void**)&L.pdev, np * sizeof(ParticleDev));
-    BIB_CUDA(c, cudaMemcpy(L.pdev, pd.data(), np * sizeof(ParticleDev), cudaMemcpyHostToDevice));
+    {  // the particles and, behind them, the patch jobs
+        const size_t pb = ((size_t)np * sizeof(ParticleDev) + 63) / 64 * 64, jb = (size_t)L.npatch * sizeof(PatchJob);
+        std::vector<unsigned char> both(pb + jb);
+        std::memcpy(both.data(), pd.data(), (size_t)np * sizeof(ParticleDev));
+        if (jb) std::memcpy(both.data() + pb, L.patch_jobs_host.data(), jb);
+        BIB_ALLOC(c, (void**)&L.pdev, both.size());
+        BIB_CUDA(c, cudaMemcpy(L.pdev, both.data(), both.size(), cudaMemcpyHostToDevice));
+        if (jb) L.patch_jobs = reinterpret_cast<PatchJob*>(reinterpret_cast<unsigned char*>(L.pdev) + pb);
+    }
     L.pdev_host = pd;
     L.membrane_smem = membrane_smem_bytes(L.max_nv);
     int dev_max = 0;
@@ -1537,24 +1584,7 @@ void bib_destroy(bib_ctx* c) {
         cudaFree(Lp->guo);
     }
     for (auto& S : c->shapes) {
-        cudaFree(S->dev.rest);
-        cudaFree(S->dev.tri);
-        cudaFree(S->dev.tri_area);
-        cudaFree(S->dev.links);
-        cudaFree(S->dev.link_len);
-        cudaFree(S->dev.pairs);
-        cudaFree(S->dev.pair_cs);
-        cudaFree(S->dev.inc_off);
-        cudaFree(S->dev.inc);
-        cudaFree(S->dev.tri_rest_f);
-        cudaFree(S->dev.tri4);
-        cudaFree(S->dev.tri_area_f);
-        cudaFree(S->dev.pair_cs_f);
-        cudaFree(S->dev.pverts);
-        cudaFree(S->dev.ptris);
-        cudaFree(S->dev.pinc_off);
-        cudaFree(S->dev.pinc);
-
+        cudaFree(S->dev.base);
     }
     for (int k = 0; k < 6; ++k)
         if (c->ev[k]) cudaEventDestroy(c->ev[k]);
@@ -2159,15 +2189,7 @@ bib_status bib_shape_store(bib_ctx* c, const double* xyz, const int64_t* tri, in
     std::string why;
     if (!build_shape(*S, xyz, tri, nv, nt, why)) return fail(c, BIB_EINVAL, "invalid mesh: %s", why.c_str());
     bib_status st;
-    if ((st = upload(c, &S->dev.rest, S->rest)) || (st = upload(c, &S->dev.tri, S->tri)) ||
-        (st = upload(c, &S->dev.tri_area, S->tri_area)) || (st = upload(c, &S->dev.links, S->links)) ||
-        (st = upload(c, &S->dev.link_len, S->link_len)) || (st = upload(c, &S->dev.pairs, S->pairs)) ||
-        (st = upload(c, &S->dev.pair_cs, S->pair_cs)) || (st = upload(c, &S->dev.inc_off, S->inc_off)) ||
-        (st = upload(c, &S->dev.inc, S->inc)) || (st = upload(c, &S->dev.tri_rest_f, S->tri_rest_f)) ||
-        (st = upload(c, &S->dev.tri_area_f, S->tri_area_f)) || (st = upload(c, &S->dev.pair_cs_f, S->pair_cs_f)) ||
-        (st = upload(c, &S->dev.tri4, S->tri4)) || (st = upload(c, &S->dev.pverts, S->pverts)) || (st = upload(c, &S->dev.ptris, S->ptris)) ||
-        (st = upload(c, &S->dev.pinc_off, S->pinc_off)) || (st = upload(c, &S->dev.pinc, S->pinc)))
-        return st;
+    if ((st = upload_shape(c, *S))) return st;
     S->dev.nv = (int)nv;
     S->dev.nt = (int)nt;
     S->dev.nl = (int)S->link_len.size();

@@ -84,9 +84,9 @@ inline size_t patch_smem_bytes(int all, int tris, int incs) {
 
 // Geometry of one reference shape, device resident.
 struct ShapeDev {
+    unsigned char* base;  // the allocation that holds the tables below
     int nv, nt, nl, np;
     double area, volume;  // rest area A0 and volume V0
-    double* rest;         // 3*nv
     int* tri;             // 3*nt
     int* tri4;            // 4*nt: the corners of each triangle and a pad, for 16-byte loads
     double* tri_area;     // nt
@@ -96,8 +96,9 @@ struct ShapeDev {
     double* pair_cs;      // 2*np
     int* inc_off;         // nv+1: per-vertex incidence lists (links, triangles, pairs)
     int* inc;             // (type << 29) | element id
+    double* tri_rest;     // 4*nt: rest l0, l0', cos(phi0), sin(phi0) of each triangle
     // FP32 copies for the reduced-precision element kernels
-    float* tri_rest_f;    // 4*nt: rest l0, l0', cos(phi0), sin(phi0) of each triangle
+    float* tri_rest_f;    // 4*nt
     float* tri_area_f;    // nt
     float* pair_cs_f;     // 2*np
     // patches
@@ -112,7 +113,6 @@ struct ParticleDev {
     int shape, model;
     int v0, nv;           // first vertex in the concatenated vertex arrays, vertex count
     int nt, nl, np;
-    const double* rest;
     const int* tri;
     const int* tri4;
     const double* tri_area;
@@ -122,6 +122,7 @@ struct ParticleDev {
     const double* pair_cs;
     const int* inc_off;
     const int* inc;
+    const double* tri_rest;
     const float* tri_rest_f;
     const float* tri_area_f;
     const float* pair_cs_f;
@@ -301,7 +302,7 @@ struct CollideView {
 };
 
 struct ShapeHost {
-    std::vector<double> rest, tri_area, link_len, pair_cs;
+    std::vector<double> rest, tri_area, link_len, pair_cs, tri_rest;
     std::vector<int> tri, tri4, links, pairs, inc_off, inc;
     std::vector<int> order;  // vertices in a spatially clustered order (Morton order of the rest shape)
     std::vector<float> tri_rest_f, tri_area_f, pair_cs_f;

@@ -845,16 +845,13 @@ __device__ __forceinline__ V3<M> operator-(V3<M> a, V3<M> b) { return mk3(a.x - 
 template <class M>
 __device__ __forceinline__ V3<M> operator*(M s, V3<M> a) { return mk3(s * a.x, s * a.y, s * a.z); }
 template <class M>
-__device__ __forceinline__ V3<M> operator/(V3<M> a, M s) { return mk3(a.x / s, a.y / s, a.z / s); }
-template <class M>
 __device__ __forceinline__ M dot3(V3<M> a, V3<M> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 template <class M>
 __device__ __forceinline__ M norm3(V3<M> a) { return fast_sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
-// a / s: one approximate reciprocal in FP32, the three IEEE divisions in FP64
+// a / s by one reciprocal (approximate in FP32)
 template <class M>
 __device__ __forceinline__ V3<M> div3(V3<M> a, M s) {
-    if constexpr (sizeof(M) == sizeof(float)) return fast_rcp(s) * a;
-    else return a / s;
+    return fast_rcp(s) * a;
 }
 template <class M>
 __device__ __forceinline__ V3<M> cross3(V3<M> a, V3<M> b) {
@@ -926,8 +923,24 @@ struct TriRest {
     float4 rest;
     float area;
 };
-__device__ __forceinline__ float4 rest_of(const ParticleDev& P, int t) { return reinterpret_cast<const float4*>(P.tri_rest_f)[t]; }
-__device__ __forceinline__ float4 rest_of(const TriRest& R, int) { return R.rest; }
+template <class M>
+struct Rest4 {
+    M x, y, z, w;
+};
+template <class M>
+__device__ __forceinline__ Rest4<M> rest_of(const ParticleDev& P, int t) {
+    if constexpr (sizeof(M) == sizeof(double)) {
+        const double2 a = reinterpret_cast<const double2*>(P.tri_rest)[2 * t], b = reinterpret_cast<const double2*>(P.tri_rest)[2 * t + 1];
+        return {a.x, a.y, b.x, b.y};
+    } else {
+        const float4 r = reinterpret_cast<const float4*>(P.tri_rest_f)[t];
+        return {r.x, r.y, r.z, r.w};
+    }
+}
+template <class M>
+__device__ __forceinline__ Rest4<M> rest_of(const TriRest& R, int) {
+    return {R.rest.x, R.rest.y, R.rest.z, R.rest.w};
+}
 template <class M>
 __device__ __forceinline__ M tri_area_of(const TriRest& R, int) {
     return R.area;
@@ -948,109 +961,54 @@ template <class M, class PD, class PS, class Sink>
 __device__ void capsule_triangle(const PD& P, int t, int4 ti, const PS& ps, int skalak, const MemCoef<M>& k,
                                  Sink& sk) {
     const int i0 = ti.x, i1 = ti.y, i2 = ti.z;
-    const int id[3] = {i0, i1, i2};
     const V3<M> p0 = ps(i0), p1 = ps(i1), p2 = ps(i2);
     const V3<M> e0 = p1 - p0, e1 = p2 - p0;
-    M l0, l0p, sin_phi_0, cos_phi_0;
-    if constexpr (sizeof(M) == sizeof(double)) {
-        const V3<M> e0_0 = mk3<M>((M)(P.rest[3 * i1] - P.rest[3 * i0]), (M)(P.rest[3 * i1 + 1] - P.rest[3 * i0 + 1]),
-                                  (M)(P.rest[3 * i1 + 2] - P.rest[3 * i0 + 2]));
-        const V3<M> e1_0 = mk3<M>((M)(P.rest[3 * i2] - P.rest[3 * i0]), (M)(P.rest[3 * i2 + 1] - P.rest[3 * i0 + 1]),
-                                  (M)(P.rest[3 * i2 + 2] - P.rest[3 * i0 + 2]));
-        l0 = norm3(e0_0);
-        l0p = norm3(e1_0);
-        sin_phi_0 = norm3(cross3(e0_0, e1_0)) / (l0 * l0p);
-        cos_phi_0 = dot3(e0_0, e1_0) / (l0 * l0p);
-    } else {
-        const float4 r = rest_of(P, t);
-        l0 = (M)r.x;
-        l0p = (M)r.y;
-        cos_phi_0 = (M)r.z;
-        sin_phi_0 = (M)r.w;
-    }
-    if constexpr (sizeof(M) == sizeof(float)) {
-        // The same forces with the corner-independent scalars gathered: every gradient of
-        // D11, D22, D12 (hence of I1, I2) is a combination of the corner gradients of
-        // l, l' and cos(phi) (gl, glp, gc below), so f_i = pref (Cl gl_i + Cp glp_i + Cq gc_i);
-        // reciprocals are taken once.
-        const M l = norm3(e0), lp = norm3(e1);
-        const M e0e1 = dot3(e0, e1), cr = norm3(cross3(e0, e1));
-        const M rl = fast_rcp(l), rlp = fast_rcp(lp), rl0 = fast_rcp(l0), rl0p = fast_rcp(l0p), rs0 = fast_rcp(sin_phi_0);
-        const M rllp = rl * rlp;
-        const M sin_phi = cr * rllp, cos_phi = e0e1 * rllp;
-        const M a = l * rl0;
-        const M b = (lp * cos_phi * rl0p - l * cos_phi_0 * rl0) * rs0;
-        const M c = sin_phi * rs0;
-        const M D11 = (a * a - M(1)) * M(0.5);
-        const M D22 = (b * b + c * c - M(1)) * M(0.5);
-        const M D12 = a * b * M(0.5);
-        const M I1 = M(2) * (D11 + D22);
-        const M I2 = I1 + M(4) * (D11 * D22 - D12 * D12);
-        M w1, w2;
-        if (skalak) {
-            w1 = I1 + M(1);
-            w2 = k.C * I2 - M(1);
-        } else {
-            const M q = M(1) + I2;
-            w1 = M(1);
-            w2 = -fast_rcp(q * q);
-        }
-        const M A11 = l * rl0 * rl0, s2 = rs0 * rs0;
-        const M k22p = s2 * (lp * rl0p * rl0p - l * cos_phi * cos_phi_0 * rl0 * rl0p);
-        const M k22l = s2 * (l * cos_phi_0 * cos_phi_0 * rl0 * rl0 - lp * cos_phi * cos_phi_0 * rl0p * rl0);
-        const M k22c = -s2 * l * lp * cos_phi_0 * rl0 * rl0p;
-        const M k12 = M(0.5) * rl0p * rs0;
-        const M k12l = k12 * (lp * cos_phi * rl0p - M(2) * l * cos_phi_0 * rl0);
-        const M k12p = k12 * l * cos_phi * rl0p, k12c = k12 * l * lp * rl0p;
-        const M al = M(2) + M(4) * D22, be = M(2) + M(4) * D11, ga = M(8) * D12;
-        const M Cl = M(2) * w1 * (A11 + k22l) + w2 * (al * A11 + be * k22l - ga * k12l);
-        const M Cp = M(2) * w1 * k22p + w2 * (be * k22p - ga * k12p);
-        const M Cq = M(2) * w1 * k22c + w2 * (be * k22c - ga * k12c);
-        const M t3 = e0e1 * rl * rl * rllp, t4 = e0e1 * rllp * rlp * rlp;
-        const M pref = -k.G * M(0.5) * tri_area_of<M>(P, t);
-        const V3<M> gl1 = rl * e0, glp2 = rlp * e1;
-        const V3<M> gc0 = (t3 - rllp) * e0 + (t4 - rllp) * e1, gc1 = rllp * e1 - t3 * e0, gc2 = rllp * e0 - t4 * e1;
-        sk(i0, pref * (M(-1) * (Cl * gl1 + Cp * glp2) + Cq * gc0));
-        sk(i1, pref * (Cl * gl1 + Cq * gc1));
-        sk(i2, pref * (Cp * glp2 + Cq * gc2));
-        return;
-    }
+    const Rest4<M> r0 = rest_of<M>(P, t);
+    const M l0 = r0.x, l0p = r0.y, cos_phi_0 = r0.z, sin_phi_0 = r0.w;
+    // The forces with the corner-independent scalars gathered: every gradient of
+    // D11, D22, D12 (hence of I1, I2) is a combination of the corner gradients of
+    // l, l' and cos(phi) (gl, glp, gc below), so f_i = pref (Cl gl_i + Cp glp_i + Cq gc_i);
+    // reciprocals are taken once (FP64: a chain of divisions per gradient bound a warp at 36.9 us).
     const M l = norm3(e0), lp = norm3(e1);
-    const M e0e1 = dot3(e0, e1);
-    const M sin_phi = norm3(cross3(e0, e1)) / (l * lp);
-    const M cos_phi = e0e1 / (l * lp);
-    const M a = l / l0;
-    const M b = (lp * cos_phi / l0p - l * cos_phi_0 / l0) / sin_phi_0;
-    const M c = lp * sin_phi / (lp * sin_phi_0);
-    const M D11 = (a * a - M(1)) / M(2);
-    const M D22 = (b * b + c * c - M(1)) / M(2);
-    const M D12 = a * b / M(2);
+    const M e0e1 = dot3(e0, e1), cr = norm3(cross3(e0, e1));
+    const M rl = fast_rcp(l), rlp = fast_rcp(lp), rl0 = fast_rcp(l0), rl0p = fast_rcp(l0p), rs0 = fast_rcp(sin_phi_0);
+    const M rllp = rl * rlp;
+    const M sin_phi = cr * rllp, cos_phi = e0e1 * rllp;
+    const M a = l * rl0;
+    const M b = (lp * cos_phi * rl0p - l * cos_phi_0 * rl0) * rs0;
+    const M c = sin_phi * rs0;
+    const M D11 = (a * a - M(1)) * M(0.5);
+    const M D22 = (b * b + c * c - M(1)) * M(0.5);
+    const M D12 = a * b * M(0.5);
     const M I1 = M(2) * (D11 + D22);
     const M I2 = I1 + M(4) * (D11 * D22 - D12 * D12);
-    const V3<M> zero = mk3<M>(0, 0, 0);
-    const V3<M> gl[3] = {e0 / (-l), e0 / l, zero};
-    const V3<M> glp[3] = {e1 / (-lp), zero, e1 / lp};
-    const V3<M> gc[3] = {(M(-1) / (l * lp) + e0e1 / (l * l * l * lp)) * e0 + (M(-1) / (l * lp) + e0e1 / (l * lp * lp * lp)) * e1,
-                         (M(1) / (l * lp)) * e1 - (e0e1 / (l * l * l * lp)) * e0,
-                         (M(1) / (l * lp)) * e0 - (e0e1 / (l * lp * lp * lp)) * e1};
-    const M s0sq = sin_phi_0 * sin_phi_0;
-    const M G = k.G, Cc = k.C;
-    const M pref = -G / M(2) * tri_area_of<M>(P, t);
-    for (int i = 0; i < 3; ++i) {
-        const V3<M> gD11 = (l / (l0 * l0)) * gl[i];
-        const V3<M> gD22 = (M(1) / s0sq) * ((lp / (l0p * l0p) - l * cos_phi * cos_phi_0 / (l0 * l0p)) * glp[i] +
-                                            (l * (cos_phi_0 * cos_phi_0) / (l0 * l0) - lp * cos_phi * cos_phi_0 / (l0p * l0)) * gl[i] -
-                                            (l * lp * cos_phi_0 / (l0 * l0p)) * gc[i]);
-        const V3<M> gD12 = (M(1) / (M(2) * l0p * sin_phi_0)) *
-                           ((lp * cos_phi / l0p - M(2) * l * cos_phi_0 / l0) * gl[i] + (l * cos_phi / l0p) * glp[i] +
-                            (l * lp / l0p) * gc[i]);
-        const V3<M> gI1 = M(2) * (gD11 + gD22);
-        const V3<M> gI2 = (M(2) + M(4) * D22) * gD11 + (M(2) + M(4) * D11) * gD22 - (M(8) * D12) * gD12;
-        V3<M> fv;
-        if (skalak) fv = pref * ((I1 + M(1)) * gI1 + (Cc * I2 - M(1)) * gI2);
-        else fv = pref * (gI1 - (M(1) / ((M(1) + I2) * (M(1) + I2))) * gI2);
-        sk(id[i], fv);
+    M w1, w2;
+    if (skalak) {
+        w1 = I1 + M(1);
+        w2 = k.C * I2 - M(1);
+    } else {
+        const M q = M(1) + I2;
+        w1 = M(1);
+        w2 = -fast_rcp(q * q);
     }
+    const M A11 = l * rl0 * rl0, s2 = rs0 * rs0;
+    const M k22p = s2 * (lp * rl0p * rl0p - l * cos_phi * cos_phi_0 * rl0 * rl0p);
+    const M k22l = s2 * (l * cos_phi_0 * cos_phi_0 * rl0 * rl0 - lp * cos_phi * cos_phi_0 * rl0p * rl0);
+    const M k22c = -s2 * l * lp * cos_phi_0 * rl0 * rl0p;
+    const M k12 = M(0.5) * rl0p * rs0;
+    const M k12l = k12 * (lp * cos_phi * rl0p - M(2) * l * cos_phi_0 * rl0);
+    const M k12p = k12 * l * cos_phi * rl0p, k12c = k12 * l * lp * rl0p;
+    const M al = M(2) + M(4) * D22, be = M(2) + M(4) * D11, ga = M(8) * D12;
+    const M Cl = M(2) * w1 * (A11 + k22l) + w2 * (al * A11 + be * k22l - ga * k12l);
+    const M Cp = M(2) * w1 * k22p + w2 * (be * k22p - ga * k12p);
+    const M Cq = M(2) * w1 * k22c + w2 * (be * k22c - ga * k12c);
+    const M t3 = e0e1 * rl * rl * rllp, t4 = e0e1 * rllp * rlp * rlp;
+    const M pref = -k.G * M(0.5) * tri_area_of<M>(P, t);
+    const V3<M> gl1 = rl * e0, glp2 = rlp * e1;
+    const V3<M> gc0 = (t3 - rllp) * e0 + (t4 - rllp) * e1, gc1 = rllp * e1 - t3 * e0, gc2 = rllp * e0 - t4 * e1;
+    sk(i0, pref * (M(-1) * (Cl * gl1 + Cp * glp2) + Cq * gc0));
+    sk(i1, pref * (Cl * gl1 + Cq * gc1));
+    sk(i2, pref * (Cp * glp2 + Cq * gc2));
 }
 
 // RBCParticle link term (WLC + POW), src/fsi/RBCParticle.hh:148-169 with
@@ -2005,9 +1963,8 @@ void launch_force_clear(const Lattice& L, int fbuf, cudaStream_t s) {
     else k_force_clear<3><<<g, 128, 0, s>>>(L.d, L.ib, L.nvert, L.spread_lo[fbuf], (float*)L.F[fbuf]);
 }
 
-// CTAs per particle of the membrane kernel: enough to give every SM two CTAs, but at least
-// one element per thread
-int membrane_split(int np, int max_elems, int block) {
+// CTAs per particle: enough to give every SM `per_sm` CTAs, but at least one element per thread
+int membrane_split(int np, int max_elems, int block, int per_sm = 2) {
     static int sms = 0;
     if (!sms) {
         int dev = 0;
@@ -2016,7 +1973,7 @@ int membrane_split(int np, int max_elems, int block) {
         if (sms <= 0) sms = 1;
     }
     if (np <= 0 || np >= sms) return 1;
-    const int want = (2 * sms + np - 1) / np;
+    const int want = (per_sm * sms + np - 1) / np;
     const int most = std::max(1, (max_elems + block - 1) / block);
     return std::max(1, std::min(want, most));
 }
@@ -2052,21 +2009,27 @@ void launch_membrane_forces(const Lattice& L, cudaStream_t s) {
         return;
     }
     if (L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) {
-        const unsigned g = (L.nvert + 127) / 128;
+        const int block = L.nvert < 32768 ? 32 : 128;  // few vertices: a warp each to the SMs (FP64 pipe)
+        const unsigned g = (L.nvert + block - 1) / block;
         if (L.storage == BIB_STORAGE_F64)
-            k_membrane_gather<double><<<g, 128, 0, s>>>(L.nvert, L.vert_particle, L.pdev, L.pos[L.pcur], L.force, L.stats, L.inter);
+            k_membrane_gather<double><<<g, block, 0, s>>>(L.nvert, L.vert_particle, L.pdev, L.pos[L.pcur], L.force, L.stats, L.inter);
         else
-            k_membrane_gather<float><<<g, 128, 0, s>>>(L.nvert, L.vert_particle, L.pdev, L.pos[L.pcur], L.force, L.stats, L.inter);
+            k_membrane_gather<float><<<g, block, 0, s>>>(L.nvert, L.vert_particle, L.pdev, L.pos[L.pcur], L.force, L.stats, L.inter);
         return;
     }
-    // few particles: spread each particle's elements over several CTAs so the launch fills the GPU
-    const int split = membrane_split(np, L.max_elems, L.membrane_block);
+    // few particles: each particle's elements over several CTAs so the launch fills the GPU, about four warps
+    // per SM (bound by the FP64 pipe, 2 lanes per cycle and SM: a warp to itself is served as fast as it
+    // can issue).  One capsule of 1280 triangles, FP64: 8 CTAs of 256 threads 53.8 us, 60 of 32 36.9
+    // (23.6 with capsule_triangle's shared scalars)
+    const int warps = (L.max_elems + 31) / 32;
+    const int split = std::min(warps, membrane_split(np, L.max_elems, 32, 4));
     if (split > 1) {
         const IbView v = single_view(L, -1);
         k_force_seed<<<(L.nvert + 127) / 128, 128, 0, s>>>(v);
         const dim3 grid((unsigned)np, (unsigned)split);
-        if (L.storage == BIB_STORAGE_F64) k_membrane<double, false><<<grid, L.membrane_block, L.membrane_smem, s>>>(L.pdev, v, nullptr);
-        else k_membrane<float, false><<<grid, L.membrane_block, L.membrane_smem, s>>>(L.pdev, v, nullptr);
+        const int block = std::min(L.membrane_block, 32 * ((warps + split - 1) / split));
+        if (L.storage == BIB_STORAGE_F64) k_membrane<double, false><<<grid, block, L.membrane_smem, s>>>(L.pdev, v, nullptr);
+        else k_membrane<float, false><<<grid, block, L.membrane_smem, s>>>(L.pdev, v, nullptr);
         return;
     }
     membrane_any<false>(L.storage, L.pdev, np, single_view(L, -1), nullptr, L.membrane_smem, L.membrane_block, s);
