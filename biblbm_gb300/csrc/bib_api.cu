@@ -600,7 +600,8 @@ bib_status sync_particles(bib_ctx* c, Lattice& L) {
     BIB_ALLOC(c, (void**)&L.vel, vb);
     BIB_ALLOC(c, (void**)&L.force, vb);
     BIB_ALLOC(c, (void**)&L.stats, STATS * np * sizeof(double));
-    BIB_ALLOC(c, (void**)&L.upd_partial, (size_t)np * 64 * 5 * sizeof(double));
+    BIB_ALLOC(c, (void**)&L.upd_partial, (size_t)np * (64 * 5 + 1) * sizeof(double));  // sums and tickets
+    BIB_CUDA(c, cudaMemset(L.upd_partial, 0, (size_t)np * (64 * 5 + 1) * sizeof(double)));
     for (int k = 0; k < 2; ++k) BIB_ALLOC(c, (void**)&L.spread_lo[k], (size_t)L.nvert * sizeof(int4));
     forces_touched(L);
     BIB_CUDA(c, cudaMemcpy(L.pos[0], L.host_pos.data(), vb, cudaMemcpyHostToDevice));

@@ -382,7 +382,7 @@ struct Lattice {
     std::vector<PatchJob> patch_jobs_host;
     int npatch = 0;
     size_t patch_smem = 0;
-    double* upd_partial = nullptr;  // partial sums of the split update (particles x 64 x 5)
+    double* upd_partial = nullptr;  // partial sums (particles x 64 x 5) and tickets of the split update
     bool particles_dirty = true;  // host copies below are authoritative until uploaded
     std::vector<double> host_pos;    // concatenated vertex positions
     std::vector<double> host_stats;  // STATS per particle

@@ -1426,14 +1426,16 @@ __device__ __forceinline__ void block_sum5(const double v[5], double* red, doubl
 
 // Per-triangle area, signed volume and area-weighted centroid of X_{n+1}, summed over the
 // triangles e0, e0 + es, ... by this CTA into sum[0..4] (shared; valid for every thread).
-template <class M>
+// M = float with STAGE: the relative positions of the whole particle are staged in sp first (one CTA for
+// many triangles); without, each triangle takes its own.
+template <class M, bool STAGE>
 __device__ __forceinline__ void update_sums(const ParticleDev& P, const IbView& V, float* sp, double* red, double* sum,
                                             int e0, int es) {
     const double* pv = V.pos_next + 3LL * P.v0;
     const double* st = V.stats + STATS * P.lpid;
     const bool rel = sizeof(M) < sizeof(double);
     const double c0 = rel ? st[2] : 0.0, c1 = rel ? st[3] : 0.0, c2 = rel ? st[4] : 0.0;
-    if (rel) {  // one FP64 subtraction and rounding per vertex coordinate
+    if (STAGE && rel) {  // one FP64 subtraction and rounding per vertex coordinate
         for (int i = threadIdx.x; i < P.nv; i += blockDim.x) {
             sp[3 * i] = (float)(pv[3 * i] - c0);
             sp[3 * i + 1] = (float)(pv[3 * i + 1] - c1);
@@ -1442,7 +1444,7 @@ __device__ __forceinline__ void update_sums(const ParticleDev& P, const IbView& 
         __syncthreads();
     }
     auto vert = [&](int i) {
-        return rel ? mk3<M>((M)sp[3 * i], (M)sp[3 * i + 1], (M)sp[3 * i + 2])
+        return STAGE && rel ? mk3<M>((M)sp[3 * i], (M)sp[3 * i + 1], (M)sp[3 * i + 2])
                    : mk3<M>((M)(pv[3 * i] - c0), (M)(pv[3 * i + 1] - c1), (M)(pv[3 * i + 2] - c2));
     };
     // per-thread partial sums in M (a few triangles each), block sums in FP64
@@ -1505,36 +1507,40 @@ template <class M>
 __device__ __forceinline__ void update_block(const ParticleDev& P, const IbView& V, float* sp, double* red,
                                              double* delta) {
     __shared__ double sum[5];
-    update_sums<M>(P, V, sp, red, sum, threadIdx.x, blockDim.x);
+    update_sums<M, true>(P, V, sp, red, sum, threadIdx.x, blockDim.x);
     update_finish<M>(P, V, sum, delta);
 }
 
-// Few particles: gridDim.y CTAs per particle write partial sums, one CTA per particle adds
-// them in slice order and finishes the update.
-constexpr int kMaxUpdateSplit = 64;
+// Few particles: gridDim.y CTAs per particle write partial sums; the one that finishes last adds them in
+// slice order and finishes the update (it waits for nothing: the others have left their sums and their
+// ticket).  `ticket` counts the CTAs done, zero between launches.  A triangle takes its vertices from global
+// memory: staging the particle in every CTA was bound by the FP64 pipe.  One membrane of 2562 vertices in
+// FP32, partial sums and finish in two launches, 11.9 + 5.7 us, now 11.4.
+constexpr int kMaxUpdateSplit = 64, kUpdateFew = 128;
 
 template <class M>
-__global__ void __launch_bounds__(256) k_update_partial(const ParticleDev* __restrict__ parts, IbView v1,
-                                                         double* __restrict__ partial) {
-    __shared__ double red[5 * 256];
-    __shared__ double sum[5];
-    extern __shared__ __align__(16) float sp[];
+__global__ void __launch_bounds__(kUpdateFew) k_update_few(const ParticleDev* __restrict__ parts, IbView v1, double* partial,
+                                                           unsigned* ticket) {
+    __shared__ double red[5 * kUpdateFew];
+    __shared__ double sum[5], delta[3];
+    __shared__ bool last;
     const ParticleDev& P = parts[blockIdx.x];
-    update_sums<M>(P, v1, sp, red, sum, blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
-    if (threadIdx.x < 5) partial[(blockIdx.x * (size_t)gridDim.y + blockIdx.y) * 5 + threadIdx.x] = sum[threadIdx.x];
-}
-
-template <class M>
-__global__ void __launch_bounds__(256) k_update_finish(const ParticleDev* __restrict__ parts, IbView v1,
-                                                        const double* __restrict__ partial, int split) {
-    __shared__ double sum[5];
-    __shared__ double delta[3];
-    const ParticleDev& P = parts[blockIdx.x];
+    const int split = gridDim.y;
+    update_sums<M, false>(P, v1, nullptr, red, sum, blockIdx.y * kUpdateFew + threadIdx.x, split * kUpdateFew);
+    double* mine = partial + (blockIdx.x * (size_t)split) * 5;
+    if (threadIdx.x < 5) mine[blockIdx.y * 5 + threadIdx.x] = sum[threadIdx.x];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket + blockIdx.x, 1u) == (unsigned)split - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
     if (threadIdx.x < 5) {
         double a = 0.0;
-        for (int y = 0; y < split; ++y) a += partial[(blockIdx.x * (size_t)split + y) * 5 + threadIdx.x];
+        for (int y = 0; y < split; ++y) a += __ldcg(mine + y * 5 + threadIdx.x);
         sum[threadIdx.x] = a;
     }
+    if (threadIdx.x == 0) ticket[blockIdx.x] = 0;
     __syncthreads();
     update_finish<M>(P, v1, sum, delta);
 }
@@ -1858,7 +1864,6 @@ void configure_membrane_kernel(size_t smem) {
     // 3 floats per vertex, at most half of the membrane kernel's 3 doubles per vertex
     cudaFuncSetAttribute(k_particle_update<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem / 2));
     cudaFuncSetAttribute(k_particle_update<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem / 2));
-    cudaFuncSetAttribute(k_update_partial<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem / 2));
 }
 
 IbView single_view(const Lattice& L, int fbuf) {
@@ -2075,20 +2080,15 @@ void launch_pp_forces(const Lattice& L, cudaStream_t s) {
 void launch_particle_update(const Lattice& L, cudaStream_t s) {
     const int np = (int)L.parts.size();
     if (np == 0) return;
-    // the split costs a second launch: worth it for the FP64 sums, and in FP32 for large meshes
-    // (measured: 642-vertex capsule FP32 slower split, 2562-vertex RBC and every FP64 case faster)
+    // FP64 sums, and in FP32 large meshes (a step of a 1280-triangle membrane in 96^3 FP32 54 us with one CTA, 56 split;
+    // of a 5120-triangle one in 160 x 128 x 128 119 and 111)
     const bool big = L.storage == BIB_STORAGE_F64 || L.max_nt >= 4096;
-    const int split = big ? std::min(kMaxUpdateSplit, membrane_split(np, L.max_nt, 256)) : 1;
+    const int split = big ? std::min(kMaxUpdateSplit, membrane_split(np, L.max_nt, kUpdateFew)) : 1;
     if (split > 1 && L.upd_partial) {
         const IbView v = single_view(L, -1);
-        const size_t sm = L.storage == BIB_STORAGE_F64 ? 0 : 3 * sizeof(float) * L.max_nv;
-        if (L.storage == BIB_STORAGE_F64) {
-            k_update_partial<double><<<dim3(np, split), 256, sm, s>>>(L.pdev, v, L.upd_partial);
-            k_update_finish<double><<<np, 256, 0, s>>>(L.pdev, v, L.upd_partial, split);
-        } else {
-            k_update_partial<float><<<dim3(np, split), 256, sm, s>>>(L.pdev, v, L.upd_partial);
-            k_update_finish<float><<<np, 256, 0, s>>>(L.pdev, v, L.upd_partial, split);
-        }
+        unsigned* ticket = reinterpret_cast<unsigned*>(L.upd_partial + (size_t)np * kMaxUpdateSplit * 5);
+        if (L.storage == BIB_STORAGE_F64) k_update_few<double><<<dim3(np, split), kUpdateFew, 0, s>>>(L.pdev, v, L.upd_partial, ticket);
+        else k_update_few<float><<<dim3(np, split), kUpdateFew, 0, s>>>(L.pdev, v, L.upd_partial, ticket);
         return;
     }
     update_any<false>(L.storage, L.pdev, np, single_view(L, -1), nullptr, L.max_nv, s);
