@@ -413,6 +413,7 @@ struct Lattice {
 enum class Coupling {
     kNone,    // collision with F[fe], no side outputs
     kDense,   // velocity j/rho + F[fe]/2 written, collision with F[1-fe], F[fe] reset to the body force
+    kReset,   // collision with F[1-fe], F[fe] reset to the body force, no velocity written
     kSparse,  // velocity j/rho + body/2 written, collision with F[1-fe]; F[fe] left for the sparse reset
 };
 void launch_collide_stream(const Lattice& L, Coupling mode, cudaStream_t s);
@@ -422,7 +423,13 @@ bool launch_collide_stream_staged(const Lattice& L, Coupling mode, cudaStream_t 
 bool launch_collide_stream_linear(const Lattice& L, Coupling mode, cudaStream_t s);
 bool collide_staged_fits(const Lattice& L);  // both step kinds fit the staged kernel
 void launch_fd_walls(const Lattice& L, int buf, int fbuf, cudaStream_t s);
+// The support nodes of the vertices are at most half as many as the cells.
+inline bool few_support_nodes(const Lattice& L) {
+    const int64_t sup = L.ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
+    return L.nvert > 0 && 2 * (int64_t)L.nvert * sup * sup * sup <= L.d.n;
+}
 void launch_velocity_field(const Lattice& L, cudaStream_t s);  // u from the current state and F[fe]
+void launch_velocity_support(const Lattice& L, cudaStream_t s);  // the same at the vertices' support nodes only
 void launch_velocity_export(const Lattice& L, double* u, cudaStream_t s);
 void launch_init_equilibrium(const Lattice& L, const double* rho, const double* u, cudaStream_t s);
 // populations of planes z0 .. z0 + nzc - 1 from / to FP64 SoA slices of `pitch` cells

@@ -37,7 +37,7 @@ struct LinearLayout {
     static constexpr unsigned OFF_FCOL = Q * POP;
     static constexpr unsigned OFF_FPREV = OFF_FCOL + (NEED_FCOL ? FRC : 0);
     static constexpr unsigned BYTES = (OFF_FPREV + (CPL == kCplDense ? FRC : 0) + 127) / 128 * 128;
-    static constexpr unsigned RESET = CPL == kCplDense ? FRC : 0;
+    static constexpr unsigned RESET = resets(CPL) ? FRC : 0;
 };
 
 struct LinearGeom {
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(LinearLayout<T, CPL, COLL>::THREADS, staged_ct
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t NS = (uint32_t)g.nstages;
     if (blockIdx.x >= g.ntiles) return;
-    if (CPL == kCplDense) fill_reset(reset, d.body, 3 * L::TILE, tid, L::THREADS);
+    if (resets(CPL)) fill_reset(reset, d.body, 3 * L::TILE, tid, L::THREADS);
     if (tid == 0) {
         for (uint32_t k = 0; k < NS; ++k) {
             mbar_init(&full[k], 1);
@@ -201,14 +201,14 @@ __global__ void __launch_bounds__(LinearLayout<T, CPL, COLL>::THREADS, staged_ct
                 continue;
             }
             load_linear<T, CPL, COLL>(g, tile, stages + s * L::BYTES, &full[s], fin, Fcol, Fprev, lane, off);
-            if (CPL == kCplDense && use > 0 && lane == 0) reset_linear(tile - NS * gridDim.x);
+            if (resets(CPL) && use > 0 && lane == 0) reset_linear(tile - NS * gridDim.x);
         }
         // copies still landing (if the consumers gave up) and the last tiles' reset
         if (lane == 0) {
             for (uint32_t k = it > NS ? it - NS : 0; k < it; ++k)
-                if (k != withheld && mbar_wait_bounded(&full[k % NS], (k / NS) & 1u) && CPL == kCplDense)
+                if (k != withheld && mbar_wait_bounded(&full[k % NS], (k / NS) & 1u) && resets(CPL))
                     reset_linear(blockIdx.x + k * gridDim.x);
-            if (CPL == kCplDense) bulk_wait_all();
+            if (resets(CPL)) bulk_wait_all();
         }
         return;
     }
@@ -317,10 +317,10 @@ bool linear_inst(const Lattice& L, cudaStream_t s) {
     }
     const unsigned grid = (unsigned)std::min<int64_t>(g.ntiles, (int64_t)nb * sms);
     const FT* Fcol = (const FT*)(CPL != kCplNone ? L.F[1 - L.fe] : L.F[L.fe]);
-    FT* Fprev = CPL == kCplDense ? (FT*)L.F[L.fe] : nullptr;
+    FT* Fprev = resets(CPL) ? (FT*)L.F[L.fe] : nullptr;
     kern<<<grid, LY::THREADS, smem, s>>>(d, g, collide_params<C>(d, L.storage), (const T*)L.f[L.cur], (T*)L.f[1 - L.cur],
                                          (const T*)L.wall, Fcol, Fprev,
-                                         CPL != kCplNone ? (typename Store<T>::U*)L.u : nullptr, L.phase, L.celltype,
+                                         writes_u(CPL) ? (typename Store<T>::U*)L.u : nullptr, L.phase, L.celltype,
                                          L.wait_err);
     return true;
 }
@@ -339,6 +339,7 @@ bool linear_t(const Lattice& L, Coupling mode, cudaStream_t s) {
     switch (mode) {
         case Coupling::kDense: return linear_coll<T, kCplDense>(L, s);
         case Coupling::kSparse: return linear_coll<T, kCplSparse>(L, s);
+        case Coupling::kReset: return linear_coll<T, kCplReset>(L, s);
         default: return linear_coll<T, kCplNone>(L, s);
     }
 }

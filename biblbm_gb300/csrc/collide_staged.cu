@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int NS = g.nstages;
     if ((int64_t)blockIdx.x >= g.ntiles) return;
-    if (CPL == kCplDense) fill_reset(reset, d.body, 3 * TILE, tid, L::THREADS);
+    if (resets(CPL)) fill_reset(reset, d.body, 3 * TILE, tid, L::THREADS);
     if (tid == 0) {
         for (int k = 0; k < NS; ++k) {
             mbar_init(&full[k], 1);
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
                 continue;
             }
             load_tile<T, CPL, COLL>(d, g, tile, stages + s * L::BYTES, &full[s], fin, wall, Fcol, Fprev, lane, pl);
-            if (CPL == kCplDense && use > 0 && lane == 0) reset_tile(d, g, tile - (int64_t)NS * gridDim.x, Fprev, reset);
+            if (resets(CPL) && use > 0 && lane == 0) reset_tile(d, g, tile - (int64_t)NS * gridDim.x, Fprev, reset);
         }
         // a copy may still be landing only if the consumers gave up; wait for it so that
         // no bulk copy writes into the shared memory of a retired CTA (a withheld tile has none); the
@@ -292,9 +292,9 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
         if (lane == 0) {
             const int issued = it;
             for (int k = issued > NS ? issued - NS : 0; k < issued; ++k)
-                if (k != withheld && mbar_wait_bounded(&full[k % NS], (unsigned)(k / NS) & 1u) && CPL == kCplDense)
+                if (k != withheld && mbar_wait_bounded(&full[k % NS], (unsigned)(k / NS) & 1u) && resets(CPL))
                     reset_tile(d, g, blockIdx.x + (int64_t)k * gridDim.x, Fprev, reset);
-            if (CPL == kCplDense) bulk_wait_all();
+            if (resets(CPL)) bulk_wait_all();
         }
         return;
     }
@@ -477,7 +477,8 @@ int staged_stages(const Lattice& L) {
     if (L.stages >= 2) return L.stages;
     const size_t limit = std::min<size_t>((size_t)optin_smem(), 228 * 1024 / staged_ctas_per_sm<T>()) - 1024;
     int best = 2;
-    for (int ns = 2; ns <= kMaxStages; ++ns)
+    // beside the membranes' kernels (reset coupling) their CTAs need room: three stages at most
+    for (int ns = 2; ns <= (CPL == kCplReset ? 3 : kMaxStages); ++ns)
         if (staged_smem<T, CPL, COLL>(ns) <= limit) best = ns;
     return best;
 }
@@ -531,9 +532,9 @@ bool staged_inst(const Lattice& L, int target, cudaStream_t s) {
     const T* fin = (const T*)L.f[L.cur];
     T* fout = (T*)L.f[1 - L.cur];
     const FT* Fcol = (const FT*)(CPL != kCplNone ? L.F[1 - L.fe] : L.F[L.fe]);
-    FT* Fprev = CPL == kCplDense ? (FT*)L.F[L.fe] : nullptr;
+    FT* Fprev = resets(CPL) ? (FT*)L.F[L.fe] : nullptr;
     kern<<<(unsigned)grid, LY::THREADS, smem, s>>>(d, g, collide_params<C>(d, L.storage), fin, fout,
-                                                       (const T*)L.wall, Fcol, Fprev, CPL != kCplNone ? (typename Store<T>::U*)L.u : nullptr,
+                                                       (const T*)L.wall, Fcol, Fprev, writes_u(CPL) ? (typename Store<T>::U*)L.u : nullptr,
                                                        L.phase, L.celltype, L.wait_err);
     return true;
 }
@@ -565,6 +566,7 @@ bool staged_t(const Lattice& L, Coupling mode, cudaStream_t s) {
     switch (mode) {
         case Coupling::kDense: return staged_coll<T, kCplDense>(L, target, s);
         case Coupling::kSparse: return staged_coll<T, kCplSparse>(L, target, s);
+        case Coupling::kReset: return staged_coll<T, kCplReset>(L, target, s);
         default: return staged_coll<T, kCplNone>(L, target, s);
     }
 }

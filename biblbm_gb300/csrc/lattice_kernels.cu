@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) k_collide_stream(LatticeDesc d, const T* 
     const int ctype = d.has_types ? celltype[k] : BIB_CELL_FLUID;
     if (ctype != BIB_CELL_FLUID) {  // BounceBack / NoDynamics node: no collision, zero velocity
         if (COUPLED) {
-            store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
+            if (u_out) store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
             if (Fprev)
                 for (int c = 0; c < 3; ++c) Fprev[3 * k + c] = (FT)d.body[c];
         }
@@ -86,20 +86,22 @@ __global__ void __launch_bounds__(256) k_collide_stream(LatticeDesc d, const T* 
         // the previous collision; that force buffer is then reset to the body force so the
         // next step can spread into it (setExternalVector).  Without Fprev (sparse force
         // reset) the velocity takes the body force and the interpolation adds the rest.
-        C u[3];
-        if (fd_wall_node(d, y)) {
-            const int side = y == 0 ? 0 : 1;
-            u[0] = (C)d.wall_u[side][0];
-            u[1] = (C)d.wall_u[side][1];
-            u[2] = (C)d.wall_u[side][2];
-        } else {
-            C Fp[3] = {(C)d.body[0], (C)d.body[1], (C)d.body[2]};
-            if (Fprev) {
-                for (int c = 0; c < 3; ++c) Fp[c] = (C)Fprev[3 * k + c];
+        if (u_out) {
+            C u[3];
+            if (fd_wall_node(d, y)) {
+                const int side = y == 0 ? 0 : 1;
+                u[0] = (C)d.wall_u[side][0];
+                u[1] = (C)d.wall_u[side][1];
+                u[2] = (C)d.wall_u[side][2];
+            } else {
+                C Fp[3] = {(C)d.body[0], (C)d.body[1], (C)d.body[2]};
+                if (Fprev) {
+                    for (int c = 0; c < 3; ++c) Fp[c] = (C)Fprev[3 * k + c];
+                }
+                velocity_with_force(f, Fp, u);
             }
-            velocity_with_force(f, Fp, u);
+            store_u<UT>(u_out, k, (UT)u[0], (UT)u[1], (UT)u[2]);
         }
-        store_u<UT>(u_out, k, (UT)u[0], (UT)u[1], (UT)u[2]);
         if (Fprev) {
             for (int c = 0; c < 3; ++c) Fprev[3 * k + c] = (FT)d.body[c];
         }
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) k_collide_stream_rows(LatticeDesc d, cons
     }
     if (active) {
         load_force2<FT>(Fcol, k0, fca, fcb);
-        if (COUPLED && !wallrow) {
+        if (COUPLED && !wallrow && u_out) {
             if (Fprev) {
                 load_force2<FT>(Fprev, k0, fpa, fpb);
             } else {  // sparse force reset: the velocity field takes the body force only
@@ -241,19 +243,21 @@ __global__ void __launch_bounds__(256) k_collide_stream_rows(LatticeDesc d, cons
         ct1 = celltype[k0 + 1];
     }
     if (COUPLED) {
-        C u0[3], u1[3];
-        if (wallrow) {
-            const int side = y == 0 ? 0 : 1;
-            for (int c = 0; c < 3; ++c) u0[c] = u1[c] = (C)d.wall_u[side][c];
-        } else {
-            C Fa[3] = {(C)fpa[0], (C)fpa[1], (C)fpa[2]}, Fb[3] = {(C)fpb[0], (C)fpb[1], (C)fpb[2]};
-            velocity_with_force(f0, Fa, u0);
-            velocity_with_force(f1, Fb, u1);
+        if (u_out) {
+            C u0[3], u1[3];
+            if (wallrow) {
+                const int side = y == 0 ? 0 : 1;
+                for (int c = 0; c < 3; ++c) u0[c] = u1[c] = (C)d.wall_u[side][c];
+            } else {
+                C Fa[3] = {(C)fpa[0], (C)fpa[1], (C)fpa[2]}, Fb[3] = {(C)fpb[0], (C)fpb[1], (C)fpb[2]};
+                velocity_with_force(f0, Fa, u0);
+                velocity_with_force(f1, Fb, u1);
+            }
+            if (ct0 != BIB_CELL_FLUID) u0[0] = u0[1] = u0[2] = C(0);
+            if (ct1 != BIB_CELL_FLUID) u1[0] = u1[1] = u1[2] = C(0);
+            store_u<UT>(u_out, k0, (UT)u0[0], (UT)u0[1], (UT)u0[2]);
+            store_u<UT>(u_out, k0 + 1, (UT)u1[0], (UT)u1[1], (UT)u1[2]);
         }
-        if (ct0 != BIB_CELL_FLUID) u0[0] = u0[1] = u0[2] = C(0);
-        if (ct1 != BIB_CELL_FLUID) u1[0] = u1[1] = u1[2] = C(0);
-        store_u<UT>(u_out, k0, (UT)u0[0], (UT)u0[1], (UT)u0[2]);
-        store_u<UT>(u_out, k0 + 1, (UT)u1[0], (UT)u1[1], (UT)u1[2]);
         if (Fprev)
             store_force2<FT>(Fprev, k0, d.body);
     }
@@ -692,8 +696,9 @@ void collide_stream_t(const Lattice& L, Coupling mode, cudaStream_t s) {
     if (L.collide_kernel != BIB_KERNEL_ROWS && (launch_collide_stream_staged(L, mode, s) || launch_collide_stream_linear(L, mode, s)))
         return;
     const bool coupled = mode != Coupling::kNone;
-    // the previous force, read for the velocity and reset (dense coupling only)
-    FT* Fprev = mode == Coupling::kDense ? (FT*)L.F[L.fe] : nullptr;
+    // the previous force: read for the velocity and reset (dense), or reset alone, without a velocity field
+    FT* Fprev = mode == Coupling::kDense || mode == Coupling::kReset ? (FT*)L.F[L.fe] : nullptr;
+    auto* u = mode == Coupling::kReset ? nullptr : (typename Store<T>::U*)L.u;
     if (L.d.nx % 2 == 0) {
         const int pairs = L.d.nx / 2;
         const int bx = std::min(256, (pairs + 31) / 32 * 32);
@@ -705,7 +710,7 @@ void collide_stream_t(const Lattice& L, Coupling mode, cudaStream_t s) {
         T* fout = (T*)L.f[1 - L.cur];
         if (coupled)
             k_collide_stream_rows<T, true><<<grid, block, 0, s>>>(L.d, fin, fout, (const T*)L.wall, (const FT*)L.F[1 - L.fe],
-                                                                  Fprev, (typename Store<T>::U*)L.u, L.phase, L.celltype, L.d.collision);
+                                                                  Fprev, u, L.phase, L.celltype, L.d.collision);
         else
             k_collide_stream_rows<T, false><<<grid, block, 0, s>>>(L.d, fin, fout, (const T*)L.wall, (const FT*)L.F[L.fe],
                                                                    nullptr, nullptr, L.phase, L.celltype, L.d.collision);
@@ -717,7 +722,7 @@ void collide_stream_t(const Lattice& L, Coupling mode, cudaStream_t s) {
     const T* wall = (const T*)L.wall;
     if (coupled) {
         k_collide_stream<T, true><<<row_grid(L.d, bx), bx, 0, s>>>(L.d, fin, fout, wall, (const FT*)L.F[1 - L.fe],
-                                                                    Fprev, (typename Store<T>::U*)L.u, L.phase, L.celltype, L.d.collision);
+                                                                    Fprev, u, L.phase, L.celltype, L.d.collision);
     } else {
         k_collide_stream<T, false><<<row_grid(L.d, bx), bx, 0, s>>>(L.d, fin, fout, wall, (const FT*)L.F[L.fe], nullptr,
                                                                      nullptr, L.phase, L.celltype, L.d.collision);
@@ -749,15 +754,21 @@ void fd_walls_t(const Lattice& L, int buf, int fbuf, cudaStream_t s) {
 // at 0.02 nodes per cell, 126 / 150 at 0.31; 64^3 71 / 76 at 0.07, 80.6 / 81.6 at 0.53, 88 / 84 at 1.06; 96^3
 // FP64 441 / 523 at 0.02; 32^3 FP32 54.3 / 53.3 at 0.13, 70 / 65 at 4.2.
 template <class T>
-void velocity_field_t(const Lattice& L, cudaStream_t s) {
+void velocity_support_t(const Lattice& L, cudaStream_t s) {
     using FT = typename Store<T>::F;
     using UT = typename Store<T>::U;
     const int sup = L.ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
     const int64_t nodes = (int64_t)L.nvert * sup * sup * sup;
-    if (L.nvert > 0 && 2 * nodes <= L.d.n && L.d.n >= 65536) {
-        auto kern = sup == 4 ? k_velocity_support<T, 4> : k_velocity_support<T, 3>;
-        kern<<<lin_grid(nodes, 128), 128, 0, s>>>(L.d, L.ib, nodes, L.pos[L.pcur], (const T*)L.f[L.cur], (const T*)L.wall,
-                                                  (const FT*)L.F[L.fe], (UT*)L.u, L.celltype);
+    auto kern = sup == 4 ? k_velocity_support<T, 4> : k_velocity_support<T, 3>;
+    kern<<<lin_grid(nodes, 128), 128, 0, s>>>(L.d, L.ib, nodes, L.pos[L.pcur], (const T*)L.f[L.cur], (const T*)L.wall,
+                                              (const FT*)L.F[L.fe], (UT*)L.u, L.celltype);
+}
+template <class T>
+void velocity_field_t(const Lattice& L, cudaStream_t s) {
+    using FT = typename Store<T>::F;
+    using UT = typename Store<T>::U;
+    if (few_support_nodes(L) && L.d.n >= 65536) {
+        velocity_support_t<T>(L, s);
         return;
     }
     const int bx = row_block(L.d);
@@ -853,6 +864,7 @@ void launch_copy_f64(double* dst, const double* src, size_t n, cudaStream_t s) {
 }
 
 void launch_velocity_field(const Lattice& L, cudaStream_t s) { BIB_DISPATCH(L.storage, velocity_field_t, L, s); }
+void launch_velocity_support(const Lattice& L, cudaStream_t s) { BIB_DISPATCH(L.storage, velocity_support_t, L, s); }
 
 void launch_velocity_export(const Lattice& L, double* u, cudaStream_t s) {
     BIB_DISPATCH(L.storage, velocity_export_t, L, u, s);

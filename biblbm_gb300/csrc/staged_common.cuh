@@ -161,8 +161,11 @@ struct TileOf {
 
 // Coupling of a staged launch: lattice only; dense (the velocity field with the previous force,
 // which is read and reset to the body force); sparse (the velocity field with the body force,
-// the previous force left to the sparse reset).
-constexpr int kCplNone = 0, kCplDense = 1, kCplSparse = 2;
+// the previous force left to the sparse reset); reset (no velocity field, the previous force reset
+// without being read).
+constexpr int kCplNone = 0, kCplDense = 1, kCplSparse = 2, kCplReset = 3;
+__host__ __device__ constexpr bool writes_u(int cpl) { return cpl == kCplDense || cpl == kCplSparse; }
+__host__ __device__ constexpr bool resets(int cpl) { return cpl == kCplDense || cpl == kCplReset; }
 
 // Stage layout (compile-time): 19 population rows, the collision force (BGK + Guo) and,
 // for the dense coupled step, the previous force (three values per cell), each TILE cells long.
@@ -179,7 +182,7 @@ struct StageLayout {
     static constexpr unsigned OFF_FPREV = OFF_FCOL + (NEED_FCOL ? 3 * FRC : 0);
     static constexpr unsigned BYTES = ((OFF_FPREV + (CPL == kCplDense ? 3 * FRC : 0)) + 127) / 128 * 128;
     // dense coupling: one tile of the body force in front of the stages, the source of the reset
-    static constexpr unsigned RESET = CPL == kCplDense ? 3 * FRC : 0;
+    static constexpr unsigned RESET = resets(CPL) ? 3 * FRC : 0;
 };
 
 constexpr int kMaxStages = 8;
@@ -202,9 +205,10 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
                                             const typename Store<T>::C* Fp) {
     using C = typename Store<T>::C;
     using UT = typename Store<T>::U;
+    constexpr bool UVEL = writes_u(CPL);
     const int ctype = d.has_types ? celltype[k] : BIB_CELL_FLUID;
     if (ctype != BIB_CELL_FLUID) {  // BounceBack / NoDynamics node: no collision, zero velocity
-        if (CPL != kCplNone) store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
+        if (UVEL) store_u<UT>(u_out, k, (UT)0.0f, (UT)0.0f, (UT)0.0f);
         if (ctype == BIB_CELL_BOUNCE_BACK) bounce_back_cell(f);
         store_cell<T, C>(fout + k, d.stride, f);
         return;
@@ -212,7 +216,7 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
     C om = cp.om0;
     if (COLL == BIB_COLLISION_BGK_GUO_VOF && d.use_phase && phase[k]) om = cp.om1;
     const CellMoments<C> m = moments_compact<C>(f, cp.invS);
-    if (CPL != kCplNone) {
+    if (UVEL) {
         // the velocity is stored before the relaxation, so that the previous force is dead while
         // the relaxation runs
         C u[3];
