@@ -271,12 +271,19 @@ struct IbView {
     const int* order = nullptr;  // single lattices: the vertex each interpolation thread takes
 };
 
+// What the relaxation of a cell takes of its rates, at the storage scale S (w, w-: omega and the TRT
+// omega of the antisymmetric parts; t0, t: the weights 1/3 and 1/36): 1 - w; BGK: w, m = 3 (1 - w/2), S t0, S t;
+// TRT: m = 3 S w- t, the weights times S w, a = 1 - (w + w-)/2, b = (w- - w)/2.
+template <class C>
+struct RelaxRates {
+    C omo, w, m, t0, t, a, b;
+};
+
 // Per-launch constants of the collision in the compute type C.
 template <class C>
 struct CollideParams {
-    C om0, om1;      // relaxation frequency of phase 0 / 1 (BGK + Guo) or the omega of BGK / TRT
-    C omm;           // TRT: omega of the antisymmetric part
-    C S, invS;       // storage scale (FP16) and its inverse, 1 otherwise
+    RelaxRates<C> r[2];  // of phase 0 / 1 (BGK + Guo); BGK / TRT: the first
+    C invS;          // inverse of the storage scale (FP16), 1 otherwise
     C body[3];       // body force, the reset value of the previous force field
     C wall_u[2][3];  // velocity of the finite-difference wall rows y = 0, ny - 1
     C mw[4][19];     // moving-wall bounce-back term per wall face and population, storage units

@@ -98,37 +98,58 @@ __device__ __forceinline__ C bgk_equilibrium(int i, C rhoBar, C invRho, const C*
 // (bgk_ma2_collision_base, src/latticeBoltzmann/dynamicsTemplates3D.h:770-838) plus the Guo term of
 // VariableViscosityDynamics.hh:47-129,
 // t_i (1 - w/2) [3 (c_i - u).F + 9 (c_i.u)(c_i.F)], collapse to
-//     f_i' = (1 - w) f_i + t_i [A + c_i.H + (c_i.u)(c_i.G)]
-//     A = w rhoBar - 1.5 w rho u.u - 3 mu u.F,  H = 3 w rho u + 3 mu F,  G = 4.5 w rho u + 9 mu F,
+//     f_i' = (1 - w) f_i + t_i [A + c_i.H + (c_i.u)(c_i.K)]
+//     H = 3 w rho u + 3 mu F,  K = 4.5 w rho u + 9 mu F,  A = w rhoBar - u.K / 3,
 // mu = 1 - w/2, evaluated once per opposite pair (i, i+9) (c_{i+9} = -c_i).  BGK without
 // forcing is the same with F = 0 and u = j/rho (BGKdynamics::collide,
 // src/basicDynamics/isoThermalDynamics.hh:329-340); TRT is Ginzburg's two-relaxation-time split
 // around the same equilibrium (no reference counterpart).  The populations may carry a common scale S
 // (FP16 storage keeps f-bar * S): moments are unscaled once, post-collision values come out
-// in scaled units.  With `u_prev` non-null the velocity j/rho + F_prev/2 of the incoming
-// state is returned as well (the reference's computeVelocity).
-// c_i . (a, b, c) with the zero components left out: multiplications by 0 are not removed
-// by the compiler under IEEE semantics (0 * inf is NaN), so they are not written.
+// in scaled units.  FP64 is bound by its arithmetic: with
+// A by its own products, the scale of FP16 storage (1) and the rates worked out per cell a step of one FP64
+// capsule in 64^3 took 138 us, so 132.
+// The weights stay outside the brackets: with w t_i rounded once and folded in, FP32 mass drifts.  Every product
+// that meets a sum is written as fmac, so that all kernels and the packed pairs round alike.
+
+// c_i . (a, b, c) of the populations 10..18, whose first component that is not zero is 1, with the zero
+// components left out: multiplications by 0 are not removed by the compiler under IEEE semantics
+// (0 * inf is NaN), so they are not written.
 template <class C>
 __device__ __forceinline__ C cdot(int i, C a, C b, C c) {
-    const C xa = cx(i) > 0 ? a : -a, yb = cy(i) > 0 ? b : -b, zc = cz(i) > 0 ? c : -c;
     if (cx(i) != 0) {
-        if (cy(i) != 0) return xa + yb;
-        if (cz(i) != 0) return xa + zc;
-        return xa;
+        if (cy(i) != 0) return cy(i) > 0 ? a + b : a - b;
+        if (cz(i) != 0) return cz(i) > 0 ? a + c : a - c;
+        return a;
     }
-    if (cy(i) != 0) return cz(i) != 0 ? yb + zc : yb;
-    return cz(i) != 0 ? zc : C(0);
+    if (cy(i) != 0) return cz(i) == 0 ? b : (cz(i) > 0 ? b + c : b - c);
+    return c;
 }
 __device__ __forceinline__ float fmac(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fmac(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float recip(float a) { return 1.0f / a; }
+__device__ __forceinline__ double recip(double a) { return 1.0 / a; }
 
-// Moments of the incoming state: rhoBar, j and 1/rho, unscaled.
+template <class C, int COLL>
+__host__ __device__ __forceinline__ RelaxRates<C> relax_rates(C w, C wm, C S) {
+    const bool trt = COLL == BIB_COLLISION_TRT;
+    RelaxRates<C> r;
+    r.omo = C(1) - w;
+    r.w = w;
+    r.m = trt ? (C(3) * wm * S) * weight<C>(4) : C(3) * (C(1) - C(0.5) * w);
+    r.t0 = (trt ? w * S : S) * weight<C>(0);
+    r.t = (trt ? w * S : S) * weight<C>(4);
+    r.a = C(1) - C(0.5) * (w + wm);
+    r.b = C(0.5) * (wm - w);
+    return r;
+}
+
+// Moments of the incoming state: rhoBar, rho, j and 1/rho, unscaled (SCALED: the populations carry the
+// scale whose inverse is invS).
 template <class C>
 struct CellMoments {
-    C rb, j0, j1, j2, invRho;
+    C rb, rho, j0, j1, j2, invRho;
 };
-template <class C>
+template <class C, bool SCALED>
 __device__ __forceinline__ CellMoments<C> moments_compact(const C* f, C invS) {
     const C sxm = f[1] + f[4] + f[5] + f[6] + f[7];
     const C sxp = f[10] + f[13] + f[14] + f[15] + f[16];
@@ -137,12 +158,14 @@ __device__ __forceinline__ CellMoments<C> moments_compact(const C* f, C invS) {
     const C szm = f[3] + f[6] + f[8] + f[16] + f[18];
     const C szp = f[7] + f[9] + f[12] + f[15] + f[17];
     const C sx0 = f[0] + f[2] + f[3] + f[8] + f[9] + f[11] + f[12] + f[17] + f[18];
+    const C sum = sxm + sx0 + sxp;
     CellMoments<C> m;
-    m.rb = (sxm + sx0 + sxp) * invS;
-    m.j0 = (sxp - sxm) * invS;
-    m.j1 = (syp - sym) * invS;
-    m.j2 = (szp - szm) * invS;
-    m.invRho = C(1) / (m.rb + C(1));
+    m.rb = SCALED ? sum * invS : sum;
+    m.rho = SCALED ? fmac(sum, invS, C(1)) : sum + C(1);
+    m.j0 = SCALED ? (sxp - sxm) * invS : sxp - sxm;
+    m.j1 = SCALED ? (syp - sym) * invS : syp - sym;
+    m.j2 = SCALED ? (szp - szm) * invS : szp - szm;
+    m.invRho = recip(m.rho);
     return m;
 }
 
@@ -156,69 +179,69 @@ __device__ __forceinline__ void velocity_compact(const CellMoments<C>& m, const 
 
 // Relaxation of one cell from its moments (scaled populations in, scaled populations out).
 template <class C, int COLL>
-__device__ __forceinline__ void relax_compact(C* f, const C* F, C omega, C S, const CellMoments<C>& m) {
-    const C rb = m.rb, j0 = m.j0, j1 = m.j1, j2 = m.j2, invRho = m.invRho;
-    if (COLL == BIB_COLLISION_TRT) {
+__device__ __forceinline__ void relax_compact(C* f, const C* F, const RelaxRates<C>& r, const CellMoments<C>& m) {
+    const C j0 = m.j0, j1 = m.j1, j2 = m.j2;
+    if constexpr (COLL == BIB_COLLISION_TRT) {
         // Two relaxation times around the BGK equilibrium of j: the symmetric part of each
-        // pair (i, i+9) relaxes with omega, the antisymmetric part with omega_minus (passed
-        // in F[0]); feq+ = t_i (rhoBar + 4.5 (c.j)^2 / rho - 1.5 j.j / rho), feq- = 3 t_i c.j.
+        // pair (i, i+9) relaxes with omega, the antisymmetric part with omega_minus;
+        // feq+ = t_i (rhoBar + 4.5 (c.j)^2 / rho - 1.5 j.j / rho), feq- = 3 t_i c.j.
         // Collected per pair: f_i' = a f_i + b f_i+9 + (w feq+ + w- feq-) and f_i+9' = a f_i+9 +
         // b f_i + (w feq+ - w- feq-), with a = 1 - (w + w-)/2 and b = (w- - w)/2.
-        const C omm = F[0];
-        const C base = rb - C(1.5) * invRho * (j0 * j0 + j1 * j1 + j2 * j2);
-        const C h = C(4.5) * invRho;
-        const C a = C(1) - C(0.5) * (omega + omm), b = C(0.5) * (omm - omega);
-        const C oS = omega * S, mS3 = C(3) * omm * S;
-        f[0] = fmac(C(1) - omega, f[0], (oS * weight<C>(0)) * base);
+        const C jj = fmac(j2, j2, fmac(j1, j1, j0 * j0));
+        const C base = fmac(C(-1.5) * m.invRho, jj, m.rb), B = r.t * base, h = r.t * (C(4.5) * m.invRho);
+        const C B2 = B + B, h2 = h + h, mp = r.m, mp2 = mp + mp;
+        f[0] = fmac(r.omo, f[0], r.t0 * base);
 #pragma unroll
         for (int i = 1; i < 10; ++i) {
-            const C cj = cdot<C>(i, j0, j1, j2);
-            const C P = (oS * weight<C>(i)) * fmac(h * cj, cj, base), M = (mS3 * weight<C>(i)) * cj;
+            const bool axis = i < 4;
+            const C cj = cdot<C>(i + 9, j0, j1, j2);
+            const C P = fmac((axis ? h2 : h) * cj, cj, axis ? B2 : B);
             const C fi = f[i], fo = f[i + 9];
-            f[i] = fmac(a, fi, fmac(b, fo, P + M));
-            f[i + 9] = fmac(a, fo, fmac(b, fi, P - M));
+            f[i] = fmac(r.a, fi, fmac(r.b, fo, fmac(axis ? -mp2 : -mp, cj, P)));
+            f[i + 9] = fmac(r.a, fo, fmac(r.b, fi, fmac(axis ? mp2 : mp, cj, P)));
         }
-        return;
-    }
-    const bool forced = COLL == BIB_COLLISION_BGK_GUO_VOF;
-    const C F0 = forced ? F[0] : C(0), F1 = forced ? F[1] : C(0), F2 = forced ? F[2] : C(0);
-    const C u0 = fmac(j0, invRho, C(0.5) * F0), u1 = fmac(j1, invRho, C(0.5) * F1), u2 = fmac(j2, invRho, C(0.5) * F2);
-    const C rho = rb + C(1);
-    const C mu = C(1) - C(0.5) * omega;
-    const C wr = omega * rho;
-    const C A = omega * rb - C(1.5) * wr * (u0 * u0 + u1 * u1 + u2 * u2) - C(3) * mu * (u0 * F0 + u1 * F1 + u2 * F2);
-    const C h3 = C(3) * wr, m3 = C(3) * mu, g45 = C(4.5) * wr, m9 = C(9) * mu;
-    const C H0 = fmac(h3, u0, m3 * F0), H1 = fmac(h3, u1, m3 * F1), H2 = fmac(h3, u2, m3 * F2);
-    const C G0 = fmac(g45, u0, m9 * F0), G1 = fmac(g45, u1, m9 * F1), G2 = fmac(g45, u2, m9 * F2);
-    const C omo = C(1) - omega;
-    f[0] = fmac(omo, f[0], (S * weight<C>(0)) * A);
+    } else {
+        const C wr = r.w * m.rho, c3 = C(3) * wr, c45 = C(4.5) * wr;
+        C u[3], H[3], K[3];
+        const C j[3] = {j0, j1, j2};
 #pragma unroll
-    for (int i = 1; i < 10; ++i) {
-        const C cu = cdot<C>(i, u0, u1, u2), cG = cdot<C>(i, G0, G1, G2), cH = cdot<C>(i, H0, H1, H2);
-        const C tw = S * weight<C>(i);
-        const C P = tw * fmac(cu, cG, A), M = tw * cH;
-        f[i] = fmac(omo, f[i], P + M);
-        f[i + 9] = fmac(omo, f[i + 9], P - M);
+        for (int a = 0; a < 3; ++a) {
+            if constexpr (COLL == BIB_COLLISION_BGK_GUO_VOF) {
+                const C mF = r.m * F[a];
+                u[a] = fmac(j[a], m.invRho, C(0.5) * F[a]);
+                H[a] = fmac(c3, u[a], mF);
+                K[a] = fmac(c45, u[a], C(3) * mF);
+            } else {
+                u[a] = j[a] * m.invRho;
+                H[a] = c3 * u[a];
+                K[a] = c45 * u[a];
+            }
+        }
+        const C A = fmac(C(-1.0 / 3.0), fmac(u[2], K[2], fmac(u[1], K[1], u[0] * K[0])), r.w * m.rb);
+        const C tp = r.t, tp2 = tp + tp;
+        f[0] = fmac(r.omo, f[0], r.t0 * A);
+#pragma unroll
+        for (int i = 1; i < 4; ++i) {
+            const C P = tp2 * fmac(u[i - 1], K[i - 1], A);
+            f[i] = fmac(r.omo, f[i], fmac(-tp2, H[i - 1], P));
+            f[i + 9] = fmac(r.omo, f[i + 9], fmac(tp2, H[i - 1], P));
+        }
+#pragma unroll
+        for (int i = 4; i < 10; ++i) {
+            const C cu = cdot<C>(i + 9, u[0], u[1], u[2]), cK = cdot<C>(i + 9, K[0], K[1], K[2]);
+            const C cH = cdot<C>(i + 9, H[0], H[1], H[2]);
+            const C P = tp * fmac(cu, cK, A);
+            f[i] = fmac(r.omo, f[i], fmac(-tp, cH, P));
+            f[i + 9] = fmac(r.omo, f[i + 9], fmac(tp, cH, P));
+        }
     }
-}
-
-template <class C, int COLL>
-__device__ __forceinline__ void collide_compact(C* f, const C* F, C omega, C S, C invS, const C* Fprev, C* u_prev) {
-    const CellMoments<C> m = moments_compact<C>(f, invS);
-    if (u_prev) velocity_compact<C>(m, Fprev, u_prev);
-    relax_compact<C, COLL>(f, F, omega, S, m);
 }
 
 // The compact operators at unit scale (FP64 / FP32 populations held as f-bar): omega_minus is the
 // TRT rate of the antisymmetric parts, unused otherwise.
 template <class C, int COLL>
 __device__ __forceinline__ void collide_unscaled(C* f, const C* F, C omega, C omega_minus) {
-    if (COLL == BIB_COLLISION_TRT) {
-        const C Fm[3] = {omega_minus, C(0), C(0)};
-        collide_compact<C, COLL>(f, Fm, omega, C(1), C(1), nullptr, nullptr);
-    } else {
-        collide_compact<C, COLL>(f, F, omega, C(1), C(1), nullptr, nullptr);
-    }
+    relax_compact<C, COLL>(f, F, relax_rates<C, COLL>(omega, omega_minus, C(1)), moments_compact<C, false>(f, C(1)));
 }
 
 __host__ __device__ inline int64_t wrap_index(int64_t i, int64_t n) { return i < 0 ? i + n : (i >= n ? i - n : i); }

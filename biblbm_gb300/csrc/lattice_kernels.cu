@@ -416,15 +416,15 @@ __device__ __forceinline__ void fd_wall_node_rebuild(const LatticeDesc& d, const
     Store<T>::store(wall + wk, weight<C>(0) * (base - third), d.scale);
 #pragma unroll
     for (int i = 1; i < 10; ++i) {
-        const C cj = cdot<C>(i, j[0], j[1], j[2]);
+        const C cj = cdot<C>(i + 9, j[0], j[1], j[2]);
         C even = fmac(h * cj, cj, base) - third;
         if (cy(i) != 0) {
             even += pyy;
             if (cx(i) != 0) even += C(cx(i) * cy(i)) * pxy;
             if (cz(i) != 0) even += C(cy(i) * cz(i)) * pyz;
         }
-        Store<T>::store(wall + i * ws + wk, weight<C>(i) * fmac(C(3), cj, even), d.scale);
-        Store<T>::store(wall + (i + 9) * ws + wk, weight<C>(i) * fmac(C(-3), cj, even), d.scale);
+        Store<T>::store(wall + i * ws + wk, weight<C>(i) * fmac(C(-3), cj, even), d.scale);
+        Store<T>::store(wall + (i + 9) * ws + wk, weight<C>(i) * fmac(C(3), cj, even), d.scale);
     }
 }
 template <class T>

@@ -140,18 +140,6 @@ __device__ __forceinline__ void store_cell<__half, float>(__half* o, int64_t str
     *o = __float2half_rn(f[Q - 1]);
 }
 
-// Collision of one cell in storage units: the compact pairwise forms (BGK + Guo, BGK, TRT) in the
-// compute type.  With u non-null the velocity j/rho + Fp/2 of the incoming state is returned.
-template <class C, int COLL>
-__device__ __forceinline__ void staged_relax(C* f, const C* F, C om, C omm, C S, const CellMoments<C>& m) {
-    if constexpr (COLL == BIB_COLLISION_TRT) {
-        const C Fm[3] = {omm, C(0), C(0)};  // the TRT branch takes omega_minus in F[0]
-        relax_compact<C, COLL>(f, Fm, om, S, m);
-    } else {
-        relax_compact<C, COLL>(f, F, om, S, m);
-    }
-}
-
 // Tile pitch in cells: the shared-memory row of one population holds up to TILE cells, so
 // every staged address is a per-thread base plus a compile-time offset.
 template <class T>
@@ -213,9 +201,9 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
         store_cell<T, C>(fout + k, d.stride, f);
         return;
     }
-    C om = cp.om0;
-    if (COLL == BIB_COLLISION_BGK_GUO_VOF && d.use_phase && phase[k]) om = cp.om1;
-    const CellMoments<C> m = moments_compact<C>(f, cp.invS);
+    RelaxRates<C> r = cp.r[0];
+    if (COLL == BIB_COLLISION_BGK_GUO_VOF && d.use_phase && phase[k]) r = cp.r[1];
+    const CellMoments<C> m = moments_compact<C, sizeof(T) == 2>(f, cp.invS);
     if (UVEL) {
         // the velocity is stored before the relaxation, so that the previous force is dead while
         // the relaxation runs
@@ -229,7 +217,7 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
         }
         store_u_from<UT, C>(u_out, k, u[0], u[1], u[2]);
     }
-    staged_relax<C, COLL>(f, F, om, cp.omm, cp.S, m);
+    relax_compact<C, COLL>(f, F, r, m);
     store_cell<T, C>(fout + k, d.stride, f);
 }
 
@@ -250,12 +238,16 @@ inline int optin_smem() {
 template <class C>
 CollideParams<C> collide_params(const LatticeDesc& d, int storage) {
     CollideParams<C> cp{};
-    const bool phase_omega = d.collision == BIB_COLLISION_BGK_GUO_VOF;
-    cp.om0 = (C)(phase_omega ? d.omega_c0 : d.omega);
-    cp.om1 = (C)(phase_omega ? d.omega_c1 : d.omega);
-    cp.omm = (C)(1.0 / (d.trt_magic / (1.0 / d.omega - 0.5) + 0.5));
     const double S = storage == BIB_STORAGE_F16 ? (double)d.scale : 1.0;
-    cp.S = (C)S;
+    const C omm = (C)(1.0 / (d.trt_magic / (1.0 / d.omega - 0.5) + 0.5));
+    if (d.collision == BIB_COLLISION_BGK_GUO_VOF) {
+        cp.r[0] = relax_rates<C, BIB_COLLISION_BGK_GUO_VOF>((C)d.omega_c0, C(0), (C)S);
+        cp.r[1] = relax_rates<C, BIB_COLLISION_BGK_GUO_VOF>((C)d.omega_c1, C(0), (C)S);
+    } else if (d.collision == BIB_COLLISION_TRT) {
+        cp.r[0] = cp.r[1] = relax_rates<C, BIB_COLLISION_TRT>((C)d.omega, omm, (C)S);
+    } else {
+        cp.r[0] = cp.r[1] = relax_rates<C, BIB_COLLISION_BGK>((C)d.omega, C(0), (C)S);
+    }
     cp.invS = (C)(storage == BIB_STORAGE_F16 ? (double)d.inv_scale : 1.0);
     for (int q = 0; q < 3; ++q) {
         cp.body[q] = (C)d.body[q];
