@@ -158,20 +158,21 @@ __device__ __forceinline__ int64_t load_tile(const LatticeDesc& d, const StagedG
     return t.row0;
 }
 
-// Consumer side of one tile: the thread's cell of every tile and its x-neighbours (periodic in
-// x within the row).
+// Consumer side of one tile: the thread's cells of every tile (one, or the two from o0) and their
+// x-neighbours (periodic in x within the row).
 struct TileCell {
     bool active;
     int r, o0, ol, orr;
 };
+template <int CELLS>
 __device__ __forceinline__ TileCell tile_cell(const LatticeDesc& d, int Ct, int ct) {
     TileCell c;
-    c.active = ct < Ct;
-    c.r = ct / d.nx;
-    const int x = ct - c.r * d.nx;
-    c.o0 = ct;
+    c.o0 = CELLS * ct;
+    c.active = c.o0 < Ct;
+    c.r = c.o0 / d.nx;
+    const int x = c.o0 - c.r * d.nx;
     c.ol = c.r * d.nx + (x == 0 ? d.nx - 1 : x - 1);
-    c.orr = c.r * d.nx + (x == d.nx - 1 ? 0 : x + 1);
+    c.orr = c.r * d.nx + (x + CELLS >= d.nx ? 0 : x + CELLS);
     return c;
 }
 
@@ -229,6 +230,128 @@ __device__ __forceinline__ void consume_cell(const LatticeDesc& d, const StagedG
     if (lane == 0) mbar_arrive(empty_s);
     if (!active) return;
     finish_cell<T, CPL, COLL>(d, cp, fout, u_out, phase, celltype, t.row0 + o0, y, fd, f, F, Fp);
+}
+
+// FP16: two neighbouring cells per consumer thread, in packed FP32 arithmetic.  At one cell per thread the
+// kernel was bound by instruction issue (72 % of the slots at 384^3 TRT, 458 instructions per cell's
+// warp); a pair takes one arithmetic instruction, one store and one address for both.  Measured: 384^3 TRT, 60 steps in a
+// row, 1208 us per step at one cell per thread, 964 in pairs (a launch alone 730, 86 % of the copy rate); coupled in
+// 512 x 128 x 128, near its bytes either way, 340 us per step of the 400-cell channel where it was 341.
+// Nodes that are not collided are stored from the same registers; by a branch of one cell at a time the kernel spilled.
+template <int CPL, int COLL>
+__device__ __forceinline__ void consume_pair(const LatticeDesc& d, const StagedGeom& g, int64_t tile, const unsigned char* st,
+                                             const CollideParams<float>& cp, __half* __restrict__ fout,
+                                             __half* __restrict__ u_out, const uint8_t* __restrict__ phase,
+                                             const uint8_t* __restrict__ celltype, const TileCell& cell, uint64_t* empty_s,
+                                             int lane) {
+    using L = StageLayout<__half, CPL, COLL>;
+    constexpr int TILE = L::TILE;
+    constexpr bool UVEL = writes_u(CPL);
+    const TileRef t = tile_ref(d, g, tile);
+    const int y = t.y0 + cell.r, o0 = cell.o0;
+    const int64_t k = t.row0 + o0;
+    const bool fd = fd_wall_node(d, y);
+    const __half* P = reinterpret_cast<const __half*>(st);
+    F2 f[Q], F[3], Fp[3];
+    int types = 0;  // of the two cells, a byte each
+    if (cell.active) {
+        auto straight = [&](int i) { return F2(__half22float2(*reinterpret_cast<const __half2*>(P + i * TILE + o0))); };
+        auto shifted = [&](int i) {
+            if (cx(i) == 0) return straight(i);
+            return cx(i) == 1 ? F2(__half2float(P[i * TILE + cell.ol]), __half2float(P[i * TILE + o0]))
+                              : F2(__half2float(P[i * TILE + o0 + 1]), __half2float(P[i * TILE + cell.orr]));
+        };
+        if (!row_special(d, y, t.z)) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) f[i] = shifted(i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                int face = -1;
+                if (!fd) {
+                    int64_t srow;
+                    face = source_row(d, i, y, t.z, srow);
+                }
+                f[i] = !fd && face < 0 ? shifted(i) : straight(i);
+                if (face >= 0) f[i] = f[i] + F2(cp.mw[face][i]);
+            }
+        }
+        const float* SFc = reinterpret_cast<const float*>(st + L::OFF_FCOL) + 3 * o0;
+        const float* SFp = reinterpret_cast<const float*>(st + L::OFF_FPREV) + 3 * o0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if (L::NEED_FCOL) F[q] = F2(SFc[q], SFc[3 + q]);
+            if (CPL == kCplDense) Fp[q] = F2(SFp[q], SFp[3 + q]);
+            else if (CPL == kCplSparse) Fp[q] = F2(cp.body[q]);
+        }
+    }
+    // the stage has been read into registers: hand it back to the producer
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_s);
+    if (!cell.active) return;
+    __half* o = fout + k;
+    if (d.has_types) {
+        types = *reinterpret_cast<const uint16_t*>(celltype + k);
+        if (types != 0) {
+            // nodes that are not collided are stored now, the other cell of their pair below
+            static_assert(BIB_CELL_FLUID == 0, "two fluid cells read as one zero word");
+            const int ta = types & 255, tb = types >> 8;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                if (ta) o[i * d.stride] = __float2half_rn(ta == BIB_CELL_BOUNCE_BACK ? f[opposite(i)].v.x : f[i].v.x);
+                if (tb) o[i * d.stride + 1] = __float2half_rn(tb == BIB_CELL_BOUNCE_BACK ? f[opposite(i)].v.y : f[i].v.y);
+            }
+        }
+    }
+    bool p0 = false, p1 = false;
+    if (COLL == BIB_COLLISION_BGK_GUO_VOF && d.use_phase) {
+        p0 = phase[k] != 0;
+        p1 = phase[k + 1] != 0;
+    }
+    auto rate = [&](float a, float b) { return F2(p0 ? b : a, p1 ? b : a); };
+    const RelaxRates<float>&r0 = cp.r[0], &r1 = cp.r[1];
+    const RelaxRates<F2> r{rate(r0.omo, r1.omo), rate(r0.w, r1.w), rate(r0.m, r1.m), rate(r0.t0, r1.t0), rate(r0.t, r1.t),
+                           rate(r0.a, r1.a), rate(r0.b, r1.b)};
+    const CellMoments<F2> m = moments_compact<F2, true>(f, F2(cp.invS));
+    if (UVEL) {
+        F2 u[3];
+        if (fd) {
+            const int side = y == 0 ? 0 : 1;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) u[q] = F2(cp.wall_u[side][q]);
+        } else {
+            velocity_compact<F2>(m, Fp, u);
+        }
+        if (types & 255) u[0].v.x = u[1].v.x = u[2].v.x = 0.0f;
+        if (types >> 8) u[0].v.y = u[1].v.y = u[2].v.y = 0.0f;
+        alignas(16) __half2 w[4] = {__floats2half2_rn(u[0].v.x, u[1].v.x), __floats2half2_rn(u[2].v.x, 0.0f),
+                        __floats2half2_rn(u[0].v.y, u[1].v.y), __floats2half2_rn(u[2].v.y, 0.0f)};
+        *reinterpret_cast<uint4*>(u_out + 4 * k) = *reinterpret_cast<const uint4*>(w);
+    }
+    relax_compact<F2, COLL>(f, F, r, m);
+    if (types == 0) {
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            *reinterpret_cast<__half2*>(o) = __float22half2_rn(f[i].v);
+            o += d.stride;
+        }
+    } else if ((types & 255) == 0 || types >> 8 == 0) {
+        const bool second = (types & 255) != 0;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) o[i * d.stride + second] = __float2half_rn(second ? f[i].v.y : f[i].v.x);
+    }
+}
+
+// A consumer thread's cells of one tile.
+template <class T, int CPL, int COLL>
+__device__ __forceinline__ void consume(const LatticeDesc& d, const StagedGeom& g, int64_t tile, const unsigned char* st,
+                                        const CollideParams<typename Store<T>::C>& cp, T* __restrict__ fout,
+                                        typename Store<T>::U* __restrict__ u_out, const uint8_t* __restrict__ phase,
+                                        const uint8_t* __restrict__ celltype, const TileCell& cell, uint64_t* empty_s, int lane) {
+    if constexpr (StageLayout<T, CPL, COLL>::CELLS == 2)
+        consume_pair<CPL, COLL>(d, g, tile, st, cp, fout, u_out, phase, celltype, cell, empty_s, lane);
+    else
+        consume_cell<T, CPL, COLL>(d, g, tile, st, cp, fout, u_out, phase, celltype, cell, empty_s, lane);
 }
 
 // Warp-specialised persistent kernel: warp 0 produces, warps 1..CONSUMERS collide.  Stage
@@ -299,8 +422,8 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
         return;
     }
 
-    // ---- consumers: thread `ct` owns cell ct of every tile
-    const TileCell cell = tile_cell(d, g.Ct, tid - 32);
+    // ---- consumers: thread `ct` owns cell ct, or cells 2 ct and 2 ct + 1, of every tile
+    const TileCell cell = tile_cell<L::CELLS>(d, g.Ct, tid - 32);
     int it = 0;
     for (int64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x, ++it) {
         const int s = it % NS;
@@ -310,7 +433,7 @@ __global__ void __launch_bounds__(StageLayout<T, CPL, COLL>::THREADS, staged_cta
             if (lane == 0) atomicExch(wait_err, 1);
             return;
         }
-        consume_cell<T, CPL, COLL>(d, g, tile, stages + s * L::BYTES, cp, fout, u_out, phase, celltype, cell, &empty[s], lane);
+        consume<T, CPL, COLL>(d, g, tile, stages + s * L::BYTES, cp, fout, u_out, phase, celltype, cell, &empty[s], lane);
     }
 }
 
@@ -447,12 +570,12 @@ __global__ void __launch_bounds__(StageLayout<T, kCplDense, COLL>::THREADS, stag
             asm volatile("bar.sync 1, %0;" ::"r"(L::CONSUMERS * 32) : "memory");
             copy_view(cview, views + vi, tid - 32, L::CONSUMERS * 32);
             asm volatile("bar.sync 1, %0;" ::"r"(L::CONSUMERS * 32) : "memory");
-            cell = tile_cell(cview->d, cview->Ct, tid - 32);  // depends on the lattice's row length
+            cell = tile_cell<L::CELLS>(cview->d, cview->Ct, tid - 32);  // depends on the lattice's row length
             cur_view = vi;
         }
         const CollideView& V = *cview;
-        consume_cell<T, kCplDense, COLL>(V.d, view_geom(V, NS), tile - V.tile0, stages + s * L::BYTES,
-                                         *reinterpret_cast<const CollideParams<C>*>(V.cp), static_cast<T*>(V.fout),
+        consume<T, kCplDense, COLL>(V.d, view_geom(V, NS), tile - V.tile0, stages + s * L::BYTES,
+                                    *reinterpret_cast<const CollideParams<C>*>(V.cp), static_cast<T*>(V.fout),
                                          static_cast<typename Store<T>::U*>(V.u), V.phase, V.celltype, cell, &empty[s], lane);
     }
 }

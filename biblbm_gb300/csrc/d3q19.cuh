@@ -129,6 +129,21 @@ __device__ __forceinline__ double fmac(double a, double b, double c) { return fm
 __device__ __forceinline__ float recip(float a) { return 1.0f / a; }
 __device__ __forceinline__ double recip(double a) { return 1.0 / a; }
 
+// Two cells' FP32 values in one register pair: an instruction for both, rounded as for one.
+struct F2 {
+    float2 v;
+    F2() = default;
+    __device__ __forceinline__ explicit F2(float a) : v(make_float2(a, a)) {}
+    __device__ __forceinline__ F2(float a, float b) : v(make_float2(a, b)) {}
+    __device__ __forceinline__ explicit F2(float2 a) : v(a) {}
+};
+__device__ __forceinline__ F2 fmac(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2(__fadd2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return F2(__fadd2_rn(a.v, make_float2(-b.v.x, -b.v.y))); }
+__device__ __forceinline__ F2 operator-(F2 a) { return F2(-a.v.x, -a.v.y); }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 recip(F2 a) { return F2(1.0f / a.v.x, 1.0f / a.v.y); }
+
 template <class C, int COLL>
 __host__ __device__ __forceinline__ RelaxRates<C> relax_rates(C w, C wm, C S) {
     const bool trt = COLL == BIB_COLLISION_TRT;

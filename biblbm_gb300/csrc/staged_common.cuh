@@ -161,7 +161,8 @@ template <class T, int CPL, int COLL>
 struct StageLayout {
     using FT = typename Store<T>::F;
     static constexpr int TILE = TileOf<T>::value;
-    static constexpr int CONSUMERS = TILE / 32;  // consumer warps: one cell per thread and tile
+    static constexpr int CELLS = sizeof(T) == 2 ? 2 : 1;  // per consumer thread and tile
+    static constexpr int CONSUMERS = TILE / 32 / CELLS;   // consumer warps
     static constexpr int THREADS = 32 * (CONSUMERS + 1);
     static constexpr bool NEED_FCOL = COLL == BIB_COLLISION_BGK_GUO_VOF;
     static constexpr unsigned POP = TILE * sizeof(T);
