@@ -260,39 +260,45 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
         S.area += ar;
         S.volume += dt(a, crs(b, c)) / 6.;
     }
-    struct L {
-        int t1 = -1, t2 = -1;
-        double len = 0;
+    // edges by (smaller, larger vertex), with the first triangle of each and the last other one: the triangles'
+    // edges bucketed by their smaller vertex, each bucket (a few entries) ordered by the larger one
+    struct Edge {
+        int i1, t;
     };
-    std::map<std::pair<int, int>, L> links;
-    for (int64_t t = 0; t < nt; ++t) {
-        int ind[4] = {S.tri[3 * t], S.tri[3 * t + 1], S.tri[3 * t + 2], S.tri[3 * t]};
-        for (int j = 0; j < 3; ++j) {
-            std::pair<int, int> key(std::min(ind[j], ind[j + 1]), std::max(ind[j], ind[j + 1]));
-            auto it = links.find(key);
-            if (it == links.end()) {
-                L l;
-                l.t1 = (int)t;
-                l.len = nrm(sub(P(key.first), P(key.second)));
-                links.emplace(key, l);
-            } else if (it->second.t1 != (int)t) {
-                it->second.t2 = (int)t;
+    std::vector<int> first((size_t)nv + 1, 0);
+    auto each_edge = [&](auto&& f) {
+        for (int64_t t = 0; t < nt; ++t)
+            for (int j = 0; j < 3; ++j) {
+                const int p = S.tri[3 * t + j], q = S.tri[3 * t + (j + 1) % 3];
+                f(std::min(p, q), Edge{std::max(p, q), (int)t});
             }
+    };
+    each_edge([&](int i0, Edge) { ++first[(size_t)i0 + 1]; });
+    for (int64_t v = 0; v < nv; ++v) first[(size_t)v + 1] += first[(size_t)v];
+    std::vector<Edge> edges(3 * (size_t)nt);
+    std::vector<int> fill(first.begin(), first.end() - 1);
+    each_edge([&](int i0, Edge e) { edges[(size_t)fill[(size_t)i0]++] = e; });
+    for (int64_t v = 0; v < nv; ++v) {
+        Edge *lo = edges.data() + first[(size_t)v], *hi = edges.data() + first[(size_t)v + 1];
+        if (hi - lo > 32) {
+            std::stable_sort(lo, hi, [](const Edge& x, const Edge& y) { return x.i1 < y.i1; });
+            continue;
         }
+        for (Edge* e = lo; e < hi; ++e)
+            for (Edge* at = e; at > lo && at->i1 < at[-1].i1; --at) std::swap(*at, at[-1]);
     }
     S.links.clear();
     S.link_len.clear();
     S.pairs.clear();
     S.pair_cs.clear();
     std::vector<std::pair<int, int>> edge_of;  // the triangles of each pair
-    for (auto& kv : links) {
-        const int i0 = kv.first.first, i1 = kv.first.second;
+    auto link = [&](int i0, int i1, int t1, int t2) {
         S.links.push_back(i0);
         S.links.push_back(i1);
-        S.link_len.push_back(kv.second.len);
-        if (kv.second.t1 < 0 || kv.second.t2 < 0) continue;
-        int a[3] = {S.tri[3 * kv.second.t1], S.tri[3 * kv.second.t1 + 1], S.tri[3 * kv.second.t1 + 2]};
-        int b[3] = {S.tri[3 * kv.second.t2], S.tri[3 * kv.second.t2 + 1], S.tri[3 * kv.second.t2 + 2]};
+        S.link_len.push_back(nrm(sub(P(i0), P(i1))));
+        if (t2 < 0) return;
+        int a[3] = {S.tri[3 * t1], S.tri[3 * t1 + 1], S.tri[3 * t1 + 2]};
+        int b[3] = {S.tri[3 * t2], S.tri[3 * t2 + 1], S.tri[3 * t2 + 2]};
         for (int g = 0; g < 3 && !((a[0] == i0 && a[2] == i1) || (a[0] == i1 && a[2] == i0)); ++g) {
             int tmp = a[0]; a[0] = a[2]; a[2] = a[1]; a[1] = tmp;
         }
@@ -301,7 +307,7 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
         }
         const int q[4] = {a[0], a[1], a[2], b[2]};
         for (int k = 0; k < 4; ++k) S.pairs.push_back(q[k]);
-        edge_of.emplace_back(kv.second.t1, kv.second.t2);
+        edge_of.emplace_back(t1, t2);
         V3d p0 = P(q[0]), p1 = P(q[1]), p2 = P(q[2]), p3 = P(q[3]);
         V3d n1 = crs(sub(p1, p0), sub(p2, p0));
         n1 = scl(n1, nrm(n1));
@@ -309,7 +315,15 @@ bool build_shape(ShapeHost& S, const double* xyz, const int64_t* tri, int64_t nv
         n2 = scl(n2, nrm(n2));
         S.pair_cs.push_back(dt(n1, n2));
         S.pair_cs.push_back((dt(sub(n1, n2), sub(p1, p3)) > 0 ? 1.0 : -1.0) * nrm(crs(n1, n2)));
-    }
+    };
+    for (int64_t v = 0; v < nv; ++v)
+        for (int e = first[(size_t)v]; e < first[(size_t)v + 1];) {
+            const int i1 = edges[(size_t)e].i1, t1 = edges[(size_t)e].t;
+            int t2 = -1;
+            for (; e < first[(size_t)v + 1] && edges[(size_t)e].i1 == i1; ++e)
+                if (edges[(size_t)e].t != t1) t2 = edges[(size_t)e].t;
+            link((int)v, i1, t1, t2);
+        }
     // rest lengths and angle of every triangle, and FP32 copies of the rest-state constants for the
     // reduced-precision element kernels
     S.tri_rest.resize(4 * nt);
