@@ -69,7 +69,7 @@ __device__ __forceinline__ PopLane pop_lane(int lane) {
 // loaded anew (its consumers have handed it back, so the previous force has been read).  Stores from
 // the consumers would touch every third word three times.  After the loads, which the refill of the
 // stage waits for, and from the tile's number: with the run kept per stage in lane registers the FP16
-// kernel at its 56 registers took 168.5 us for 512 x 128 x 128 cells, so 160.8 (162.7 with one force
+// kernel, then at one cell per thread and 56 registers, took 168.5 us for 512 x 128 x 128 cells, so 160.8 (162.7 with one force
 // array per component and the reset stored by the consumers).
 template <class FT>
 __device__ __forceinline__ void reset_tile(const LatticeDesc& d, const StagedGeom& g, int64_t tile, FT* Fprev, const FT* reset) {

@@ -80,46 +80,22 @@ struct Staged;
 template <>
 struct Staged<__half> {
     static __device__ __forceinline__ float one(const __half* p) { return __half2float(*p); }
-    static __device__ __forceinline__ void two(const __half* p, float& a, float& b) {
-        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(p));
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store(__half* p, float a, float b) {
-        *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
-    }
     static __device__ __forceinline__ void put(__half* p, float a) { *p = __float2half_rn(a); }
 };
 template <>
 struct Staged<float> {
     static __device__ __forceinline__ float one(const float* p) { return *p; }
-    static __device__ __forceinline__ void two(const float* p, float& a, float& b) {
-        const float2 v = *reinterpret_cast<const float2*>(p);
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store(float* p, float a, float b) {
-        *reinterpret_cast<float2*>(p) = make_float2(a, b);
-    }
     static __device__ __forceinline__ void put(float* p, float a) { *p = a; }
 };
 template <>
 struct Staged<double> {
     static __device__ __forceinline__ double one(const double* p) { return *p; }
-    static __device__ __forceinline__ void two(const double* p, double& a, double& b) {
-        const double2 v = *reinterpret_cast<const double2*>(p);
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store(double* p, double a, double b) {
-        *reinterpret_cast<double2*>(p) = make_double2(a, b);
-    }
     static __device__ __forceinline__ void put(double* p, double a) { *p = a; }
 };
 
 // The 19 post-collision values of one cell to their arrays (stride apart); FP16 converts two
-// values per instruction (same rounding; measured on the 400-cell channel: the collide-and-stream
-// 0.1763 -> 0.1748 ms, the lattice-only TRT kernel 56,680 -> 57,370 MLUPS at 384^3).
+// values per instruction (same rounding; measured on row tiles with one cell per thread, 400-cell channel:
+// 0.1763 -> 0.1748 ms).
 template <class T, class C>
 __device__ __forceinline__ void store_cell(T* o, int64_t stride, const C* f) {
 #pragma unroll
@@ -222,7 +198,7 @@ __device__ __forceinline__ void finish_cell(const LatticeDesc& d, const CollideP
     store_cell<T, C>(fout + k, d.stride, f);
 }
 
-// Resident CTAs per SM the kernel is built for: FP16 needs two (32 consumer warps) to hide
+// Resident CTAs per SM the kernels are built for: FP16 needs two (32 consumer warps; 16 of packed pairs) to hide
 // the latency of its arithmetic; FP32 and FP64 run one CTA with a deeper pipeline.
 template <class T>
 constexpr int staged_ctas_per_sm() {
