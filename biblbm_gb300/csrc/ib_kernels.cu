@@ -2048,17 +2048,24 @@ void launch_membrane_forces(const Lattice& L, cudaStream_t s) {
             k_membrane_gather<float><<<g, block, 0, s>>>(L.nvert, L.vert_particle, L.pdev, L.pos[L.pcur], L.force, L.stats, L.inter);
         return;
     }
-    // few particles: each particle's elements over several CTAs so the launch fills the GPU, about four warps
-    // per SM (bound by the FP64 pipe, 2 lanes per cycle and SM: a warp to itself is served as fast as it
-    // can issue).  One capsule of 1280 triangles, FP64: 8 CTAs of 256 threads 53.8 us, 60 of 32 36.9
-    // (23.6 with capsule_triangle's shared scalars)
+    // Few particles: each particle's elements over several CTAs so the launch fills the GPU.
+    // FP64: about four warps per SM (bound by the FP64 pipe, 2 lanes per cycle and SM: a warp to itself is served
+    // as fast as it can issue).  One capsule of 1280 triangles: 8 CTAs of 256 threads 53.8 us, 60 of 32 36.9
+    // (23.6 with capsule_triangle's shared scalars); the step of 40 red cells of 2562 vertices with link springs 793 us
+    // with the CTAs of the FP32 rule, so 734.
+    // FP32 (membranes with link springs, the others go by patches): two CTAs of membrane_block threads per SM, since
+    // every CTA clears, stages and adds the whole membrane.  Steps with such red cells, one-warp CTAs as in
+    // FP64 against these: 1 of 642 vertices 57.7 / 42.0 us, 10 76.0 / 62.5, 100 169 / 165; 1 of 2562 96.7 / 70.8, 10 112 / 83.6,
+    // 40 169 / 162.
+    const bool f64 = L.storage == BIB_STORAGE_F64;
     const int warps = (L.max_elems + 31) / 32;
-    const int split = std::min(warps, membrane_split(np, L.max_elems, 32, 4));
+    const int split = f64 ? std::min(warps, membrane_split(np, L.max_elems, 32, 4))
+                          : membrane_split(np, L.max_elems, L.membrane_block);
     if (split > 1) {
         const IbView v = single_view(L, -1);
         k_force_seed<<<(L.nvert + 127) / 128, 128, 0, s>>>(v);
         const dim3 grid((unsigned)np, (unsigned)split);
-        const int block = std::min(L.membrane_block, 32 * ((warps + split - 1) / split));
+        const int block = f64 ? std::min(L.membrane_block, 32 * ((warps + split - 1) / split)) : L.membrane_block;
         if (L.storage == BIB_STORAGE_F64) k_membrane<double, false><<<grid, block, L.membrane_smem, s>>>(L.pdev, v, nullptr);
         else k_membrane<float, false><<<grid, block, L.membrane_smem, s>>>(L.pdev, v, nullptr);
         return;
