@@ -822,15 +822,41 @@ void membrane_and_spread(bib_ctx* c, Lattice& L, int fbuf, bool record_nodes, bo
     record(c, 2);
 }
 
-// Few vertices in a large lattice: what the membranes need of the lattice, the velocity at their support
+// Few vertices in a lattice: what the membranes need of the lattice, the velocity at their support
 // nodes, is there before the collision (j/rho + F[fe]/2 of the state it starts from), so interpolation, move,
 // update and the next step's membrane forces run beside the collide-and-stream and the walls on a second
-// stream.  The collision then neither reads the previous force nor writes a velocity field.  Measured, steps of
-// one capsule or red cell between velocity walls, one after another against beside: FP32 64^3 with 642 vertices 38.9
-// / 29.7 us, 128 x 64 x 64 with 2562 57.4 / 44.1, 160 x 128 x 128 129 / 111, 33^3 with 162 23.6 / 20.1; FP16 64^3 34.8 / 29.8;
-// FP64 64^3 144 / 132, 33^3 82 / 56.
+// stream.  The collision then neither reads the previous force nor writes a velocity field.
+//
+// What it saves grows with the cells (20 to 28 bytes each) and with the latency of the membranes' kernels, what it
+// costs with the support nodes: 19 scattered loads each, once per vertex that shares it.  So the nodes have a limit
+// that rises with the cells of large lattices.  Steps one after another / beside, in us (R3, R4: red cells of 642, 2562
+// vertices with bending; S3: capsules of 642; 27 nodes per vertex):
+//   FP16  64^3 1 R3 33.8 / 29.6, 4 32.8 / 36.2; 160 x 128 x 128 1 R3 88.5 / 85.4, 4 88.7 / 96.6, 16 90.1 / 105;
+//     256 x 128 x 128 4 R3 120 / 108, 16 121 / 123; 512 x 128 x 128 14 R3 207 / 197, 48 219 / 235, 241 259 / 516
+//   FP32  64^3 1 R3 40.0 / 29.1, 4 40.4 / 35.0; 128 x 64 x 64 1 R4 49.3 / 43.2; 96^3 5 R3 60.5 / 65.2, 16 66.6 / 72.8;
+//     160 x 128 x 128 4 R3 120 / 114, 16 123 / 127; 512 x 128 x 128 48 R3 331 / 309, 96 343 / 361, 241 368 / 516
+//     link springs: 128 x 64 x 64 1 of 642 58.4 / 42.9, 1 of 2562 65.7 / 72.7
+//   FP64 with staged tiles, whose membranes want the pipe that the collision is bound by: 64^3 1 S3 137 / 126, 2 133 / 157,
+//     1 R3 153 / 161, 1 red cell of 162 vertices 147 / 122; 160 x 128 x 128 1 R3 922 / 889, 4 923 / 942, 2 S3 906 / 886
+//   FP64 with the direct kernels, for which the velocity field is dear: 129 x 65 x 65 1 R3 332 / 282, 8 S3 319 / 294;
+//     513 x 127 x 127 238 R3 (half a node per cell) 3999 / 3714.
+bool overlap_pays(const Lattice& L) {
+    if (!few_support_nodes(L)) return false;  // at most half as many nodes as cells
+    const int64_t sup = L.ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
+    const int64_t n = L.d.n, nodes = (int64_t)L.nvert * sup * sup * sup;
+    bool springs = false, pairs = false;  // membranes with link springs; with adjacent-triangle pairs
+    for (const ParticleHost& ph : L.parts) {
+        springs = springs || ph.model == BIB_MODEL_RBC_WLCPOW;
+        pairs = pairs || ph.model == BIB_MODEL_RBC_WLCPOW || ph.model == BIB_MODEL_SKALAK_BENDING;
+    }
+    if (L.storage == BIB_STORAGE_F16) return nodes <= std::max<int64_t>(40960, n / 16 - 131072);
+    if (L.storage == BIB_STORAGE_F32) return nodes <= std::max<int64_t>(springs ? 40960 : 81920, n / 6 - 196608);
+    if (L.collide_kernel == BIB_KERNEL_ROWS || !collide_staged_fits(L)) return true;
+    return nodes <= n / 64 + (pairs ? 5120 : 18432);
+}
+
 bool overlapped_step(const bib_ctx* c, const Lattice& L) {
-    return !c->profiling && few_support_nodes(L) && !L.phase && L.inter.npp == 0 && !sparse_coupling(L);
+    return !c->profiling && !L.phase && L.inter.npp == 0 && !sparse_coupling(L) && overlap_pays(L);
 }
 
 // One step of that kind, of a sequence: have_forces, the previous step has left this one's membrane forces;
