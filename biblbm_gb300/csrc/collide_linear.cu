@@ -291,25 +291,33 @@ bool linear_inst(const Lattice& L, cudaStream_t s) {
     }
     g.wait_ns = L.wait_ns;
     g.withhold = L.withhold_tile;
+    // pipeline depth: the tuning value, else as many stages as fit the resident CTAs of an SM.  The reset coupling takes
+    // them too, beside the membranes' kernels (three against four, steps of one 642-vertex capsule: FP16 65^3 30.3 / 30.7
+    // us, 129^3 77.0 / 79.8, FP32 101^3 64.1 / 63.3, 129^3 94.4 / 95.1; the same within 2 us at 33^3 to 129^3)
     const size_t limit = std::min<size_t>((size_t)optin_smem(), 228 * 1024 / staged_ctas_per_sm<T>()) - 1024;
-    g.nstages = 2;
-    for (int ns = 2; ns <= kMaxStages; ++ns)
+    g.nstages = L.stages >= 2 ? L.stages : 2;
+    for (int ns = 2; L.stages < 2 && ns <= kMaxStages; ++ns)
         if (linear_smem<T, CPL, COLL>(ns) <= limit) g.nstages = ns;
     const size_t smem = linear_smem<T, CPL, COLL>(g.nstages);
-    if (smem > limit) return false;
+    if (smem + 1024 > (size_t)optin_smem()) return false;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     auto kern = k_collide_stream_linear<T, CPL, COLL>;
-    // per device: the shared memory set and the resident CTAs per SM
+    // per device: the shared memory allowed (only ever raised) and, for each size, the resident CTAs per SM
     static std::mutex mu;
-    static std::unordered_map<int, int> resident;
+    static std::unordered_map<int, size_t> allowed;
+    static std::unordered_map<int64_t, int> resident;
     int nb = 0;
     {
         std::lock_guard<std::mutex> lock(mu);
-        int& r = resident[dev];
-        if (r == 0 && (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-                       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, LY::THREADS, smem) != cudaSuccess || r < 1)) {
+        size_t& lim = allowed[dev];
+        if (smem > lim) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+            lim = smem;
+        }
+        int& r = resident[((int64_t)dev << 32) | (int64_t)smem];
+        if (r == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, LY::THREADS, smem) != cudaSuccess || r < 1)) {
             r = 0;
             return false;
         }

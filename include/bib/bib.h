@@ -140,7 +140,7 @@ typedef struct {
 typedef struct {
     int32_t collide_kernel; /* BIB_KERNEL_*: AUTO takes the shared-memory staged kernel where the x-row fits */
     int32_t tile_cells;     /* staged kernel: cells per tile (whole x-rows); 0 = 512 (256 for FP64) */
-    int32_t stages;         /* staged kernel: pipeline depth 2..4; 0 = the deepest that keeps the CTAs resident */
+    int32_t stages;         /* staged kernels: pipeline depth 2..4; 0 = the deepest that keeps the CTAs resident */
     int32_t membrane_block; /* threads per particle of the membrane kernel: 64 .. 512 (power of two), 0 = 256 */
     int32_t force_reset;    /* BIB_FORCE_RESET_*: how the coupled step resets the previous force field */
     int32_t wait_limit_us;  /* staged kernel: bound of each hand-off wait between its warps, in microseconds
