@@ -833,8 +833,9 @@ void membrane_and_spread(bib_ctx* c, Lattice& L, int fbuf, bool record_nodes, bo
 // vertices with bending; S3: capsules of 642; 27 nodes per vertex):
 //   FP16  64^3 1 R3 33.8 / 29.6, 4 32.8 / 36.2; 160 x 128 x 128 1 R3 88.5 / 85.4, 4 88.7 / 96.6, 16 90.1 / 105;
 //     256 x 128 x 128 4 R3 120 / 108, 16 121 / 123; 512 x 128 x 128 14 R3 207 / 197, 48 219 / 235, 241 259 / 516
-//   FP32  64^3 1 R3 40.0 / 29.1, 4 40.4 / 35.0; 128 x 64 x 64 1 R4 49.3 / 43.2; 96^3 5 R3 60.5 / 65.2, 16 66.6 / 72.8;
-//     160 x 128 x 128 4 R3 120 / 114, 16 123 / 127; 512 x 128 x 128 48 R3 331 / 309, 96 343 / 361, 241 368 / 516
+//   FP32  64^3 1 R3 40.0 / 29.1, 2 39.9 / 39.6, 4 41.0 / 40.9; 96 x 40 x 40 2 R3 32.8 / 29.5, 4 32.5 / 34.1, 16 red cells
+//     of 162 30.7 / 33.9; one cell, whose kernels wait longer, 64^3 R4 41.9 / 35.1, 128 x 64 x 64 R4 49.3 / 43.2;
+//     160 x 128 x 128 4 R3 120 / 114, 16 123 / 127; 512 x 128 x 128 48 R3 331 / 309, 96 343 / 361, 241 368 / 516;
 //     link springs: 128 x 64 x 64 1 of 642 58.4 / 42.9, 1 of 2562 65.7 / 72.7
 //   FP64 with staged tiles, whose membranes want the pipe that the collision is bound by: 64^3 1 S3 137 / 126, 2 133 / 157,
 //     1 R3 153 / 161, 1 red cell of 162 vertices 147 / 122; 160 x 128 x 128 1 R3 922 / 889, 4 923 / 942, 2 S3 906 / 886
@@ -845,12 +846,13 @@ bool overlap_pays(const Lattice& L) {
     const int64_t sup = L.ib.dirac == BIB_DIRAC_PESKIN ? 4 : 3;
     const int64_t n = L.d.n, nodes = (int64_t)L.nvert * sup * sup * sup;
     bool springs = false, pairs = false;  // membranes with link springs; with adjacent-triangle pairs
+    const bool one = L.parts.size() == 1;
     for (const ParticleHost& ph : L.parts) {
         springs = springs || ph.model == BIB_MODEL_RBC_WLCPOW;
         pairs = pairs || ph.model == BIB_MODEL_RBC_WLCPOW || ph.model == BIB_MODEL_SKALAK_BENDING;
     }
     if (L.storage == BIB_STORAGE_F16) return nodes <= std::max<int64_t>(40960, n / 16 - 131072);
-    if (L.storage == BIB_STORAGE_F32) return nodes <= std::max<int64_t>(springs ? 40960 : 81920, n / 6 - 196608);
+    if (L.storage == BIB_STORAGE_F32) return nodes <= std::max<int64_t>(one && !springs ? 81920 : 40960, n / 6 - 196608);
     if (L.collide_kernel == BIB_KERNEL_ROWS || !collide_staged_fits(L)) return true;
     return nodes <= n / 64 + (pairs ? 5120 : 18432);
 }
