@@ -2804,35 +2804,38 @@ bib_status ckpt_get_device(bib_ctx* c, CkptFile& F, void* dev, size_t bytes, std
     return BIB_OK;
 }
 
-// A force field in the file's order, one array per component: component by component out of (into) the
-// device's cells of three.
-template <class FT>
-bib_status ckpt_put_force(bib_ctx* c, CkptFile& F, const Lattice& L, const void* dev) {
-    const int64_t stride = L.d.stride, chunk = (int64_t)(kCkptChunk / (3 * sizeof(FT)));
-    std::vector<FT> cells, one;
+// A force field in the file's order, one array per component, out of the device's cells of three: taken apart on the
+// device, in `part` (the population buffer that the next step overwrites), so that every value crosses the link
+// once and the host holds one chunk.
+bib_status ckpt_put_force(bib_ctx* c, CkptFile& F, const Lattice& L, int k, void* part, std::vector<unsigned char>& buf) {
+    const size_t w = force_bytes(L.storage);
+    const int64_t chunk = (int64_t)(kCkptChunk / w);
     for (int a = 0; a < 3; ++a)
-        for (int64_t k = 0; k < stride; k += chunk) {
-            const int64_t n = std::min(chunk, stride - k);
-            cells.resize((size_t)(3 * n));
-            one.resize((size_t)n);
-            BIB_CUDA(c, cudaMemcpy(cells.data(), static_cast<const FT*>(dev) + 3 * k, 3 * n * sizeof(FT), cudaMemcpyDeviceToHost));
-            for (int64_t i = 0; i < n; ++i) one[(size_t)i] = cells[(size_t)(3 * i + a)];
-            if (!F.put(one.data(), (size_t)n * sizeof(FT))) return fail(c, BIB_EINVAL, "checkpoint write failed");
+        for (int64_t o = 0; o < L.d.stride; o += chunk) {
+            const int64_t n = std::min(chunk, L.d.stride - o);
+            buf.resize((size_t)n * w);
+            launch_force_component(L, k, part, a, o, n, false, c->stream);
+            BIB_CHECK_LAUNCH(c);
+            BIB_CUDA(c, cudaMemcpyAsync(buf.data(), part, (size_t)n * w, cudaMemcpyDeviceToHost, c->stream));
+            BIB_CUDA(c, cudaStreamSynchronize(c->stream));
+            if (!F.put(buf.data(), (size_t)n * w)) return fail(c, BIB_EINVAL, "checkpoint write failed");
         }
     return BIB_OK;
 }
 
-template <class FT>
-bib_status ckpt_get_force(bib_ctx* c, CkptFile& F, const Lattice& L, void* dev) {
-    const int64_t stride = L.d.stride;
-    std::vector<FT> cells((size_t)(3 * stride)), one((size_t)std::min<int64_t>(stride, kCkptChunk / sizeof(FT)));
+bib_status ckpt_get_force(bib_ctx* c, CkptFile& F, const Lattice& L, int k, void* part, std::vector<unsigned char>& buf) {
+    const size_t w = force_bytes(L.storage);
+    const int64_t chunk = (int64_t)(kCkptChunk / w);
     for (int a = 0; a < 3; ++a)
-        for (int64_t k = 0; k < stride; k += (int64_t)one.size()) {
-            const int64_t n = std::min((int64_t)one.size(), stride - k);
-            if (!F.get(one.data(), (size_t)n * sizeof(FT))) return fail(c, BIB_EINVAL, "checkpoint file is truncated");
-            for (int64_t i = 0; i < n; ++i) cells[(size_t)(3 * (k + i) + a)] = one[(size_t)i];
+        for (int64_t o = 0; o < L.d.stride; o += chunk) {
+            const int64_t n = std::min(chunk, L.d.stride - o);
+            buf.resize((size_t)n * w);
+            if (!F.get(buf.data(), (size_t)n * w)) return fail(c, BIB_EINVAL, "checkpoint file is truncated");
+            BIB_CUDA(c, cudaMemcpyAsync(part, buf.data(), (size_t)n * w, cudaMemcpyHostToDevice, c->stream));
+            launch_force_component(L, k, part, a, o, n, true, c->stream);
+            BIB_CHECK_LAUNCH(c);
+            BIB_CUDA(c, cudaStreamSynchronize(c->stream));
         }
-    BIB_CUDA(c, cudaMemcpy(dev, cells.data(), cells.size() * sizeof(FT), cudaMemcpyHostToDevice));
     return BIB_OK;
 }
 
@@ -2897,9 +2900,7 @@ bib_status bib_checkpoint_save(bib_ctx* c, int32_t h, const char* path) {
     if ((st = ckpt_put_device(c, F, L->f[L->cur], pb, buf))) return st;
     if (L->d.fd_walls && (st = ckpt_put_device(c, F, L->wall, wall_bytes(*L), buf))) return st;
     for (int k = 0; k < 2; ++k)
-        if ((st = L->storage == BIB_STORAGE_F64 ? ckpt_put_force<double>(c, F, *L, L->F[k])
-                                                : ckpt_put_force<float>(c, F, *L, L->F[k])))
-            return st;
+        if ((st = ckpt_put_force(c, F, *L, k, L->f[1 - L->cur], buf))) return st;
     if (L->phase && (st = ckpt_put_device(c, F, L->phase, (size_t)L->d.stride, buf))) return st;
     if (L->celltype && (st = ckpt_put_device(c, F, L->celltype, (size_t)L->d.n, buf))) return st;
     for (const ParticleHost& ph : L->parts) {
@@ -2994,9 +2995,7 @@ bib_status bib_checkpoint_load(bib_ctx* c, int32_t h, const char* path) {
     if ((st = ckpt_get_device(c, F, L->f[hd.cur], pb, buf))) return st;
     if (L->d.fd_walls && (st = ckpt_get_device(c, F, L->wall, wall_bytes(*L), buf))) return st;
     for (int k = 0; k < 2; ++k)
-        if ((st = L->storage == BIB_STORAGE_F64 ? ckpt_get_force<double>(c, F, *L, L->F[k])
-                                                : ckpt_get_force<float>(c, F, *L, L->F[k])))
-            return st;
+        if ((st = ckpt_get_force(c, F, *L, k, L->f[1 - hd.cur], buf))) return st;
     if (L->phase && (st = ckpt_get_device(c, F, L->phase, (size_t)L->d.stride, buf))) return st;
     if (hd.has_types) {
         std::vector<uint8_t> types((size_t)L->d.n);

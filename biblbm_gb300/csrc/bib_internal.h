@@ -449,6 +449,8 @@ void launch_import_aos(const Lattice& L, const double* src, int per, int x0, int
 void launch_export_aos(const Lattice& L, double* dst, int per, int x0, int nxc, cudaStream_t s);
 void launch_force_import(const Lattice& L, int buf, const double* src, cudaStream_t s);
 void launch_force_export(const Lattice& L, int buf, double* dst, cudaStream_t s);
+// component a of cells k0 .. k0 + n - 1 of F[buf] from (in) or to `part`, in the field's type
+void launch_force_component(const Lattice& L, int buf, void* part, int a, int64_t k0, int64_t n, bool in, cudaStream_t s);
 void launch_force_fill(const Lattice& L, int buf, cudaStream_t s);
 void launch_phase_import(const Lattice& L, const double* src, cudaStream_t s);
 void launch_nan_scan(const Lattice& L, int* flag, cudaStream_t s);

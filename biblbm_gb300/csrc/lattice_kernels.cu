@@ -661,6 +661,16 @@ __global__ void k_force_export(LatticeDesc d, const FT* __restrict__ F, double* 
     for (int a = 0; a < 3; ++a) dst[a * d.n + k] = (double)F[3 * k + a];
 }
 
+// One component of the cells k0 .. k0 + n - 1 out of (IN: into) the force field, for files that hold one array per
+// component.
+template <class FT, bool IN>
+__global__ void k_force_component(FT* __restrict__ F, FT* __restrict__ part, int a, int64_t k0, int64_t n) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    if (IN) F[3 * (k0 + k) + a] = part[k];
+    else part[k] = F[3 * (k0 + k) + a];
+}
+
 template <class FT>
 __global__ void k_force_fill(LatticeDesc d, FT* __restrict__ F) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -888,6 +898,16 @@ void launch_import_aos(const Lattice& L, const double* src, int per, int x0, int
 
 void launch_export_aos(const Lattice& L, double* dst, int per, int x0, int nxc, cudaStream_t s) {
     if (nxc > 0) BIB_DISPATCH(L.storage, export_aos_t, L, dst, per, x0, nxc, s);
+}
+
+void launch_force_component(const Lattice& L, int buf, void* part, int a, int64_t k0, int64_t n, bool in, cudaStream_t s) {
+    auto run = [&](auto zero) {
+        using FT = decltype(zero);
+        auto kern = in ? k_force_component<FT, true> : k_force_component<FT, false>;
+        kern<<<lin_grid(n, 256), 256, 0, s>>>((FT*)L.F[buf], (FT*)part, a, k0, n);
+    };
+    if (L.storage == BIB_STORAGE_F64) run(double{});
+    else run(float{});
 }
 
 void launch_force_import(const Lattice& L, int buf, const double* src, cudaStream_t s) {
