@@ -238,9 +238,7 @@ __global__ void __launch_bounds__(LinearLayout<T, CPL, COLL>::THREADS, staged_ct
             if (CPL == kCplDense) Fp[q] = (C)SFp[q];
             else if (CPL == kCplSparse) Fp[q] = cp.body[q];
         }
-        // the stage has been read into registers: hand it back to the producer
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
+        release_stage(&empty[s], lane);
         if (!active) continue;
         const Cell3 c = cell_of(d, k);
         if (c.y == 0 || c.y == d.ny - 1 || c.z == 0 || c.z == d.nz - 1) {

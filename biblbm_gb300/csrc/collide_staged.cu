@@ -225,9 +225,7 @@ __device__ __forceinline__ void consume_cell(const LatticeDesc& d, const StagedG
             for (int q = 0; q < 3; ++q) Fp[q] = cp.body[q];
         }
     }
-    // the stage has been read into registers: hand it back to the producer
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty_s);
+    release_stage(empty_s, lane);
     if (!active) return;
     finish_cell<T, CPL, COLL>(d, cp, fout, u_out, phase, celltype, t.row0 + o0, y, fd, f, F, Fp);
 }
@@ -285,9 +283,7 @@ __device__ __forceinline__ void consume_pair(const LatticeDesc& d, const StagedG
             else if (CPL == kCplSparse) Fp[q] = F2(cp.body[q]);
         }
     }
-    // the stage has been read into registers: hand it back to the producer
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty_s);
+    release_stage(empty_s, lane);
     if (!cell.active) return;
     __half* o = fout + k;
     if (d.has_types) {
