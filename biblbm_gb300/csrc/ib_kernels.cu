@@ -2040,7 +2040,10 @@ void launch_membrane_forces(const Lattice& L, cudaStream_t s) {
         return;
     }
     if (L.ib.spread_mode == BIB_SPREAD_DETERMINISTIC) {
-        const int block = L.nvert < 32768 ? 32 : 128;  // few vertices: a warp each to the SMs (FP64 pipe)
+        // one-warp CTAs: few vertices spread over more SMs (FP64 pipe), many take as long either way.  Step with red
+        // cells of 642 vertices, FP64, 32 against 128 threads: 1 cell 350 / 366 us, 10 439 / 460, 30 552 / 552, 260
+        // 3637 / 3642; FP32 with link springs the same within 1 % from 1 to 260
+        const int block = 32;
         const unsigned g = (L.nvert + block - 1) / block;
         if (L.storage == BIB_STORAGE_F64)
             k_membrane_gather<double><<<g, block, 0, s>>>(L.nvert, L.vert_particle, L.pdev, L.pos[L.pcur], L.force, L.stats, L.inter);
@@ -2113,9 +2116,10 @@ void launch_pp_forces(const Lattice& L, cudaStream_t s) {
 void launch_particle_update(const Lattice& L, cudaStream_t s) {
     const int np = (int)L.parts.size();
     if (np == 0) return;
-    // FP64 sums, and in FP32 large meshes (a step of a 1280-triangle membrane in 96^3 FP32 54 us with one CTA, 56 split;
-    // of a 5120-triangle one in 160 x 128 x 128 119 and 111)
-    const bool big = L.storage == BIB_STORAGE_F64 || L.max_nt >= 4096;
+    // FP64 sums, and in FP32 large meshes.  FP32 step of one membrane in 96^3, one CTA against split: 1216 triangles
+    // 59.1 / 59.2 us, 1932 61.7 / 61.7, 2592 65.5 / 60.5, 3248 66.2 / 60.6, 4200 71.2 / 62.0; 16 of 3248 129 / 111, 64 of them
+    // 132 / 136
+    const bool big = L.storage == BIB_STORAGE_F64 || L.max_nt >= 2048;
     const int split = big ? std::min(kMaxUpdateSplit, membrane_split(np, L.max_nt, kUpdateFew)) : 1;
     if (split > 1 && L.upd_partial) {
         const IbView v = single_view(L, -1);
