@@ -391,7 +391,6 @@ bib_status upload(bib_ctx* c, T** dptr, const std::vector<T>& v) {
     return BIB_OK;
 }
 
-// DeformableParticle3D::update (DeformableParticle3D.hh:54-82) on the host, FP64.
 // The tables of a shape in one allocation (S.dev.base).
 bib_status upload_shape(bib_ctx* c, ShapeHost& S) {
     std::vector<unsigned char> all;
@@ -428,6 +427,7 @@ bib_status upload_shape(bib_ctx* c, ShapeHost& S) {
     return BIB_OK;
 }
 
+// DeformableParticle3D::update (DeformableParticle3D.hh:54-82) on the host, FP64.
 void particle_update(const ShapeHost& S, const double* pos, double* st) {
     double area = 0, vol = 0, cx = 0, cy = 0, cz = 0;
     const int nt = (int)S.tri_area.size();

@@ -9,8 +9,8 @@
 // other end, in the first and last rows and planes from the periodic image, the wall rule or the wall
 // buffer.  Those few are read from global memory after the stage has been handed back.
 //
-// Bound by HBM (FP32) and by HBM and issue (FP16) as the row tiles are: 201^3 FP32 5.2 TB/s (3.9 with one
-// thread per cell straight from global memory), FP16 4.1 TB/s (1.25).
+// Bound by HBM (FP32) and by HBM and issue (FP16) as the row tiles are: 201^3, 100 steps in a row, FP32 5.6 TB/s (4.0
+// with one thread per cell straight from global memory), FP16 4.5 TB/s (1.1).
 #include <type_traits>
 
 #include "staged_common.cuh"
@@ -353,12 +353,12 @@ bool linear_t(const Lattice& L, Coupling mode, cudaStream_t s) {
 }  // namespace
 
 // Where the linear tiles take over from the direct kernels (one thread per cell for odd rows, two cells per
-// thread for even ones).  Measured, one lattice-only step (coupled), linear against direct:
-//   FP16, from 2^15 cells: 33^3 10.3 / 10.3 us, 41^3 10.4 / 12.3, 129^3 51 / 162, 201^3 152 / 493 (171 / 630),
-//     1024 x 64 x 64 98 / 266 (112 / 288): the direct kernels' 2-byte accesses are half empty;
-//   FP32 odd rows, from 2^19: 61^3 16.3 / 12.4, 81^3 22 / 33, 201^3 239 / 316 (289 / 361);
+// thread for even ones).  Measured, lattice-only steps in a row, linear against direct:
+//   FP16, from 2^15 cells: 33^3 10.3 / 10.3 us, 41^3 10.3 / 11.3, 81^3 22 / 41, 129^3 47 / 181, 201^3 138 / 555,
+//     1024 x 64 x 64 89 / 266: the direct kernels' 2-byte accesses are half empty;
+//   FP32 odd rows, from 2^19: 61^3 16.3 / 12.4, 81^3 20.4 / 32.8, 129^3 65 / 94, 201^3 221 / 305;
 //   FP32 even rows, from 2^19, only where the direct kernel leaves a quarter of its lanes without a cell:
-//     102 x 101 x 100 45 / 39, 1024 x 64 x 64 141 / 116 (lanes full); 520 x 64 x 64 76 / 98 (half full).
+//     102 x 101 x 100 45 / 39, 1024 x 64 x 64 141 / 114 (lanes full); 520 x 64 x 64 70 / 97 (half full).
 // FP64 is bound by its arithmetic and stays with the direct kernels.
 bool launch_collide_stream_linear(const Lattice& L, Coupling mode, cudaStream_t s) {
     const LatticeDesc& d = L.d;

@@ -1,7 +1,7 @@
 // Immersed-boundary kernels: delta interpolation of the lattice velocity to the
-// membrane vertices, membrane forces + explicit vertex motion + area / volume /
-// centre-of-mass update (one CTA per particle), and delta spreading of the vertex
-// forces into the lattice force field.
+// membrane vertices and their motion, membrane forces (by patches, elements or vertices),
+// delta spreading of the vertex forces into the lattice force field, and the area / volume /
+// centre-of-mass update.
 //
 // Vertices of all particles of a lattice are concatenated: positions (FP64, two
 // buffers swapped every step), velocities and forces (FP64).
@@ -229,7 +229,6 @@ __device__ __noinline__ void move_near_pipe(const IbView& V, int v, const C* u3)
 // adds the share of the previous step's force, sum of w (Fold - body) / 2 over the support
 // nodes off the finite-difference wall rows (whose velocity is the wall's); the sum of the two
 // is the interpolation of j/rho + Fold/2, the reference's computeVelocity field.
-//
 //
 // Many vertices: one thread per vertex.
 template <class UT, int S, bool FOLD = false>

@@ -109,16 +109,6 @@ struct Pair<__half> {
     static __device__ __forceinline__ void store(__half* p, float a, float b, float s) {
         *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a * s, b * s);
     }
-    // scaled values as stored (f-bar * S)
-    static __device__ __forceinline__ void load_raw(const __half* p, float& a, float& b) {
-        const float2 v = __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
-        a = v.x;
-        b = v.y;
-    }
-    static __device__ __forceinline__ void store_raw(__half* p, float a, float b) {
-        *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
-    }
-    static __device__ __forceinline__ float load1_raw(const __half* p) { return __half2float(__ldg(p)); }
 };
 template <>
 struct Pair<float> {
@@ -130,9 +120,6 @@ struct Pair<float> {
     static __device__ __forceinline__ void store(float* p, float a, float b, float) {
         *reinterpret_cast<float2*>(p) = make_float2(a, b);
     }
-    static __device__ __forceinline__ void load_raw(const float* p, float& a, float& b) { load(p, 1.0f, a, b); }
-    static __device__ __forceinline__ void store_raw(float* p, float a, float b) { store(p, a, b, 1.0f); }
-    static __device__ __forceinline__ float load1_raw(const float* p) { return __ldg(p); }
 };
 template <>
 struct Pair<double> {
