@@ -839,6 +839,8 @@ void membrane_and_spread(bib_ctx* c, Lattice& L, int fbuf, bool record_nodes, bo
 //     link springs: 128 x 64 x 64 1 of 642 58.4 / 42.9, 1 of 2562 65.7 / 72.7
 //   FP64 with staged tiles, whose membranes want the pipe that the collision is bound by: 64^3 1 S3 137 / 126, 2 133 / 157,
 //     1 R3 153 / 161, 1 red cell of 162 vertices 147 / 122; 160 x 128 x 128 1 R3 922 / 889, 4 923 / 942, 2 S3 906 / 886
+//     one large cell, whose CTAs' shared memory keeps them one to an SM: 64^3 R4 167 / 164, 128 x 64 x 64 R4 246 / 236, 96^3
+//     R4 352 / 337, a capsule of 2562 336 / 323
 //   FP64 with the direct kernels, for which the velocity field is dear: 129 x 65 x 65 1 R3 332 / 282, 8 S3 319 / 294;
 //     513 x 127 x 127 238 R3 (half a node per cell) 3999 / 3714.
 bool overlap_pays(const Lattice& L) {
@@ -854,7 +856,7 @@ bool overlap_pays(const Lattice& L) {
     if (L.storage == BIB_STORAGE_F16) return nodes <= std::max<int64_t>(40960, n / 16 - 131072);
     if (L.storage == BIB_STORAGE_F32) return nodes <= std::max<int64_t>(one && !springs ? 81920 : 40960, n / 6 - 196608);
     if (L.collide_kernel == BIB_KERNEL_ROWS || !collide_staged_fits(L)) return true;
-    return nodes <= n / 64 + (pairs ? 5120 : 18432);
+    return nodes <= n / 64 + (pairs ? 5120 : 18432) || (one && L.max_nv >= 2048);
 }
 
 bool overlapped_step(const bib_ctx* c, const Lattice& L) {

@@ -20,7 +20,8 @@ def ctx():
 
 # cells of 642 (level 3) or 162 vertices (level 2): nodes below and above the limit of 64 x 48 x 48 cells
 CASES = [("f16", 64, "skalak_bending", 3, (2, 3)), ("f32", 64, "skalak_bending", 3, (2, 3)), ("f32", 64, "rbc_wlcpow", 3, (2, 3)),
-         ("f64", 64, "capsule_skalak", 3, (1, 2)), ("f64", 64, "skalak_bending", 2, (1, 2)), ("f64", 63, "skalak_bending", 3, (1, 4))]
+         ("f64", 64, "capsule_skalak", 3, (1, 2)), ("f64", 64, "skalak_bending", 2, (1, 2)), ("f64", 63, "skalak_bending", 3, (1, 4)),
+         ("f64", 64, "skalak_bending", 4, (1,))]
 
 
 @pytest.mark.parametrize("storage,nx,model,level,counts", CASES)
