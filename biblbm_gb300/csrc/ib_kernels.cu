@@ -470,10 +470,19 @@ __global__ void __launch_bounds__(128) k_force_clear(LatticeDesc d, IbDesc ib, i
 }
 
 // ---------------------------------------------------------------- spreading
-// The whole share of one vertex by one thread, node by node: with a positive field offset, where the
-// periodic remap leaves nodes out.
+// The whole share of vertex v by one thread, node by node: with a positive field offset, where the periodic
+// remap leaves nodes out.
 template <class FT, int S>
-__device__ __noinline__ void spread_vertex_nodes(const LatticeDesc& d, const IbDesc& ib, const double* p, const FT* fv, FT* F) {
+__device__ __noinline__ void spread_vertex_nodes(const IbView& V, int v) {
+    const LatticeDesc& d = V.d;
+    const IbDesc& ib = V.ib;
+    const double* p = V.pos + 3LL * v;
+    const double* force = V.force + 3LL * v;
+    FT* F = static_cast<FT*>(V.F);
+    const double wp = ib.has_pipe ? pipe_weight(ib, p, S == 4 ? 2.0 : 1.5) : 1.0;
+    if (wp <= 0) return;
+    const double share = wp < 1 ? (double)(FT)wp : 1.0;
+    const FT fv[3] = {(FT)(force[0] * share), (FT)(force[1] * share), (FT)(force[2] * share)};
     const int off = (int)ib.offset;
     int64_t lo[3];
     FT w[3][4];
@@ -497,10 +506,12 @@ __device__ __noinline__ void spread_vertex_nodes(const LatticeDesc& d, const IbD
 // by one thread; the kernel's share goes by rows like that of any other vertex.  Measured, the step of 300 cells of
 // 642 vertices in a 256 x 104 x 104 pipe, FP32: Roma 210 us, Peskin 235; node by node for every vertex of a
 // lattice with a pipe boundary 309 and 463.
-template <class FT>
-__device__ __noinline__ void spread_near_wall(const IbView& V, int v, double wp) {
+template <class FT, int S>
+__device__ __noinline__ void spread_near_wall(const IbView& V, int v) {
     const double* p = V.pos + 3LL * v;
     const double* force = V.force + 3LL * v;
+    const double wp = pipe_weight(V.ib, p, S == 4 ? 2.0 : 1.5);
+    if (!(wp < 1)) return;
     const double st = wp <= 0 ? 1.0 : 1. - wp;
     const FT ft[3] = {(FT)(force[0] * st), (FT)(force[1] * st), (FT)(force[2] * st)};
     tophat_spread<FT>(V.d, V.ib, p, ft, static_cast<FT*>(V.F));
@@ -541,7 +552,6 @@ template <class FT, int S, class View>
 __device__ __forceinline__ void spread_tile(SpreadTile<FT, S>& T, const View& view, int v, int inst, const FT* f) {
     using SV = SpreadVertex<FT, S>;
     const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double wp = 1.0;  // warp 0: weight of the kernel against the TopHat, below 1 near a pipe's wall
     if (a < 3) {  // warp a prepares axis a of the 32 vertices
         constexpr int dirac = S == 4 ? BIB_DIRAC_PESKIN : BIB_DIRAC_ROMA;
         bool in = false;
@@ -560,10 +570,11 @@ __device__ __forceinline__ void spread_tile(SpreadTile<FT, S>& T, const View& vi
                 s.inst = inst;
                 s.gx = in ? remap_global(per, N, lo, off) : -1;
                 FT g[3] = {f[0], f[1], f[2]};
-                if (V.ib.has_pipe) {
-                    wp = pipe_weight(V.ib, V.pos + 3LL * v, half_support(dirac));
+                if (V.ib.has_pipe) {  // near the wall the rows take the share wp of the force, or nothing
+                    const double wp = pipe_weight(V.ib, V.pos + 3LL * v, half_support(dirac));
                     if (wp < 1)
                         for (int q = 0; q < 3; ++q) g[q] = (FT)(V.force[3LL * v + q] * (double)(FT)wp);
+                    if (wp <= 0) s.gx = -1;
                 }
 #pragma unroll
                 for (int m = 0; m < S; ++m) {
@@ -585,23 +596,17 @@ __device__ __forceinline__ void spread_tile(SpreadTile<FT, S>& T, const View& vi
         if (lane == 0) T.inside[a] = m;
     }
     __syncthreads();
-    bool in = false;
     if (a == 0) {
-        in = ((T.inside[0] & T.inside[1] & T.inside[2]) >> lane) & 1u;
+        const bool in = ((T.inside[0] & T.inside[1] & T.inside[2]) >> lane) & 1u;
         const IbView& V = view(inst);
         const bool nodewise = in && (int)V.ib.offset > 0;
-        if (!in || nodewise || wp <= 0) T.sv[lane].gx = -1;
+        if (!in || nodewise) T.sv[lane].gx = -1;
         if (v >= 0 && V.spread_lo)
             V.spread_lo[v] = in ? make_int4(T.lo_rec[0][lane], T.lo_rec[1][lane], T.lo_rec[2][lane], 1) : make_int4(0, 0, 0, 0);
-        if (nodewise && !(wp <= 0)) {
-            const FT share = wp < 1 ? (FT)wp : FT(1);
-            FT g[3];
-            for (int q = 0; q < 3; ++q) g[q] = (FT)(V.force[3LL * v + q] * (double)share);
-            spread_vertex_nodes<FT, S>(V.d, V.ib, V.pos + 3LL * v, g, static_cast<FT*>(V.F));
-        }
+        if (nodewise) spread_vertex_nodes<FT, S>(V, v);
+        if (in && V.ib.has_pipe) spread_near_wall<FT, S>(V, v);
     }
     __syncthreads();
-    if (in && wp < 1) spread_near_wall<FT>(view(inst), v, wp);
     for (int it = threadIdx.x; it < kSpreadVerts * SV::ITEMS; it += kSpreadThreads) {
         const int t = it / SV::ITEMS, r = it - t * SV::ITEMS, row = r / SV::WORDS, j = r - row * SV::WORDS;
         const SV& s = T.sv[t];
@@ -1352,7 +1357,7 @@ __global__ void __launch_bounds__(kSpreadThreads, 7) k_membrane_patch(const Patc
     __syncthreads();
     if (v >= 0) {  // one component of an owned vertex per thread
         // summed with the rounding errors beside the sum: an FP64 sum of the corners rounded once, without its
-        // FP64 additions (3 us of the 400 cells' step)
+        // FP64 additions (1.5 us of the 400 cells' step against 3)
         float sum = 0.0f, err = 0.0f;
         for (int e = inc_off[lane]; e < inc_off[lane + 1]; ++e) {
             const float a = tf[3 * inc[e] + warp], s = sum + a, t = s - sum;
