@@ -504,7 +504,7 @@ __device__ __noinline__ void spread_vertex_nodes(const IbView& V, int v) {
 
 // Near the wall of a pipe (weight wp < 1): the TopHat takes the share 1 - wp of a vertex's force, its 24 values
 // by one thread; the kernel's share goes by rows like that of any other vertex.  Measured, the step of 300 cells of
-// 642 vertices in a 256 x 104 x 104 pipe, FP32: Roma 210 us, Peskin 235; node by node for every vertex of a
+// 642 vertices in a 256 x 104 x 104 pipe, FP32: Roma 215 us, Peskin 240; node by node for every vertex of a
 // lattice with a pipe boundary 309 and 463.
 template <class FT, int S>
 __device__ __noinline__ void spread_near_wall(const IbView& V, int v) {
